@@ -114,9 +114,9 @@ template <class CF, int PREC, int REFILL>
 __global__ void __launch_bounds__(KernShape<PREC>::tpb, KernShape<PREC>::min_ctas) batch_kernel(const BatchObj<CF>* objs, int n_objs, FitView<CF> V,
                                                        int64_t budget)
 {
-    __shared__ float4 trig[PREC == AST_PREC_MIXED ? kTrigTable : 1];
+    __shared__ float4 trig[kTrigEntries<PREC>];
     if (PREC == AST_PREC_MIXED) {
-        trig_table_fill(trig);
+        trig_table_fill(trig, kTrigEntries<PREC>);
         __syncthreads();
     }
     const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -447,10 +447,10 @@ __global__ void __launch_bounds__(256, 1) coop_kernel(const BatchObj<CF>* objs, 
                                                       int64_t budget)
 {
     constexpr int G = kCoopLanes;
-    __shared__ float4 trig[PREC == AST_PREC_MIXED ? kTrigTable : 1];
+    __shared__ float4 trig[kTrigEntries<PREC>];
     extern __shared__ __align__(16) unsigned char coop_smem[];
     if (PREC == AST_PREC_MIXED) {
-        trig_table_fill(trig);
+        trig_table_fill(trig, kTrigEntries<PREC>);
         __syncthreads();
     }
     const int r = threadIdx.x % G;

@@ -216,29 +216,77 @@ AST_HD df df_div_fast(df x, df y)
 
 // ---------------------------------------------------------------- sincos
 
-constexpr int kTrigTable = 256;  // table points over one turn
+constexpr int kTrigPoints = 256;  // points over one turn of df_sincos's table
+constexpr int kTurn = 4096;       // points over one turn of the compact angles' table (turn.cuh)
+// float4 entries of both: df_sincos's points, then the compact angles' table, sin(k 2pi/T) as
+// double-floats, its T high words before its T low words.
+constexpr int kTrigTable = kTrigPoints + 2 * kTurn / 4;
 
-// Table entry k: (sin_hi, sin_lo, cos_hi, cos_lo) of k * 2*pi / kTrigTable.
+// The compact angles' table, computed by the compiler: the Taylor series of sin and cos over an
+// eighth of a turn in FP64 (error 2e-16; what is kept has 48 bits), the rest by symmetry.
+struct alignas(16) TurnTable {
+    float v[2 * kTurn];
+};
+constexpr TurnTable make_turn_table()
+{
+    TurnTable t{};
+    for (int k = 0; k <= kTurn / 8; k++) {
+        const double x = 6.283185307179586477 * k / kTurn, x2 = x * x;
+        double s = x, c = 1.0, ts = x, tc = 1.0;
+        for (int i = 1; i <= 10; i++) {
+            ts *= -x2 / ((2 * i) * (2 * i + 1));
+            tc *= -x2 / ((2 * i - 1) * (2 * i));
+            s += ts;
+            c += tc;
+        }
+        const int at[8] = {k,             kTurn / 2 - k, kTurn / 4 - k,     kTurn / 4 + k,
+                           kTurn / 2 + k, kTurn - k,     3 * kTurn / 4 - k, 3 * kTurn / 4 + k};
+        for (int q = 0; q < 8; q++) {
+            const double v = (q & 2 ? c : s) * (q < 4 ? 1.0 : -1.0);
+            const float hi = (float)v;
+            t.v[at[q] & (kTurn - 1)] = hi;
+            t.v[kTurn + (at[q] & (kTurn - 1))] = (float)(v - (double)hi);
+        }
+    }
+    return t;
+}
+#ifdef __CUDACC__
+static __device__ const TurnTable d_turn_table = make_turn_table();
+#endif
+
+// Entry k: (sin_hi, sin_lo, cos_hi, cos_lo) of k * 2*pi / kTrigPoints, or from kTrigPoints on
+// four words of the compact angles' table.
 AST_HD float4 trig_table_entry(int k)
 {
+    float4 v;
+    if (k >= kTrigPoints) {
+#ifdef __CUDA_ARCH__
+        return reinterpret_cast<const float4*>(d_turn_table.v)[k - kTrigPoints];
+#else
+        static constexpr TurnTable table = make_turn_table();
+        const float* f = table.v + 4 * (k - kTrigPoints);
+        v.x = f[0]; v.y = f[1]; v.z = f[2]; v.w = f[3];
+        return v;
+#endif
+    }
     double s, c;
 #ifdef __CUDA_ARCH__
-    sincospi(2.0 * k / kTrigTable, &s, &c);
+    sincospi(2.0 * k / kTrigPoints, &s, &c);
 #else
-    s = sin(2.0 * 3.14159265358979323846 * k / kTrigTable);
-    c = cos(2.0 * 3.14159265358979323846 * k / kTrigTable);
+    s = sin(2.0 * 3.14159265358979323846 * k / kTrigPoints);
+    c = cos(2.0 * 3.14159265358979323846 * k / kTrigPoints);
 #endif
     const df S = df_from_double(s), C = df_from_double(c);
-    float4 v;
     v.x = S.hi; v.y = S.lo; v.z = C.hi; v.w = C.lo;
     return v;
 }
 
 #ifdef __CUDACC__
-// Fill the shared-memory table from every thread of the CTA (then __syncthreads()).
-__device__ __forceinline__ void trig_table_fill(float4* t)
+// Fill the first n entries of the shared-memory table from every thread of the CTA (then
+// __syncthreads()): kTrigPoints for a kernel without compact angles.
+__device__ __forceinline__ void trig_table_fill(float4* t, int n = kTrigTable)
 {
-    for (int k = threadIdx.x; k < kTrigTable; k += blockDim.x) t[k] = trig_table_entry(k);
+    for (int k = threadIdx.x; k < n; k += blockDim.x) t[k] = trig_table_entry(k);
 }
 #endif
 
@@ -259,11 +307,11 @@ AST_HD void df_sincos(df a, const float4* __restrict__ table, df* s_out, df* c_o
     if (fabsf(a.hi) > 65536.0f) a = df_reduce_2pi(a);
     // k = round(a * TABLE / 2pi) with the 1.5*2^23 trick (exact for |k| < 2^22); the low
     // mantissa bits of the biased sum are k mod 2^22, so k mod TABLE is a mask.
-    const float inv_step = (float)(kTrigTable / (2.0 * 3.14159265358979323846));
+    const float inv_step = (float)(kTrigPoints / (2.0 * 3.14159265358979323846));
     const float magic = 12582912.0f;
     const float kb = DF_ADD(DF_MUL(a.hi, inv_step), magic);
     const float k = DF_SUB(kb, magic);
-    const int idx = DF_BITS(kb) & (kTrigTable - 1);
+    const int idx = DF_BITS(kb) & (kTrigPoints - 1);
     // e = a - k * (2pi/TABLE), 2pi/TABLE = C1 + C2 + C3 as three floats.  a.hi - k*C1 is exact
     // in one fma (Cody-Waite with a fused multiply-add): both are multiples of ulp(C1) = 2^-29
     // and |a.hi - k*C1| < 2^-5 for |a.hi| <= 65536, so the difference has at most 24 bits.
@@ -389,7 +437,7 @@ AST_HD void df2_sincos(df2 a, const float4* __restrict__ table, df2* s_out, df2*
         const df ay = fabsf(a.hi.y) > 65536.0f ? df_reduce_2pi(df2_y(a)) : df2_y(a);
         a = df2_pack(ax, ay);
     }
-    const float inv_step = (float)(kTrigTable / (2.0 * 3.14159265358979323846));
+    const float inv_step = (float)(kTrigPoints / (2.0 * 3.14159265358979323846));
     const float magic = 12582912.0f;
     // The table index in scalar operations: the compiler contracts a packed product whose only use
     // is a packed add into one fused multiply-add, even written as mul.rn.f32x2 and add.rn.f32x2
@@ -398,8 +446,8 @@ AST_HD void df2_sincos(df2 a, const float4* __restrict__ table, df2* s_out, df2*
     // never merged, so k is the scalar df_sincos's.
     const float2 kb = make_float2(DF_ADD(DF_MUL(a.hi.x, inv_step), magic), DF_ADD(DF_MUL(a.hi.y, inv_step), magic));
     const float2 k = f2_sub(kb, f2(magic));
-    const float4 T0 = table[DF_BITS(kb.x) & (kTrigTable - 1)];
-    const float4 T1 = table[DF_BITS(kb.y) & (kTrigTable - 1)];
+    const float4 T0 = table[DF_BITS(kb.x) & (kTrigPoints - 1)];
+    const float4 T1 = table[DF_BITS(kb.y) & (kTrigPoints - 1)];
     const float2 e0 = f2_fma(f2_neg(k), f2(0.02454369328916073f), a.hi);
     df2 e = two_sum2(e0, a.lo);
     e = df2_sub_fast(e, two_prod2(k, f2(-6.829904419802801e-10f)));

@@ -121,9 +121,9 @@ __global__ void __launch_bounds__(128) eval_kernel(DevModel M, const void* g_obs
 {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t bar;
-    __shared__ float4 trig[PREC != AST_PREC_FP64 ? kTrigTable : 1];
+    __shared__ float4 trig[kTrigEntries<PREC>];
     if (PREC != AST_PREC_FP64) {
-        trig_table_fill(trig);
+        trig_table_fill(trig, kTrigEntries<PREC>);
         __syncthreads();
     }
     const bool staged = use_smem ? bulk_stage(smem, g_obs, (uint32_t)L.bytes, &bar, err) : false;
@@ -318,8 +318,11 @@ static int launch_eval(ast_ctx* c, const DevModel& dm, const double* d_params, i
     int rc = obs_smem_for(kern, (size_t)c->layout.bytes, c->smem_optin, &smem);
     if (rc) return rc;
     const int tpb = 128;
-    int per_sm = 1;
-    AST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, tpb, smem));
+    // Staged in shared memory only where that leaves the SM as many CTAs (fit_launch_core's rule).
+    int per_sm = 1, staged = 0;
+    AST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, tpb, 0));
+    if (smem) AST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&staged, kern, tpb, smem));
+    if (staged < per_sm) smem = 0;
     if (per_sm < 1) per_sm = 1;
     int64_t blocks = (n + tpb - 1) / tpb;
     const int64_t cap = (int64_t)c->sm_count * per_sm;

@@ -48,9 +48,9 @@ __global__ void __launch_bounds__(MINB == 3 ? 128 : 256, MINB) fit_kernel(DevMod
 {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t bar;
-    __shared__ float4 trig[PREC != AST_PREC_FP64 ? kTrigTable : 1];
+    __shared__ float4 trig[kTrigEntries<PREC>];
     if (PREC != AST_PREC_FP64) {
-        trig_table_fill(trig);
+        trig_table_fill(trig, kTrigEntries<PREC>);
         __syncthreads();
     }
     const bool staged = use_smem ? bulk_stage(smem, g_obs, (uint32_t)L.bytes, &bar, &V.ctr[4], V.stage_wait) : false;

@@ -14,8 +14,13 @@
 #include <math.h>
 #include "dfloat.cuh"
 #include "model.cuh"
+#include "turn.cuh"
 
 namespace ast {
+
+// Entries of the shared trig table (trig_table_fill) that a kernel of a precision needs.
+template <int PREC>
+constexpr int kTrigEntries = PREC == AST_PREC_FP64 ? 1 : PREC == AST_PREC_MIXED_RHS32 ? kTrigPoints : kTrigTable;
 
 // f(t) = t - (1 - t^2) atanh(t) for 0 <= t < 1, without cancellation: for t < 1/2 the series
 // sum_k 2 t^(2k+1) / ((2k-1)(2k+1)), else the closed form (cancellation at most 6x there).
@@ -151,11 +156,11 @@ AST_HD void rk4_step_df2(df2* y, float4 hq, float4 hw, const df* mu, const float
 // |e| <= pi/256, sin e = e (1 - e^2/6), cos e = 1 - e^2/2 (truncation < 2e-10).
 AST_HD void f_sincos_tab(float a, const float4* __restrict__ tab, float* s, float* c)
 {
-    const float inv_step = (float)(kTrigTable / (2.0 * 3.14159265358979323846));
+    const float inv_step = (float)(kTrigPoints / (2.0 * 3.14159265358979323846));
     const float magic = 12582912.0f;
     const float kb = DF_ADD(DF_MUL(a, inv_step), magic);
     const float k = DF_SUB(kb, magic);
-    const int idx = DF_BITS(kb) & (kTrigTable - 1);
+    const int idx = DF_BITS(kb) & (kTrigPoints - 1);
     const float e = DF_FMA(-k, -6.829904419802801e-10f, DF_FMA(-k, 0.02454369328916073f, a));
     const float e2 = DF_MUL(e, e);
     const float se = DF_MUL(e, DF_FMA(e2, -1.0f / 6.0f, 1.0f));  // sin e
@@ -434,11 +439,13 @@ struct MixedFrame {
 };
 constexpr int kMixedFrameFloats = 16;
 
-// The integrated state of one evaluation of the mixed path: y and the ODE constants mu as
-// double-floats (and in FP32 for the FP32 right-hand side), the magnitude frame.
+// The integrated state of one evaluation of the mixed path: the compact state s with the ODE
+// constants mu (turn.cuh), or for the FP32 right-hand side y and muf; the magnitude frame.  y and mu
+// are set up in the ODE's own units and turned into s by mixed_begin.
 struct MixedState {
     df y[6];
     df mu[6];
+    Spin s;
     float muf[6];
     bool torque, bw;
     MixedFrame F;
@@ -519,20 +526,89 @@ AST_HD void mixed_setup(const DevModel& M, const double* params, MixedState& S)
 #undef AST_P
 }
 
+// The compact state from the set-up's initial state.
+AST_HD void mixed_begin(MixedState& S)
+{
+    const Turn phi = turn_from(S.torque ? S.y[3] : S.y[0]);
+    const Turn th = turn_from(S.torque ? S.y[4] : S.y[1]);
+    const Turn ps = S.torque ? turn_from(S.y[5]) : turn_from(S.y[2], 2);
+    S.s.phi = phi;
+    S.s.a = Turn2{ps.k, th.k, make_float2(ps.e, th.e), make_float2(ps.t, th.t)};
+    for (int k = 0; k < 3; k++) {
+        S.s.w[k] = S.y[k];
+        S.s.r[k] = 0.0f;
+        if (S.torque) S.mu[k] = df_from_double(DD_MUL(df_to_double(S.mu[k]), kTurnStep));
+    }
+}
+
+// Euler angles of the compact state.
+AST_HD void spin_angles(const Spin& s, bool torque, df* ang)
+{
+    ang[0] = turn_value(s.phi.k, s.phi.e, s.phi.t, 1);
+    ang[1] = turn_value(s.a.k1, s.a.e.y, s.a.t.y, 1);
+    ang[2] = turn_value(s.a.k0, s.a.e.x, s.a.t.x, torque ? 1 : 2);
+    if (!torque) ang[2] = df{0.5f * ang[2].hi, 0.5f * ang[2].lo};
+}
+
+// The step for a state that turn_step_* declines, an angle that advances by more than 1000 turns in
+// one step: rk4_step_df2 on the angles themselves (a rotation the fixed step does not resolve; any
+// finite or non-finite outcome, as long as it is the model's).  Cold: one copy, not inlined.
+static __host__ __device__ __noinline__ void spin_step_general(Spin* s, bool torque, const df* mu, float4 hq, float4 hw,
+                                                               const float4* tab)
+{
+    df ang[3];
+    spin_angles(*s, torque, ang);
+    const float4 gq = make_float4(hq.x, hq.y, 0.5f * hq.x, 0.5f * hq.y);
+    const float4 gw = make_float4(hw.x, hw.y, 2.0f * hw.x, 2.0f * hw.y);
+    df m[6];
+    for (int k = 0; k < (torque ? 6 : 3); k++)
+        m[k] = torque && k < 3 ? df_from_double(df_to_double(mu[k]) / kTurnStep) : mu[k];
+    if (torque) {
+        df2 Y[3] = {df2_pack(s->w[0], s->w[1]), df2_pack(s->w[2], ang[0]), df2_pack(ang[2], ang[1])};
+        rk4_step_df2<6>(Y, gq, gw, m, tab);
+        s->w[0] = df2_x(Y[0]);
+        s->w[1] = df2_y(Y[0]);
+        s->w[2] = df2_x(Y[1]);
+        s->r[0] = s->r[1] = s->r[2] = 0.0f;
+        ang[0] = df2_y(Y[1]);
+        ang[2] = df2_x(Y[2]);
+        ang[1] = df2_y(Y[2]);
+    } else {
+        df2 Y[2] = {df2_pack(ang[2], ang[1]), df2_pack(ang[0], df{0.0f, 0.0f})};
+        rk4_step_df2<3>(Y, gq, gw, m, tab);
+        ang[2] = df2_x(Y[0]);
+        ang[1] = df2_y(Y[0]);
+        ang[0] = df2_x(Y[1]);
+    }
+    const Turn th = turn_from(ang[1]), ps = turn_from(ang[2], torque ? 1 : 2);
+    s->phi = turn_from(ang[0]);
+    s->a = Turn2{ps.k, th.k, make_float2(ps.e, th.e), make_float2(ps.t, th.t)};
+}
+
+// Called on copies, so that the state itself stays in registers.
+AST_HD void spin_step_beyond(MixedState& S, float4 hq, float4 hw, const float4* tab)
+{
+    Spin t = S.s;
+    df mu[6];
+    for (int k = 0; k < (S.torque ? 6 : 3); k++) mu[k] = S.mu[k];
+    spin_step_general(&t, S.torque, mu, hq, hw, tab);
+    S.s = t;
+}
+
 // Integrate from observation i-1 to i (cuda.c:319-372; nothing for i = 0) and return the Euler
-// angles (phi, theta, psi) reduced to [-pi, pi].  They enter the right-hand side and the
-// brightness only through sin and cos, so the state itself is kept reduced: the double-float then
-// resolves the phase to ~1e-14 rad instead of u^2 of the accumulated angle.  RHS32: the FP32
-// right-hand side (AST_PREC_MIXED_RHS32), a separate instantiation so that the double-float
-// kernels carry none of its code.
+// angles (phi, theta, psi) in [-pi, pi].  They enter the right-hand side and the brightness only
+// through sin and cos, so the state keeps no whole turns.  RHS32: the FP32 right-hand side
+// (AST_PREC_MIXED_RHS32), a separate instantiation so that the double-float kernels carry none of
+// its code.
 template <bool RHS32>
 AST_HD void mixed_advance(MixedState& S, const ObsView& o, int i, const float4* tab, df* ang)
 {
-    if (i > 0) {
-        const int N_steps = o.nst[i];
-        const float4 hq = o.hq[i], hw = o.hw[i];
-        // Not unrolled: one copy of the step keeps the hot loop inside the instruction cache.
-        if (RHS32) {
+    if (RHS32) {
+        if (i > 0) {
+            const int N_steps = o.nst[i];
+            const float4 q = o.hq[i], w = o.hw[i];
+            const float4 hq = make_float4(q.x, q.y, 0.5f * q.x, 0.5f * q.y);  // (h, h/2)
+            const float4 hw = make_float4(w.x, w.y, 2.0f * w.x, 2.0f * w.y);  // (h/6, h/3)
             if (S.torque) {
 #pragma unroll 1
                 for (int l = 0; l < N_steps; l++) rk4_step_f32<6>(S.y, hq, hw, S.muf, tab);
@@ -540,41 +616,52 @@ AST_HD void mixed_advance(MixedState& S, const ObsView& o, int i, const float4* 
 #pragma unroll 1
                 for (int l = 0; l < N_steps; l++) rk4_step_f32<3>(S.y, hq, hw, S.muf, tab);
             }
-        } else if (S.torque) {
-            df2 Y[3] = {df2_pack(S.y[0], S.y[1]), df2_pack(S.y[2], S.y[3]), df2_pack(S.y[5], S.y[4])};
-#pragma unroll 1
-            for (int l = 0; l < N_steps; l++) rk4_step_df2<6>(Y, hq, hw, S.mu, tab);
-            S.y[0] = df2_x(Y[0]);
-            S.y[1] = df2_y(Y[0]);
-            S.y[2] = df2_x(Y[1]);
-            S.y[3] = df2_y(Y[1]);
-            S.y[5] = df2_x(Y[2]);
-            S.y[4] = df2_y(Y[2]);
+        }
+        // (Constant indices only: an index computed at run time would move y to local memory.)
+        if (S.torque) {
+            S.y[3] = df_reduce_2pi(S.y[3]);
+            S.y[4] = df_reduce_2pi(S.y[4]);
+            S.y[5] = df_reduce_2pi(S.y[5]);
+            ang[0] = S.y[3];
+            ang[1] = S.y[4];
+            ang[2] = S.y[5];
         } else {
-            df2 Y[2] = {df2_pack(S.y[2], S.y[1]), df2_pack(S.y[0], df{0.0f, 0.0f})};
+            S.y[0] = df_reduce_2pi(S.y[0]);
+            S.y[1] = df_reduce_2pi(S.y[1]);
+            S.y[2] = df_reduce_2pi(S.y[2]);
+            ang[0] = S.y[0];
+            ang[1] = S.y[1];
+            ang[2] = S.y[2];
+        }
+        return;
+    }
+    if (i > 0) {
+        const int N_steps = o.nst[i];
+        const float4 hq = o.hq[i], hw = o.hw[i];
+        const float* turn = reinterpret_cast<const float*>(tab + kTrigPoints);
+        SpinStep C;
+        C.q = df{hq.z, hq.w};
+        C.c6 = df{hw.z, hw.w};
+        if (S.torque) {
+            const df qh = df_mul_fast(C.q, df{hq.x, hq.y});
+            for (int k = 0; k < 3; k++) C.k[k] = df_mul_fast(S.mu[3 + k], qh);
+        } else {
+            C.k[0] = df_mul_fast(S.mu[0], C.q);
+            C.k[1] = df_mul_fast(C.k[0], S.mu[1]);
+            C.k[2] = df_mul_fast(C.k[0], S.mu[2]);
+        }
+        // Not unrolled: one copy of the step keeps the hot loop inside the instruction cache.
+        if (S.torque) {
 #pragma unroll 1
-            for (int l = 0; l < N_steps; l++) rk4_step_df2<3>(Y, hq, hw, S.mu, tab);
-            S.y[2] = df2_x(Y[0]);
-            S.y[1] = df2_y(Y[0]);
-            S.y[0] = df2_x(Y[1]);
+            for (int l = 0; l < N_steps; l++)
+                if (!turn_step_torque(S.s, C, S.mu, turn)) spin_step_beyond(S, hq, hw, tab);
+        } else {
+#pragma unroll 1
+            for (int l = 0; l < N_steps; l++)
+                if (!turn_step_free(S.s, C, turn)) spin_step_beyond(S, hq, hw, tab);
         }
     }
-    // (Constant indices only: an index computed at run time would move y to local memory.)
-    if (S.torque) {
-        S.y[3] = df_reduce_2pi(S.y[3]);
-        S.y[4] = df_reduce_2pi(S.y[4]);
-        S.y[5] = df_reduce_2pi(S.y[5]);
-        ang[0] = S.y[3];
-        ang[1] = S.y[4];
-        ang[2] = S.y[5];
-    } else {
-        S.y[0] = df_reduce_2pi(S.y[0]);
-        S.y[1] = df_reduce_2pi(S.y[1]);
-        S.y[2] = df_reduce_2pi(S.y[2]);
-        ang[0] = S.y[0];
-        ang[1] = S.y[1];
-        ang[2] = S.y[2];
-    }
+    spin_angles(S.s, S.torque, ang);
 }
 
 // FP32 model magnitude at observation i for the Euler angles (phi, theta, psi): the body frame
@@ -669,6 +756,7 @@ __host__ __device__ CF chi2_mixed(const DevModel& M, const ObsView& o, const dou
     int n_cand = 0;
     MixedState S;
     mixed_setup(M, params, S);
+    if (!RHS32) mixed_begin(S);
     DfFrame F;
     if (flags & AST_NUDGE) F = make_df_frame(M, params);
     for (int i = 0; i < N_data; i++) {
@@ -824,6 +912,7 @@ __device__ CF chi2_mixed_tile(const DevModel& M, const ObsView& o, const double*
     for (int m = 0; m < N_filters; m++) { sum_y2[m] = df{0.0f, 0.0f}; sum_y[m] = df{0.0f, 0.0f}; }
     MixedState S;
     mixed_setup(M, params, S);
+    mixed_begin(S);
     frame_store(fr, lane, S.F);
     const bool bw = S.bw;
     for (int i0 = 0; i0 < N_data; i0 += T) {

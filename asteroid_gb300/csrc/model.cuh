@@ -72,8 +72,8 @@ struct ObsView {
     const double* sz;
     // Derived for the mixed-precision path (prep_obs_point): step sizes as double-floats,
     // unit vectors rounded to float, per-filter weight sums.
-    const float4* hq;      // (h, h/2)
-    const float4* hw;      // (h/6, h/3)
+    const float4* hq;      // (h, q), q = h T/2pi (turn.cuh)
+    const float4* hw;      // (h/6, 1/(6q))
     const float* efx;
     const float* efy;
     const float* efz;

@@ -7,8 +7,8 @@
 // float, per-filter weight sums).  The functions are __host__ __device__ so that a host build
 // can prepare a block the same way.
 #pragma once
-#include "dfloat.cuh"
 #include "model.cuh"
+#include "turn.cuh"
 
 namespace ast {
 
@@ -58,12 +58,14 @@ AST_HD void prep_obs_point(const DevModel& M, char* base, const ObsLayout& L, in
         ef[k * n + i] = (float)ex[k * n + i];
         sf[k * n + i] = (float)sx[k * n + i];
     }
-    const df H = df_from_double(hi), HH = df_from_double(0.5 * hi);
-    const df H6 = df_from_double(hi / 6.0), H3 = df_from_double(hi / 3.0);
+    // h, h/6; and of the step counted in compact angles' table points, q = h T/2pi: q, 1/(6q).
+    const double q = hi / kTurnStep;
+    const df H = df_from_double(hi), H6 = df_from_double(hi / 6.0);
+    const df Q = df_from_double(q), C6 = df_from_double(i == 0 ? 0.0 : 1.0 / (6.0 * q));
     float4* hq = (float4*)(base + L.off_hq);
     float4* hw = (float4*)(base + L.off_hw);
-    hq[i] = float4{H.hi, H.lo, HH.hi, HH.lo};
-    hw[i] = float4{H6.hi, H6.lo, H3.hi, H3.lo};
+    hq[i] = float4{H.hi, H.lo, Q.hi, Q.lo};
+    hw[i] = float4{H6.hi, H6.lo, C6.hi, C6.lo};
 }
 
 // Per-filter sums of the weights, in observation order (the sum_w of cuda.c:707-714, which

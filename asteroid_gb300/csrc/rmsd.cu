@@ -63,9 +63,9 @@ struct RmsdView {
 template <class CF, int PREC>
 __global__ void rmsd_setup_kernel(DevModel M, const void* g_obs, ObsLayout L, const double* p0, CF* x0, CF* f01)
 {
-    __shared__ float4 trig[PREC == AST_PREC_MIXED ? kTrigTable : 1];
+    __shared__ float4 trig[kTrigEntries<PREC>];
     if (PREC == AST_PREC_MIXED) {
-        trig_table_fill(trig);
+        trig_table_fill(trig, kTrigEntries<PREC>);
         __syncthreads();
     }
     if (threadIdx.x != 0) return;
@@ -146,9 +146,9 @@ __global__ void __launch_bounds__(KernShape<PREC>::tpb, KernShape<PREC>::min_cta
 {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t bar;
-    __shared__ float4 trig[PREC == AST_PREC_MIXED ? kTrigTable : 1];
+    __shared__ float4 trig[kTrigEntries<PREC>];
     if (PREC == AST_PREC_MIXED) {
-        trig_table_fill(trig);
+        trig_table_fill(trig, kTrigEntries<PREC>);
         __syncthreads();
     }
     const bool staged = use_smem ? bulk_stage(smem, g_obs, (uint32_t)L.bytes, &bar, &V.ctr[4]) : false;
