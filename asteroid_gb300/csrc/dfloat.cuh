@@ -218,14 +218,15 @@ AST_HD df df_div_fast(df x, df y)
 
 constexpr int kTrigPoints = 256;  // points over one turn of df_sincos's table
 constexpr int kTurn = 4096;       // points over one turn of the compact angles' table (turn.cuh)
+constexpr int kTurnRow = kTurn + kTurn / 4;  // a quarter of a turn more: cos at k is sin at k + T/4
 // float4 entries of both: df_sincos's points, then the compact angles' table, sin(k 2pi/T) as
-// double-floats, its T high words before its T low words.
-constexpr int kTrigTable = kTrigPoints + 2 * kTurn / 4;
+// double-floats, its row of high words before its row of low words.
+constexpr int kTrigTable = kTrigPoints + 2 * kTurnRow / 4;
 
 // The compact angles' table, computed by the compiler: the Taylor series of sin and cos over an
 // eighth of a turn in FP64 (error 2e-16; what is kept has 48 bits), the rest by symmetry.
 struct alignas(16) TurnTable {
-    float v[2 * kTurn];
+    float v[2 * kTurnRow];
 };
 constexpr TurnTable make_turn_table()
 {
@@ -245,8 +246,12 @@ constexpr TurnTable make_turn_table()
             const double v = (q & 2 ? c : s) * (q < 4 ? 1.0 : -1.0);
             const float hi = (float)v;
             t.v[at[q] & (kTurn - 1)] = hi;
-            t.v[kTurn + (at[q] & (kTurn - 1))] = (float)(v - (double)hi);
+            t.v[kTurnRow + (at[q] & (kTurn - 1))] = (float)(v - (double)hi);
         }
+    }
+    for (int k = kTurn; k < kTurnRow; k++) {
+        t.v[k] = t.v[k - kTurn];
+        t.v[kTurnRow + k] = t.v[kTurnRow + k - kTurn];
     }
     return t;
 }

@@ -5,8 +5,8 @@
 // the FP32 operations.  The kernels that run it are bound by the FP32 pipe, so its lane operations
 // are its time.  What it does differently:
 //
-//  * An angle is k table steps plus a remainder, a = k 2pi/T + e + t with |e| <= pi/T and t a
-//    small correction (Turn).  Advancing it adds the increment to (e, t) and takes the nearest
+//  * An angle is k table steps plus a remainder, a = (k + e + t) 2pi/T with |e| <= 1/2 and t a small
+//    correction (Turn).  Advancing it adds the increment to (e, t) and takes the nearest
 //    whole number of steps out again: four operations that are at the same time the argument
 //    reduction of the next sin and cos.  The rounding of an update is u^2 of the increment, not
 //    of the accumulated angle.
@@ -64,7 +64,8 @@ AST_HD df2 u_axpy2(df2 y, float2 c, df2 k)
 
 // ------------------------------------------------ compact angles
 
-// The angle (k + e + t) 2pi/T, |e| <= 1/2, k taken modulo a multiple of T by its owner.
+// The angle (k/4 + e + t) 2pi/T, |e| <= 1/2, k taken modulo a multiple of 4 T by its owner: k counts
+// the bytes of the table, so that one mask gives the address of all four words of sin and cos.
 struct Turn {
     uint32_t k;
     float e, t;
@@ -85,28 +86,29 @@ AST_HD Turn turn_reduce(df a, uint32_t k0)
 {
     const float magic = 12582912.0f;
     const float kb = DF_ADD(a.hi, magic);
-    return Turn{k0 + (uint32_t)DF_BITS(kb), DF_SUB(a.hi, DF_SUB(kb, magic)), a.lo};
+    return Turn{k0 + 4u * (uint32_t)DF_BITS(kb), DF_SUB(a.hi, DF_SUB(kb, magic)), a.lo};
 }
 AST_HD Turn2 turn_reduce2(df2 a, uint32_t k0, uint32_t k1)
 {
     const float2 magic = f2(12582912.0f);
     const float2 kb = f2_add(a.hi, magic);
-    return Turn2{k0 + (uint32_t)DF_BITS(kb.x), k1 + (uint32_t)DF_BITS(kb.y), f2_sub(a.hi, f2_sub(kb, magic)), a.lo};
+    return Turn2{k0 + 4u * (uint32_t)DF_BITS(kb.x), k1 + 4u * (uint32_t)DF_BITS(kb.y),
+                 f2_sub(a.hi, f2_sub(kb, magic)), a.lo};
 }
 AST_HD df2 turn_rest(const Turn2& a) { return df2{a.e, a.t}; }
 
-// The value in radians of a compact angle whose k counts modulo `turns` times T, in
+// The value in radians of a compact angle whose k/4 counts modulo `turns` times T, in
 // [-turns pi, turns pi].
 AST_HD df turn_value(uint32_t k, float e, float t, int turns)
 {
     const int half = turns * kTurn / 2;
-    int m = (int)((k + (uint32_t)half) & (uint32_t)(turns * kTurn - 1)) - half;
+    int m = (int)(((k >> 2) + (uint32_t)half) & (uint32_t)(turns * kTurn - 1)) - half;
     if (m == -half && e < 0.0f) m = half;
     const float n = (float)m;
     return df_mul(df_add_f(two_sum(n, e), t), df{kTurnStepHi, kTurnStepLo});
 }
 
-// An angle in radians as a compact one (turns = 1), or twice it (turns = 2, its k modulo 2 T).
+// An angle in radians as a compact one (turns = 1), or twice it (turns = 2, its k/4 modulo 2 T).
 AST_HD Turn turn_from(df a, int turns = 1)
 {
     const df r = df_mul(df_reduce_2pi(a), df_from_double(turns / kTurnStep));
@@ -120,10 +122,11 @@ AST_HD Turn turn_from(df a, int turns = 1)
 // would carry that much rounding through every product and sum that follows.
 AST_HD void turn_sincos2(const Turn2& a, const float* __restrict__ tab, df2* s, df2* c)
 {
-    const uint32_t i0 = a.k0 & (kTurn - 1), i1 = a.k1 & (kTurn - 1);
-    const uint32_t j0 = (a.k0 + kTurn / 4) & (kTurn - 1), j1 = (a.k1 + kTurn / 4) & (kTurn - 1);
-    const float2 Sh = make_float2(tab[i0], tab[i1]), Sl = make_float2(tab[kTurn + i0], tab[kTurn + i1]);
-    const float2 Ch = make_float2(tab[j0], tab[j1]), Cl = make_float2(tab[kTurn + j0], tab[kTurn + j1]);
+    const float* t0 = reinterpret_cast<const float*>(reinterpret_cast<const char*>(tab) + (a.k0 & (4 * kTurn - 1)));
+    const float* t1 = reinterpret_cast<const float*>(reinterpret_cast<const char*>(tab) + (a.k1 & (4 * kTurn - 1)));
+    const float2 Sh = make_float2(t0[0], t1[0]), Sl = make_float2(t0[kTurnRow], t1[kTurnRow]);
+    const float2 Ch = make_float2(t0[kTurn / 4], t1[kTurn / 4]);
+    const float2 Cl = make_float2(t0[kTurnRow + kTurn / 4], t1[kTurnRow + kTurn / 4]);
     const float2 c1 = f2(kTurnStepHi);
     const float2 xh = f2_mul(c1, a.e);
     const float2 xl = f2_fma(c1, a.t, f2_fma(f2(kTurnStepLo), a.e, f2_fma(c1, a.e, f2_neg(xh))));
@@ -179,7 +182,7 @@ AST_HD void word3_mad(df& w, float& r, df c, df a)
 }
 
 // The integrated state.  Torque (cuda.c:46-58): angular velocity w in rad/day (three words each),
-// phi, and a = (psi, theta).  Free rotation (cuda.c:69-75): phi and a = (2 psi, theta), the first k
+// phi, and a = (psi, theta).  Free rotation (cuda.c:69-75): phi and a = (2 psi, theta), the first k/4
 // modulo 2 T, so that psi is half of it modulo 2 pi.
 struct Spin {
     df w[3];
@@ -203,15 +206,13 @@ AST_HD bool turn_step_torque(Spin& Y, const SpinStep& C, const df* mu, const flo
     df w2 = W2;
     Turn2 a = Y.a;
     const df2 A = turn_rest(a);
-    df2 acc01{f2(0.0f), f2(0.0f)}, acc23 = acc01, accA = acc01;  // w0 w1, w2 phi, psi theta
+    df2 K01, K23, KA;  // w0 w1, w2 phi, psi theta
     float big = 0.0f;
-#pragma unroll 1
-    for (int st = 0; st < 4; st++) {
+    auto rhs = [&]() {
         df2 s, c;
         turn_sincos2(a, tab, &s, &c);
         const df w0 = df2_x(w01), w1 = df2_y(w01);
-        const df s5 = df2_x(s), c5 = df2_x(c), c4 = df2_y(c);
-        const df s4 = df2_y(s);
+        const df s5 = df2_x(s), c5 = df2_x(c), s4 = df2_y(s), c4 = df2_y(c);
         const df K0 = u_add(u_mul(mu[0], u_mul(w1, w2)), C.k[0]);
         const df K1 = u_add(u_mul(mu[1], u_mul(w2, w0)), C.k[1]);
         const df K2 = u_add(u_mul(mu[2], u_mul(w0, w1)), C.k[2]);
@@ -223,21 +224,35 @@ AST_HD bool turn_step_torque(Spin& Y, const SpinStep& C, const df* mu, const flo
         const float p = DF_MUL(q, c4.hi);
         const float pe = DF_FMA(K3.lo, c4.hi, DF_FMA(q, c4.lo, DF_FMA(q, c4.hi, -p)));
         const df d = two_sum(w2.hi, -p);
-        const df K5{d.hi, DF_ADD(d.lo, DF_SUB(w2.lo, pe))};
-        const df2 K01 = df2_pack(K0, K1), K23 = df2_pack(K2, K3), KA = df2_pack(K5, K4);
-        const float2 wt = f2((st == 1 || st == 2) ? 2.0f : 1.0f);  // K1 + 2 K2 + 2 K3 + K4
-        acc01 = u_axpy2(acc01, wt, K01);
-        acc23 = u_axpy2(acc23, wt, K23);
-        accA = u_axpy2(accA, wt, KA);
-        if (st < 3) {
-            const float cs = st < 2 ? 0.5f : 1.0f;
-            w01 = u_axpy2(W01, f2(cs), K01);
-            w2 = u_axpy(W2, cs, K2);
-            const df2 b = u_axpy2(A, f2(cs), KA);
-            big = fmaxf(big, fmaxf(fabsf(b.hi.x), fabsf(b.hi.y)));
-            a = turn_reduce2(b, Y.a.k0, Y.a.k1);
-        }
+        K01 = df2_pack(K0, K1);
+        K23 = df2_pack(K2, K3);
+        KA = df2_pack(df{d.hi, DF_ADD(d.lo, DF_SUB(w2.lo, pe))}, K4);
+    };
+    auto next = [&](float h) {  // the next stage's point, y + h K
+        w01 = u_axpy2(W01, f2(h), K01);
+        w2 = u_axpy(W2, h, df2_x(K23));
+        const df2 b = u_axpy2(A, f2(h), KA);
+        big = fmaxf(big, fmaxf(fabsf(b.hi.x), fabsf(b.hi.y)));
+        a = turn_reduce2(b, Y.a.k0, Y.a.k1);
+    };
+    // K1 + 2 K2 + 2 K3 + K4.  The ends apart: their sums and their next point need less, and the
+    // middle stays one rolled copy for the instruction cache (33.0 ms against 35.1 rolled whole
+    // and 34.9 unrolled whole, 58 368 evaluations of a 60-day light curve).
+    rhs();
+    df2 acc01 = K01, acc23 = K23, accA = KA;
+    next(0.5f);
+#pragma unroll 1
+    for (int st = 1; st < 3; st++) {
+        rhs();
+        acc01 = u_axpy2(acc01, f2(2.0f), K01);
+        acc23 = u_axpy2(acc23, f2(2.0f), K23);
+        accA = u_axpy2(accA, f2(2.0f), KA);
+        next(st == 1 ? 0.5f : 1.0f);
     }
+    rhs();
+    acc01 = u_axpy2(acc01, f2(1.0f), K01);
+    acc23 = u_axpy2(acc23, f2(1.0f), K23);
+    accA = u_axpy2(accA, f2(1.0f), KA);
     const df2 b = turn_sixth2(A, accA);
     const df f = turn_sixth(Y.phi.e, Y.phi.t, df2_y(acc23));
     big = fmaxf(fmaxf(big, fabsf(f.hi)), fmaxf(fabsf(b.hi.x), fabsf(b.hi.y)));
@@ -254,27 +269,36 @@ AST_HD bool turn_step_free(Spin& Y, const SpinStep& C, const float* __restrict__
 {
     Turn2 a = Y.a;
     const df2 A = turn_rest(a);
-    df2 accA{f2(0.0f), f2(0.0f)};
-    df accF{0.0f, 0.0f};
+    df2 KA;
+    df K0;
     float big = 0.0f;
-#pragma unroll 1
-    for (int st = 0; st < 4; st++) {
+    auto rhs = [&]() {
         df2 s, c;
         turn_sincos2(a, tab, &s, &c);
-        const df K0 = u_add(C.k[1], df_neg(u_mul(C.k[2], df2_x(c))));
+        K0 = u_add(C.k[1], df_neg(u_mul(C.k[2], df2_x(c))));
         const df K1 = u_mul(u_mul(C.k[2], df2_y(s)), df2_x(s));
         const df d = u_add(C.k[0], df_neg(K0));
-        const df K2 = u_mul(df2_y(c), df{DF_MUL(2.0f, d.hi), DF_MUL(2.0f, d.lo)});
-        const df2 KA = df2_pack(K2, K1);
-        const float wt = (st == 1 || st == 2) ? 2.0f : 1.0f;
-        accA = u_axpy2(accA, f2(wt), KA);
-        accF = u_axpy(accF, wt, K0);
-        if (st < 3) {
-            const df2 b = u_axpy2(A, f2(st < 2 ? 0.5f : 1.0f), KA);
-            big = fmaxf(big, fmaxf(fabsf(b.hi.x), fabsf(b.hi.y)));
-            a = turn_reduce2(b, Y.a.k0, Y.a.k1);
-        }
+        KA = df2_pack(u_mul(df2_y(c), df{DF_MUL(2.0f, d.hi), DF_MUL(2.0f, d.lo)}), K1);
+    };
+    auto next = [&](float h) {
+        const df2 b = u_axpy2(A, f2(h), KA);
+        big = fmaxf(big, fmaxf(fabsf(b.hi.x), fabsf(b.hi.y)));
+        a = turn_reduce2(b, Y.a.k0, Y.a.k1);
+    };
+    rhs();
+    df2 accA = KA;
+    df accF = K0;
+    next(0.5f);
+#pragma unroll 1
+    for (int st = 1; st < 3; st++) {
+        rhs();
+        accA = u_axpy2(accA, f2(2.0f), KA);
+        accF = u_axpy(accF, 2.0f, K0);
+        next(st == 1 ? 0.5f : 1.0f);
     }
+    rhs();
+    accA = u_axpy2(accA, f2(1.0f), KA);
+    accF = u_axpy(accF, 1.0f, K0);
     const df2 b = turn_sixth2(A, accA);
     const df f = turn_sixth(Y.phi.e, Y.phi.t, accF);
     big = fmaxf(fmaxf(big, fabsf(f.hi)), fmaxf(fabsf(b.hi.x), fabsf(b.hi.y)));

@@ -22,7 +22,7 @@ void h_turn_sincos(int n, const int* k, const float* e, const float* t, float* o
     const std::vector<float4> tab = table();
     for (int i = 0; i < n; i++) {
         df2 s, c;
-        turn_sincos2(Turn2{(uint32_t)k[2 * i], (uint32_t)k[2 * i + 1], make_float2(e[2 * i], e[2 * i + 1]),
+        turn_sincos2(Turn2{4u * (uint32_t)k[2 * i], 4u * (uint32_t)k[2 * i + 1], make_float2(e[2 * i], e[2 * i + 1]),
                            make_float2(t[2 * i], t[2 * i + 1])},
                      reinterpret_cast<const float*>(tab.data() + kTrigPoints), &s, &c);
         const float v[8] = {s.hi.x, s.lo.x, c.hi.x, c.lo.x, s.hi.y, s.lo.y, c.hi.y, c.lo.y};
