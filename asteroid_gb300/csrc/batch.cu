@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(256, 1) coop_kernel(const BatchObj<CF>* objs, 
 
 // One CTA per (object, group) of gmap.
 template <class CF>
-__global__ void batch_group_best_kernel(const BatchObj<CF>* objs, const int2* gmap, FitView<CF> V)
+__global__ void __launch_bounds__(256) batch_group_best_kernel(const BatchObj<CF>* objs, const int2* gmap, FitView<CF> V)
 {
     const int2 kg = gmap[blockIdx.x];
     const BatchObj<CF>& B = objs[kg.x];

@@ -13,6 +13,7 @@
 
 #include "asteroid_gb300.h"
 #include "engine.cuh"
+#include "group64.cuh"
 #include "mixed.cuh"
 #include "model.cuh"
 #include "prep.cuh"
@@ -147,37 +148,61 @@ __global__ void __launch_bounds__(128, MINB) eval_kernel(DevModel M, const void*
     bulk_drain(&bar, staged || !use_smem);
 }
 
-// Model magnitudes (and, with geo, the renderer's geometry) of one parameter vector at every
-// observation (single thread: the RK4 recursion is sequential in time).
-__global__ void model_curve_kernel(DevModel M, const void* g_obs, ObsLayout L, const double* params, double* vmod,
-                                   double* geo = nullptr)
+// The FP64 evaluation by groups of G lanes (group64.cuh), one warp a CTA: few vectors take as many SMs
+// as there are warps.
+template <class CF, int G>
+__global__ void __launch_bounds__(32, 8) eval_group_kernel(DevModel M, const void* g_obs, ObsLayout L,
+                                                        const double* __restrict__ params, int64_t n,
+                                                        double* __restrict__ chi2, double* __restrict__ dv)
 {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    const ObsView o = L.view(g_obs, M.n_data);
+    const int64_t k = (blockIdx.x * (int64_t)32 + threadIdx.x) / G;
+    const int64_t kk = k < n ? k : n - 1;  // the last warp's spare groups repeat the last vector
+    double p[AST_MAX_PARAMS];
+    for (int i = 0; i < M.n_params; i++) p[i] = params[kk * M.n_params + i];
+    CF d[AST_MAX_FILTERS];
+    for (int m = 0; m < M.n_filters; m++) d[m] = 0;
+    const CF r = chi2_fp64_group<CF, G>(M, o, p, d);
+    if (k >= n || threadIdx.x % G) return;
+    chi2[k] = (double)r;
+    if (dv)
+        for (int m = 0; m < M.n_filters; m++) dv[k * M.n_filters + m] = (double)d[m];
+}
+
+// Model magnitudes (and, with geo, the renderer's geometry) of one parameter vector at every
+// observation, by one warp: the RK4 recursion is sequential in time.
+__global__ void __launch_bounds__(32, 1) model_curve_kernel(DevModel M, const void* g_obs, ObsLayout L, const double* params,
+                                                         double* vmod, double* geo = nullptr)
+{
     const ObsView o = L.view(g_obs, M.n_data);
     double p[AST_MAX_PARAMS];
     for (int i = 0; i < M.n_params; i++) p[i] = params[i];
     double d[AST_MAX_FILTERS];
     DevModel M2 = M;
     M2.flags &= ~AST_NUDGE;  // the curve is the brightness model alone
-    chi2_fp64<double>(M2, o, p, d, vmod, nullptr, geo);
+    chi2_fp64_group<double, 32>(M2, o, p, d, vmod, nullptr, geo);
 }
 
-// Euler angles at every observation along the FP64 or the mixed-precision integration.
+// Euler angles at every observation along the FP64 (one warp) or the mixed-precision integration (one
+// thread).
 template <int PREC>
-__global__ void model_angles_kernel(DevModel M, const void* g_obs, ObsLayout L, const double* params, double* ang)
+__global__ void __launch_bounds__(32, 1) model_angles_kernel(DevModel M, const void* g_obs, ObsLayout L, const double* params,
+                                                          double* ang)
 {
-    __shared__ float4 trig[kTrigTable];
-    trig_table_fill(trig);
-    __syncthreads();
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    __shared__ float4 trig[kTrigEntries<PREC>];
     const ObsView o = L.view(g_obs, M.n_data);
     double p[AST_MAX_PARAMS];
     for (int i = 0; i < M.n_params; i++) p[i] = params[i];
     double d[AST_MAX_FILTERS];
     DevModel M2 = M;
     M2.flags &= ~AST_NUDGE;
-    if (PREC == AST_PREC_FP64) chi2_fp64<double>(M2, o, p, d, nullptr, ang);
-    else chi2_mixed<double, PREC == AST_PREC_MIXED_RHS32>(M2, o, p, d, trig, ang);
+    if (PREC == AST_PREC_FP64) {
+        chi2_fp64_group<double, 32>(M2, o, p, d, nullptr, ang);
+        return;
+    }
+    trig_table_fill(trig, kTrigEntries<PREC>);
+    __syncthreads();
+    if (threadIdx.x == 0) chi2_mixed<double, PREC == AST_PREC_MIXED_RHS32>(M2, o, p, d, trig, ang);
 }
 
 // FMA throughput probe (roofline denominators for CUDA-core bound kernels).
@@ -310,10 +335,37 @@ extern "C" void ast_destroy(ast_ctx* c)
 
 extern "C" void* ast_stream(ast_ctx* c) { return c ? (void*)c->stream : nullptr; }
 
+// Lanes a vector in FP64 by the number of vectors (0: one thread each, eval_kernel).  A warp alone on its
+// quarter of the SM costs its FP64 instructions times 64 cycles, four on an SM 19 each (group64.cuh):
+// eight lanes a vector need 2.2 to 3 times fewer, so they win until the SMs hold four such warps
+// twice over; from there the FP64 unit is full either way and threads do the least.  Thirty-two
+// lanes share the magnitudes of four times as many observations and win while every vector still
+// has a quarter of an SM.
+static int eval_group(int64_t n, int sm_count)
+{
+    if (n <= 4 * (int64_t)sm_count) return 32;
+    if (n <= 32 * (int64_t)sm_count) return 8;
+    return 0;
+}
+
+template <class CF, int G>
+static int launch_eval_group(ast_ctx* c, const DevModel& dm, const double* d_params, int64_t n, double* d_chi2,
+                             double* d_dv, cudaStream_t s)
+{
+    eval_group_kernel<CF, G><<<(unsigned)((n * G + 31) / 32), 32, 0, s>>>(dm, c->d_obs, c->layout, d_params, n, d_chi2, d_dv);
+    AST_CUDA(cudaGetLastError());
+    return AST_OK;
+}
+
 template <class CF, int PREC>
 static int launch_eval(ast_ctx* c, const DevModel& dm, const double* d_params, int64_t n, double* d_chi2, double* d_dv,
                        cudaStream_t s, unsigned long long* d_err)
 {
+    if (PREC == AST_PREC_FP64) {
+        const int g = eval_group(n, c->sm_count);
+        if (g == 32) return launch_eval_group<CF, 32>(c, dm, d_params, n, d_chi2, d_dv, s);
+        if (g == 8) return launch_eval_group<CF, 8>(c, dm, d_params, n, d_chi2, d_dv, s);
+    }
     // As the fits (fit_launch_core): the precision's own shape when the vectors fill it, the full
     // register file when they do not (1001 vectors of 480 points, mixed: 1.19 ms against 1.33).
     constexpr int kFull = KernShape<PREC>::min_ctas;

@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(MINB == 3 ? 128 : 256, MINB) fit_kernel(DevMod
 // Per-group argmin over the chains' results (lowest chi^2, lowest chain on ties, as the serial
 // loop of cuda.c:1770-1782) and the stage hand-off or the final output (cuda.c:1785-1823).
 template <class CF>
-__global__ void group_best_kernel(DevModel M, FitView<CF> V, double* out_f, double* out_p, double* out_dv,
+__global__ void __launch_bounds__(256) group_best_kernel(DevModel M, FitView<CF> V, double* out_f, double* out_p, double* out_dv,
                                   const void* g_obs, ObsLayout L, int fp64_result)
 {
     const ObsView o = L.view(g_obs, M.n_data);

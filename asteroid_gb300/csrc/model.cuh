@@ -351,18 +351,81 @@ __device__ __forceinline__ void rk4_step(double* y, double h, const double* mu)
 
 // ------------------------------------------------------------------ chi^2, FP64
 
-// Per-observation brightness from body axes (a, b, c), unit E and S (cuda.c:475-689).
-struct Geometry {
+// Initial state, ODE constants and spin-axis frame of one parameter vector (cuda.c:195-252).
+struct Fp64Setup {
     double M_x, M_y, M_z, XM_x, XM_z, YM_x, YM_y, YM_z;
+    double y[6], mu[6];
+    double b_ph, c_ph, kappa;
+    bool torque, bw;
 };
 
-// chi2one (cuda.c:81-1011) for one parameter vector over the object's observations.
-// Returns CHI_FLOAT; delta_V is written only when the evaluation runs to the end (the NUDGE
-// "more than M_MAX minima" exit returns 1e30 and leaves it, as the reference does).
-// vmod_out, when non-null, receives the model magnitude of every observation (the reference's
-// Nplot > 0 mode, cuda.c:699-704, without the delta_V shift); ang_out the Euler angles
-// (phi, theta, psi) at every observation; geo_out the kAstGeo inputs of the ANIMATE renderer
-// at every observation (compute_rgb's arguments, cuda.c:576-586).
+__device__ __forceinline__ void fp64_setup(const DevModel& M, const double* params, Fp64Setup& S)
+{
+    const int flags = M.flags;
+    const ast_type_ids& T = M.t;
+#define AST_P(tt) params[M.idx[T.tt]]
+    const double th_M = AST_P(theta_M), ph_M = AST_P(phi_M);
+    const double M_x = sin(th_M) * cos(ph_M);
+    const double M_y = sin(th_M) * sin(ph_M);
+    const double M_z = cos(th_M);
+    const double XM = sqrt(M_z * M_z + M_x * M_x);
+    const double XM_x = M_z / XM;
+    const double XM_z = -M_x / XM;
+    S.M_x = M_x;
+    S.M_y = M_y;
+    S.M_z = M_z;
+    S.XM_x = XM_x;
+    S.XM_z = XM_z;
+    S.YM_x = M_y * XM_z;
+    S.YM_y = M_z * XM_x - M_x * XM_z;
+    S.YM_z = -M_y * XM_x;
+    const double bt = AST_P(b_tumb), ct = AST_P(c_tumb);
+    const double Is = (1.0 + bt * bt) / (bt * bt + ct * ct);
+    const double Ii = (1.0 + ct * ct) / (bt * bt + ct * ct);
+    const double Is_inv = 1.0 / Is;
+    const double Ii_inv = 1.0 / Ii;
+    const double psi0 = AST_P(psi_0);
+    S.torque = (flags & AST_TORQUE) != 0;
+    {
+        const double phi = AST_P(phi_0);
+        const double theta = asin(sqrt((AST_P(Es) - 1.0) / (sin(psi0) * sin(psi0) * (Ii_inv - Is_inv) + Is_inv - 1.0)));
+        const double psi = psi0;
+        if (S.torque) {
+            S.mu[0] = (Is - 1.0) * Ii_inv;
+            S.mu[1] = (1.0 - Ii) * Is_inv;
+            S.mu[2] = Ii - Is;
+            S.mu[3] = AST_P(Ti);
+            S.mu[4] = AST_P(Ts);
+            S.mu[5] = AST_P(Tl);
+            const double L = AST_P(L);
+            S.y[0] = L * Ii_inv * sin(theta) * sin(psi);
+            S.y[1] = L * Is_inv * sin(theta) * cos(psi);
+            S.y[2] = L * cos(theta);
+            S.y[3] = phi;
+            S.y[4] = theta;
+            S.y[5] = psi;
+        } else {
+            const double Ip = 0.5 * (Ii_inv + Is_inv);
+            const double Im = 0.5 * (Ii_inv - Is_inv);
+            S.mu[0] = AST_P(L);
+            S.mu[1] = Ip;
+            S.mu[2] = Im;
+            S.y[0] = phi;
+            S.y[1] = theta;
+            S.y[2] = psi;
+        }
+    }
+    S.b_ph = S.c_ph = S.kappa = 0;
+    S.bw = (flags & AST_BW_BALL) != 0;
+    if (S.bw) {
+        S.kappa = AST_P(kappa);
+    } else {
+        S.b_ph = (flags & AST_BC) ? AST_P(b) : bt;
+        S.c_ph = (flags & AST_BC) ? AST_P(c) : ct;
+    }
+}
+
+// Doubles of the renderer's geometry at one observation (compute_rgb's arguments, cuda.c:576-586).
 constexpr int kAstGeo = 20;
 
 __device__ __forceinline__ void write_geo(double* g, double b, double c, double Ex, double Ey, double Ez, double Epb,
@@ -379,216 +442,140 @@ __device__ __forceinline__ void write_geo(double* g, double b, double c, double 
     g[17] = ax; g[18] = ay; g[19] = az;
 }
 
-template <class CF>
-__device__ CF chi2_fp64(const DevModel& M, const ObsView& o, const double* params, CF* delta_V,
-                        double* vmod_out = nullptr, double* ang_out = nullptr, double* geo_out = nullptr)
+// Model magnitude at observation i for the Euler angles (phi, theta, psi): the body axes
+// (cuda.c:432-473), then the brightness (cuda.c:475-689).  geo, when non-null, receives the kAstGeo
+// inputs of the renderer.
+__device__ __forceinline__ double fp64_vmod(const DevModel& M, const double* params, const Fp64Setup& F, double phi,
+                                            double theta, double psi, const ObsView& o, int i, double* geo)
 {
-    const int flags = M.flags;
     const ast_type_ids& T = M.t;
-    const int N_data = M.n_data, N_filters = M.n_filters;
-    double sum_y2[AST_MAX_FILTERS], sum_y[AST_MAX_FILTERS], sum_w[AST_MAX_FILTERS];
-    for (int m = 0; m < N_filters; m++) { sum_y2[m] = 0.0; sum_y[m] = 0.0; sum_w[m] = 0.0; }
-    int Mmin = 0;
-    float t_mod[AST_M_MAX], V_mod[AST_M_MAX];
-    float t_old[2] = {0.f, 0.f}, V_old[2] = {0.f, 0.f};
+    const double M_x = F.M_x, M_y = F.M_y, M_z = F.M_z;
+    const double XM_x = F.XM_x, XM_z = F.XM_z, YM_x = F.YM_x, YM_y = F.YM_y, YM_z = F.YM_z;
+    double cos_phi, sin_phi;
+    sincos(phi, &sin_phi, &cos_phi);
+    double N_x = XM_x * cos_phi + YM_x * sin_phi;
+    double N_y = YM_y * sin_phi;
+    double N_z = XM_z * cos_phi + YM_z * sin_phi;
+    double p_x = N_y * M_z - N_z * M_y;
+    double p_y = N_z * M_x - N_x * M_z;
+    double p_z = N_x * M_y - N_y * M_x;
+    double cos_theta, sin_theta;
+    sincos(theta, &sin_theta, &cos_theta);
+    double a_x = M_x * cos_theta + p_x * sin_theta;
+    double a_y = M_y * cos_theta + p_y * sin_theta;
+    double a_z = M_z * cos_theta + p_z * sin_theta;
+    const double w_x = a_y * N_z - a_z * N_y;
+    const double w_y = a_z * N_x - a_x * N_z;
+    const double w_z = a_x * N_y - a_y * N_x;
+    double sin_psi, cos_psi;
+    sincos(psi, &sin_psi, &cos_psi);
+    const double b_x = N_x * cos_psi + w_x * sin_psi;
+    const double b_y = N_y * cos_psi + w_y * sin_psi;
+    const double b_z = N_z * cos_psi + w_z * sin_psi;
+    const double c_x = a_y * b_z - a_z * b_y;
+    const double c_y = a_z * b_x - a_x * b_z;
+    const double c_z = a_x * b_y - a_y * b_x;
 
-#define AST_P(tt) params[M.idx[T.tt]]
-    const double th_M = AST_P(theta_M), ph_M = AST_P(phi_M);
-    const double M_x = sin(th_M) * cos(ph_M);
-    const double M_y = sin(th_M) * sin(ph_M);
-    const double M_z = cos(th_M);
-    const double XM = sqrt(M_z * M_z + M_x * M_x);
-    const double XM_x = M_z / XM;
-    const double XM_z = -M_x / XM;
-    const double YM_x = M_y * XM_z;
-    const double YM_y = M_z * XM_x - M_x * XM_z;
-    const double YM_z = -M_y * XM_x;
-    const double bt = AST_P(b_tumb), ct = AST_P(c_tumb);
-    const double Is = (1.0 + bt * bt) / (bt * bt + ct * ct);
-    const double Ii = (1.0 + ct * ct) / (bt * bt + ct * ct);
-    const double Is_inv = 1.0 / Is;
-    const double Ii_inv = 1.0 / Ii;
-    const double psi0 = AST_P(psi_0);
-    double y[6];
-    double mu[6];
-    const bool torque = (flags & AST_TORQUE) != 0;
-    {
-        const double phi = AST_P(phi_0);
-        const double theta = asin(sqrt((AST_P(Es) - 1.0) / (sin(psi0) * sin(psi0) * (Ii_inv - Is_inv) + Is_inv - 1.0)));
-        const double psi = psi0;
-        if (torque) {
-            mu[0] = (Is - 1.0) * Ii_inv;
-            mu[1] = (1.0 - Ii) * Is_inv;
-            mu[2] = Ii - Is;
-            mu[3] = AST_P(Ti);
-            mu[4] = AST_P(Ts);
-            mu[5] = AST_P(Tl);
-            const double L = AST_P(L);
-            y[0] = L * Ii_inv * sin(theta) * sin(psi);
-            y[1] = L * Is_inv * sin(theta) * cos(psi);
-            y[2] = L * cos(theta);
-            y[3] = phi;
-            y[4] = theta;
-            y[5] = psi;
-        } else {
-            const double Ip = 0.5 * (Ii_inv + Is_inv);
-            const double Im = 0.5 * (Ii_inv - Is_inv);
-            mu[0] = AST_P(L);
-            mu[1] = Ip;
-            mu[2] = Im;
-            y[0] = phi;
-            y[1] = theta;
-            y[2] = psi;
-        }
-    }
-    double b_ph = 0, c_ph = 0, kappa = 0, cos_phR = 0, sin_phR = 0, cos_thR = 0, sin_thR = 0;
-    const bool bw = (flags & AST_BW_BALL) != 0;
-    if (bw) {
-        kappa = AST_P(kappa);
+    const double E_x1 = o.ex[i], E_y1 = o.ey[i], E_z1 = o.ez[i];
+    const double S_x1 = o.sx[i], S_y1 = o.sy[i], S_z1 = o.sz[i];
+    double Vmod;
+    if (F.bw) {
+        // Brightness frame rotated by theta_R, phi_R (cuda.c:475-497), then the
+        // black-and-white ball (cuda.c:596-607).
+        double cos_phR, sin_phR, cos_thR, sin_thR;
+        sincos(AST_P(phi_R), &sin_phR, &cos_phR);
+        sincos(AST_P(theta_R), &sin_thR, &cos_thR);
+        N_x = b_x * cos_phR + c_x * sin_phR;
+        N_y = b_y * cos_phR + c_y * sin_phR;
+        N_z = b_z * cos_phR + c_z * sin_phR;
+        p_x = N_y * a_z - N_z * a_y;
+        p_y = N_z * a_x - N_x * a_z;
+        p_z = N_x * a_y - N_y * a_x;
+        a_x = a_x * cos_thR + p_x * sin_thR;
+        a_y = a_y * cos_thR + p_y * sin_thR;
+        a_z = a_z * cos_thR + p_z * sin_thR;
+        const double Ep_a = a_x * E_x1 + a_y * E_y1 + a_z * E_z1;
+        if (geo)
+            write_geo(geo, AST_P(b_tumb), AST_P(c_tumb), E_x1, E_y1, E_z1, b_x * E_x1 + b_y * E_y1 + b_z * E_z1,
+                      c_x * E_x1 + c_y * E_y1 + c_z * E_z1, Ep_a, b_x * S_x1 + b_y * S_y1 + b_z * S_z1,
+                      c_x * S_x1 + c_y * S_y1 + c_z * S_z1, a_x * S_x1 + a_y * S_y1 + a_z * S_z1, b_x, b_y, b_z,
+                      c_x, c_y, c_z, a_x, a_y, a_z);
+        const double cos_zeta = Ep_a;
+        Vmod = -2.5 * log10(0.5 * (F.kappa * (1 + cos_zeta) + 0.5 * (1 - cos_zeta)));
     } else {
-        b_ph = (flags & AST_BC) ? AST_P(b) : bt;
-        c_ph = (flags & AST_BC) ? AST_P(c) : ct;
+        const double Ep_b = b_x * E_x1 + b_y * E_y1 + b_z * E_z1;
+        const double Ep_c = c_x * E_x1 + c_y * E_y1 + c_z * E_z1;
+        const double Ep_a = a_x * E_x1 + a_y * E_y1 + a_z * E_z1;
+        const double Sp_b = b_x * S_x1 + b_y * S_y1 + b_z * S_z1;
+        const double Sp_c = c_x * S_x1 + c_y * S_y1 + c_z * S_z1;
+        const double Sp_a = a_x * S_x1 + a_y * S_y1 + a_z * S_z1;
+        // Lommel-Seeliger ellipsoid, Muinonen & Lumme (2015) eqs. 10-14 (cuda.c:664-689).
+        const double b = F.b_ph, c = F.c_ph;
+        if (geo)
+            write_geo(geo, b, c, E_x1, E_y1, E_z1, Ep_b, Ep_c, Ep_a, Sp_b, Sp_c, Sp_a,
+                      b_x, b_y, b_z, c_x, c_y, c_z, a_x, a_y, a_z);
+        const double scalar_Sun = sqrt(Sp_b * Sp_b / (b * b) + Sp_c * Sp_c / (c * c) + Sp_a * Sp_a);
+        const double scalar_Earth = sqrt(Ep_b * Ep_b / (b * b) + Ep_c * Ep_c / (c * c) + Ep_a * Ep_a);
+        const double cos_alpha_p = (Sp_b * Ep_b / (b * b) + Sp_c * Ep_c / (c * c) + Sp_a * Ep_a) / (scalar_Sun * scalar_Earth);
+        const double sin_alpha_p = sqrt(1.0 - cos_alpha_p * cos_alpha_p);
+        const double alpha_p = atan2(sin_alpha_p, cos_alpha_p);
+        const double scalar = sqrt(scalar_Sun * scalar_Sun + scalar_Earth * scalar_Earth + 2 * scalar_Sun * scalar_Earth * cos_alpha_p);
+        const double cos_lambda_p = (scalar_Sun + scalar_Earth * cos_alpha_p) / scalar;
+        const double sin_lambda_p = scalar_Earth * sin_alpha_p / scalar;
+        const double lambda_p = atan2(sin_lambda_p, cos_lambda_p);
+        Vmod = -2.5 * log10(b * c * scalar_Sun * scalar_Earth / scalar *
+                            (cos(lambda_p - alpha_p) + cos_lambda_p +
+                             sin_lambda_p * sin(lambda_p - alpha_p) * log(1.0 / tan(0.5 * lambda_p) / tan(0.5 * (alpha_p - lambda_p)))));
     }
-
-    for (int i = 0; i < N_data; i++) {
-        if (i > 0) {
-            const int N_steps = o.nst[i];
-            const double h = o.h[i];
-            if (torque) {
-#pragma unroll 1
-                for (int l = 0; l < N_steps; l++) rk4_step<6>(y, h, mu);
-            } else {
-#pragma unroll 1
-                for (int l = 0; l < N_steps; l++) rk4_step<3>(y, h, mu);
-            }
-        }
-        const double phi = torque ? y[3] : y[0];
-        const double theta = torque ? y[4] : y[1];
-        const double psi = torque ? y[5] : y[2];
-        if (ang_out) {
-            ang_out[3 * i] = phi;
-            ang_out[3 * i + 1] = theta;
-            ang_out[3 * i + 2] = psi;
-        }
-
-        double cos_phi, sin_phi;
-        sincos(phi, &sin_phi, &cos_phi);
-        double N_x = XM_x * cos_phi + YM_x * sin_phi;
-        double N_y = YM_y * sin_phi;
-        double N_z = XM_z * cos_phi + YM_z * sin_phi;
-        double p_x = N_y * M_z - N_z * M_y;
-        double p_y = N_z * M_x - N_x * M_z;
-        double p_z = N_x * M_y - N_y * M_x;
-        double cos_theta, sin_theta;
-        sincos(theta, &sin_theta, &cos_theta);
-        double a_x = M_x * cos_theta + p_x * sin_theta;
-        double a_y = M_y * cos_theta + p_y * sin_theta;
-        double a_z = M_z * cos_theta + p_z * sin_theta;
-        const double w_x = a_y * N_z - a_z * N_y;
-        const double w_y = a_z * N_x - a_x * N_z;
-        const double w_z = a_x * N_y - a_y * N_x;
-        double sin_psi, cos_psi;
-        sincos(psi, &sin_psi, &cos_psi);
-        const double b_x = N_x * cos_psi + w_x * sin_psi;
-        const double b_y = N_y * cos_psi + w_y * sin_psi;
-        const double b_z = N_z * cos_psi + w_z * sin_psi;
-        const double c_x = a_y * b_z - a_z * b_y;
-        const double c_y = a_z * b_x - a_x * b_z;
-        const double c_z = a_x * b_y - a_y * b_x;
-
-        const double E_x1 = o.ex[i], E_y1 = o.ey[i], E_z1 = o.ez[i];
-        const double S_x1 = o.sx[i], S_y1 = o.sy[i], S_z1 = o.sz[i];
-        double Vmod;
-        if (bw) {
-            // Brightness frame rotated by theta_R, phi_R (cuda.c:475-497), then the
-            // black-and-white ball (cuda.c:596-607).
-            sincos(AST_P(phi_R), &sin_phR, &cos_phR);
-            sincos(AST_P(theta_R), &sin_thR, &cos_thR);
-            N_x = b_x * cos_phR + c_x * sin_phR;
-            N_y = b_y * cos_phR + c_y * sin_phR;
-            N_z = b_z * cos_phR + c_z * sin_phR;
-            p_x = N_y * a_z - N_z * a_y;
-            p_y = N_z * a_x - N_x * a_z;
-            p_z = N_x * a_y - N_y * a_x;
-            a_x = a_x * cos_thR + p_x * sin_thR;
-            a_y = a_y * cos_thR + p_y * sin_thR;
-            a_z = a_z * cos_thR + p_z * sin_thR;
-            const double Ep_a = a_x * E_x1 + a_y * E_y1 + a_z * E_z1;
-            if (geo_out)
-                write_geo(geo_out + (int64_t)kAstGeo * i, bt, ct, E_x1, E_y1, E_z1, b_x * E_x1 + b_y * E_y1 + b_z * E_z1,
-                          c_x * E_x1 + c_y * E_y1 + c_z * E_z1, Ep_a, b_x * S_x1 + b_y * S_y1 + b_z * S_z1,
-                          c_x * S_x1 + c_y * S_y1 + c_z * S_z1, a_x * S_x1 + a_y * S_y1 + a_z * S_z1, b_x, b_y, b_z,
-                          c_x, c_y, c_z, a_x, a_y, a_z);
-            const double cos_zeta = Ep_a;
-            Vmod = -2.5 * log10(0.5 * (kappa * (1 + cos_zeta) + 0.5 * (1 - cos_zeta)));
-        } else {
-            const double Ep_b = b_x * E_x1 + b_y * E_y1 + b_z * E_z1;
-            const double Ep_c = c_x * E_x1 + c_y * E_y1 + c_z * E_z1;
-            const double Ep_a = a_x * E_x1 + a_y * E_y1 + a_z * E_z1;
-            const double Sp_b = b_x * S_x1 + b_y * S_y1 + b_z * S_z1;
-            const double Sp_c = c_x * S_x1 + c_y * S_y1 + c_z * S_z1;
-            const double Sp_a = a_x * S_x1 + a_y * S_y1 + a_z * S_z1;
-            // Lommel-Seeliger ellipsoid, Muinonen & Lumme (2015) eqs. 10-14 (cuda.c:664-689).
-            const double b = b_ph, c = c_ph;
-            if (geo_out)
-                write_geo(geo_out + (int64_t)kAstGeo * i, b, c, E_x1, E_y1, E_z1, Ep_b, Ep_c, Ep_a, Sp_b, Sp_c, Sp_a,
-                          b_x, b_y, b_z, c_x, c_y, c_z, a_x, a_y, a_z);
-            const double scalar_Sun = sqrt(Sp_b * Sp_b / (b * b) + Sp_c * Sp_c / (c * c) + Sp_a * Sp_a);
-            const double scalar_Earth = sqrt(Ep_b * Ep_b / (b * b) + Ep_c * Ep_c / (c * c) + Ep_a * Ep_a);
-            const double cos_alpha_p = (Sp_b * Ep_b / (b * b) + Sp_c * Ep_c / (c * c) + Sp_a * Ep_a) / (scalar_Sun * scalar_Earth);
-            const double sin_alpha_p = sqrt(1.0 - cos_alpha_p * cos_alpha_p);
-            const double alpha_p = atan2(sin_alpha_p, cos_alpha_p);
-            const double scalar = sqrt(scalar_Sun * scalar_Sun + scalar_Earth * scalar_Earth + 2 * scalar_Sun * scalar_Earth * cos_alpha_p);
-            const double cos_lambda_p = (scalar_Sun + scalar_Earth * cos_alpha_p) / scalar;
-            const double sin_lambda_p = scalar_Earth * sin_alpha_p / scalar;
-            const double lambda_p = atan2(sin_lambda_p, cos_lambda_p);
-            Vmod = -2.5 * log10(b * c * scalar_Sun * scalar_Earth / scalar *
-                                (cos(lambda_p - alpha_p) + cos_lambda_p +
-                                 sin_lambda_p * sin(lambda_p - alpha_p) * log(1.0 / tan(0.5 * lambda_p) / tan(0.5 * (alpha_p - lambda_p)))));
-        }
-        if (vmod_out) vmod_out[i] = Vmod;
-
-        {   // Per-filter sums (cuda.c:707-714).
-            const int m = o.f[i];
-            const double yv = o.v[i] - Vmod;
-            const float wi = o.w[i];
-            sum_y2[m] = sum_y2[m] + yv * yv * wi;
-            sum_y[m] = sum_y[m] + yv * wi;
-            sum_w[m] = sum_w[m] + wi;
-        }
-
-        if (flags & AST_NUDGE) {
-            // Model minima (V maxima) near the observed ones (cuda.c:716-760).
-            if (i < 2) {
-                t_old[i] = (float)o.t[i];
-                V_old[i] = (float)Vmod;
-            } else {
-                if (V_old[1] > V_old[0] && V_old[1] >= Vmod) {
-                    bool local = false;
-                    for (int ii = 0; ii < M.n_min; ii++)
-                        if (fabsf(t_old[1] - M.t_min[ii]) < AST_DT_MAX2) local = true;
-                    if (local) {
-                        Mmin++;
-                        if (Mmin > AST_M_MAX) return (CF)kHuge;
-                        const double ti = o.t[i];
-                        const double a = ((Vmod - V_old[1]) / (ti - t_old[1]) - (V_old[1] - V_old[0]) / (t_old[1] - t_old[0])) / (ti - t_old[0]);
-                        const double b = (V_old[1] - V_old[0]) / (t_old[1] - t_old[0]) - a * (t_old[1] + t_old[0]);
-                        const double c = V_old[1] - a * t_old[1] * t_old[1] - b * t_old[1];
-                        t_mod[Mmin - 1] = (float)(-b / 2.0 / a);
-                        V_mod[Mmin - 1] = (float)(a * t_mod[Mmin - 1] * t_mod[Mmin - 1] + b * t_mod[Mmin - 1] + c);
-                    }
-                }
-                t_old[0] = t_old[1];
-                V_old[0] = V_old[1];
-                t_old[1] = (float)o.t[i];
-                V_old[1] = (float)Vmod;
-            }
-        }
-    }
+    return Vmod;
+}
 #undef AST_P
 
-    // Per-filter chi^2 and delta_V (cuda.c:887-910); under RMSD the root of the summed chi^2 over
-    // the summed weights (cuda.c:890,901-908).
+// Model minima (V maxima) near the observed ones, observation by observation (cuda.c:716-760).
+struct Fp64Minima {
+    int n = 0;
+    float t_mod[AST_M_MAX], V_mod[AST_M_MAX];
+    float t_old[2] = {0.f, 0.f}, V_old[2] = {0.f, 0.f};
+};
+// Observation i at time ti with model magnitude Vmod; false once there are more than M_MAX minima.
+__device__ __forceinline__ bool fp64_minima(const DevModel& M, Fp64Minima& Q, int i, double ti, double Vmod)
+{
+    float* t_old = Q.t_old;
+    float* V_old = Q.V_old;
+    if (i < 2) {
+        t_old[i] = (float)ti;
+        V_old[i] = (float)Vmod;
+        return true;
+    }
+    if (V_old[1] > V_old[0] && V_old[1] >= Vmod) {
+        bool local = false;
+        for (int ii = 0; ii < M.n_min; ii++)
+            if (fabsf(t_old[1] - M.t_min[ii]) < AST_DT_MAX2) local = true;
+        if (local) {
+            Q.n++;
+            if (Q.n > AST_M_MAX) return false;
+            const double a = ((Vmod - V_old[1]) / (ti - t_old[1]) - (V_old[1] - V_old[0]) / (t_old[1] - t_old[0])) / (ti - t_old[0]);
+            const double b = (V_old[1] - V_old[0]) / (t_old[1] - t_old[0]) - a * (t_old[1] + t_old[0]);
+            const double c = V_old[1] - a * t_old[1] * t_old[1] - b * t_old[1];
+            const int m = Q.n - 1;
+            Q.t_mod[m] = (float)(-b / 2.0 / a);
+            Q.V_mod[m] = (float)(a * Q.t_mod[m] * Q.t_mod[m] + b * Q.t_mod[m] + c);
+        }
+    }
+    t_old[0] = t_old[1];
+    V_old[0] = V_old[1];
+    t_old[1] = (float)ti;
+    V_old[1] = (float)Vmod;
+    return true;
+}
+
+// Per-filter chi^2 and delta_V (cuda.c:887-910); under RMSD the root of the summed chi^2 over the
+// summed weights (cuda.c:890,901-908).  Then the reward and punishment factors of the minima.
+template <class CF>
+__device__ __forceinline__ CF fp64_finish(const DevModel& M, const double* sum_y2, const double* sum_y,
+                                          const double* sum_w, const Fp64Minima& Q, CF* delta_V)
+{
+    const int N_filters = M.n_filters;
     CF chi2m, chi2a = 0.0, SUM_w = 0.0;
     CF dv[AST_MAX_FILTERS];
     for (int m = 0; m < N_filters; m++) {
@@ -597,25 +584,25 @@ __device__ CF chi2_fp64(const DevModel& M, const ObsView& o, const double* param
         dv[m] = (CF)(sum_y[m] / sum_w[m]);
         SUM_w = (CF)((double)SUM_w + sum_w[m]);
     }
-    if (flags & AST_RMSD)
+    if (M.flags & AST_RMSD)
         chi2a = sqrt(chi2a / SUM_w);
     else
-        chi2a = chi2a / (CF)(N_data - M.n_params - N_filters);
+        chi2a = chi2a / (CF)(M.n_data - M.n_params - N_filters);
 
-    if (flags & AST_NUDGE) {
+    if (M.flags & AST_NUDGE) {
         // Reward and punishment factors (cuda.c:912-993).
         float S_M = 0.0f;
         float P_tot = 1.0f;
-        for (int imod = 0; imod < Mmin; imod++) {
+        for (int imod = 0; imod < Q.n; imod++) {
             for (int iobs = 0; iobs < M.n_min; iobs++) {
-                const float dt = fabsf(t_mod[imod] - M.t_min[iobs]);
+                const float dt = fabsf(Q.t_mod[imod] - M.t_min[iobs]);
                 if (dt < AST_DT_MAX2) {
                     if (dt > AST_DT_MAX) {
                         const float x = (AST_DT_MAX2 - dt) / (AST_DT_MAX2 - AST_DT_MAX);
                         S_M = (float)(S_M + x * x * (-2.0 * x + 3.0));
                     } else {
                         S_M = (float)(S_M + 1.0);
-                        const float dV = (float)(V_mod[imod] + dv[0] - M.v_min[iobs]);
+                        const float dV = (float)(Q.V_mod[imod] + dv[0] - M.v_min[iobs]);
                         const float x = sqrtf(dt * dt / AST_DT_MAX / AST_DT_MAX + dV * dV / AST_DV_MAX / AST_DV_MAX);
                         if (x < 1.0f) {
                             const float P_i = AST_L_A * x * x / (x * x + AST_L_RC2);
@@ -646,6 +633,48 @@ __device__ CF chi2_fp64(const DevModel& M, const ObsView& o, const double* param
     }
     for (int m = 0; m < N_filters; m++) delta_V[m] = dv[m];
     return chi2a;
+}
+
+// chi2one (cuda.c:81-1011) for one parameter vector over the object's observations.
+// Returns CHI_FLOAT; delta_V is written only when the evaluation runs to the end (the NUDGE
+// "more than M_MAX minima" exit returns 1e30 and leaves it, as the reference does).
+template <class CF>
+__device__ CF chi2_fp64(const DevModel& M, const ObsView& o, const double* params, CF* delta_V)
+{
+    const int flags = M.flags;
+    const int N_data = M.n_data, N_filters = M.n_filters;
+    double sum_y2[AST_MAX_FILTERS], sum_y[AST_MAX_FILTERS], sum_w[AST_MAX_FILTERS];
+    for (int m = 0; m < N_filters; m++) { sum_y2[m] = 0.0; sum_y[m] = 0.0; sum_w[m] = 0.0; }
+    Fp64Minima Q;
+    Fp64Setup S;
+    fp64_setup(M, params, S);
+    for (int i = 0; i < N_data; i++) {
+        if (i > 0) {
+            const int N_steps = o.nst[i];
+            const double h = o.h[i];
+            if (S.torque) {
+#pragma unroll 1
+                for (int l = 0; l < N_steps; l++) rk4_step<6>(S.y, h, S.mu);
+            } else {
+#pragma unroll 1
+                for (int l = 0; l < N_steps; l++) rk4_step<3>(S.y, h, S.mu);
+            }
+        }
+        const double phi = S.torque ? S.y[3] : S.y[0];
+        const double theta = S.torque ? S.y[4] : S.y[1];
+        const double psi = S.torque ? S.y[5] : S.y[2];
+        const double Vmod = fp64_vmod(M, params, S, phi, theta, psi, o, i, nullptr);
+        {   // Per-filter sums (cuda.c:707-714).
+            const int m = o.f[i];
+            const double yv = o.v[i] - Vmod;
+            const float wi = o.w[i];
+            sum_y2[m] = sum_y2[m] + yv * yv * wi;
+            sum_y[m] = sum_y[m] + yv * wi;
+            sum_w[m] = sum_w[m] + wi;
+        }
+        if ((flags & AST_NUDGE) && !fp64_minima(M, Q, i, o.t[i], Vmod)) return (CF)kHuge;
+    }
+    return fp64_finish<CF>(M, sum_y2, sum_y, sum_w, Q, delta_V);
 }
 
 }  // namespace ast

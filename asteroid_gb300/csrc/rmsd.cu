@@ -68,13 +68,18 @@ __global__ void rmsd_setup_kernel(DevModel M, const void* g_obs, ObsLayout L, co
         trig_table_fill(trig, kTrigEntries<PREC>);
         __syncthreads();
     }
-    if (threadIdx.x != 0) return;
+    if (threadIdx.x >= (PREC == AST_PREC_FP64 ? 32 : 1)) return;
     const ObsView o = L.view(g_obs, M.n_data);
     double p[AST_MAX_PARAMS];
     for (int i = 0; i < M.n_params; i++) p[i] = p0[i];
-    params2x<CF>(M, p, x0);
     CF dv[AST_MAX_FILTERS];
-    const CF f0 = eval_point<CF, PREC>(M, o, p, dv, trig);
+    CF f0;
+    if (PREC == AST_PREC_FP64)
+        f0 = chi2_fp64_group<CF, 32>(M, o, p, dv);  // the warp together
+    else
+        f0 = eval_point<CF, PREC>(M, o, p, dv, trig);
+    if (threadIdx.x != 0) return;
+    params2x<CF>(M, p, x0);
     f01[0] = f0;
     f01[1] = f0 + f0 / sqrt((CF)(M.n_data - M.n_params - M.n_filters));
 }

@@ -9,6 +9,7 @@
 #pragma once
 #include <stdint.h>
 #include "asteroid_gb300.h"
+#include "group64.cuh"
 #include "mixed.cuh"
 #include "model.cuh"
 #include "philox.cuh"
@@ -386,7 +387,10 @@ __device__ void group_best_body(const DevModel& M, const FitView<CF>& V, int64_t
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) { sf[warp] = best; si[warp] = bi; }
     __syncthreads();
-    if (threadIdx.x != 0) return;
+    if (threadIdx.x >= 32) return;
+    // The first warp together: every lane the same, the first one writes.
+    best = sf[0];
+    bi = si[0];
     for (int w = 1; w < (int)(blockDim.x + 31) / 32; w++)
         if (sf[w] < best || (sf[w] == best && si[w] < bi)) { best = sf[w]; bi = si[w]; }
     // Strictly below 1e30, else the group's first chain (the reference's thread_min = 0).
@@ -400,19 +404,22 @@ __device__ void group_best_body(const DevModel& M, const FitView<CF>& V, int64_t
             x2params<CF>(M, 0, xb, p);
             params2x<CF>(M, p, xb);
         }
-        for (int i = 0; i < N; i++) V.group_x[g * N + i] = xb[i];
-    } else {
-        out_f[g] = best < kHuge ? best : kHuge;
-        double p[AST_MAX_PARAMS];
-        for (int i = 0; i < N; i++) p[i] = 0;
-        if (best < kHuge) x2params<CF>(M, V.reopt, xb, p);
-        if (fp64_obs && best < kHuge) {
-            double d[AST_MAX_FILTERS];
-            out_f[g] = (double)chi2_fp64<double>(M, *fp64_obs, p, d);
-        }
-        for (int i = 0; i < N; i++) out_p[g * N + i] = p[i];
-        for (int m = 0; m < NF; m++) out_dv[g * NF + m] = best < kHuge ? V.chain_dv[cb * NF + m] : 0.0;
+        if (threadIdx.x == 0)
+            for (int i = 0; i < N; i++) V.group_x[g * N + i] = xb[i];
+        return;
     }
+    double f = best < kHuge ? best : kHuge;
+    double p[AST_MAX_PARAMS];
+    for (int i = 0; i < N; i++) p[i] = 0;
+    if (best < kHuge) x2params<CF>(M, V.reopt, xb, p);
+    if (fp64_obs && best < kHuge) {
+        double d[AST_MAX_FILTERS];
+        f = chi2_fp64_group<double, 32>(M, *fp64_obs, p, d);
+    }
+    if (threadIdx.x != 0) return;
+    out_f[g] = f;
+    for (int i = 0; i < N; i++) out_p[g * N + i] = p[i];
+    for (int m = 0; m < NF; m++) out_dv[g * NF + m] = best < kHuge ? V.chain_dv[cb * NF + m] : 0.0;
 }
 
 
