@@ -335,19 +335,6 @@ extern "C" void ast_destroy(ast_ctx* c)
 
 extern "C" void* ast_stream(ast_ctx* c) { return c ? (void*)c->stream : nullptr; }
 
-// Lanes a vector in FP64 by the number of vectors (0: one thread each, eval_kernel).  A warp alone on its
-// quarter of the SM costs its FP64 instructions times 64 cycles, four on an SM 19 each (group64.cuh):
-// eight lanes a vector need 2.2 to 3 times fewer, so they win until the SMs hold four such warps
-// twice over; from there the FP64 unit is full either way and threads do the least.  Thirty-two
-// lanes share the magnitudes of four times as many observations and win while every vector still
-// has a quarter of an SM.
-static int eval_group(int64_t n, int sm_count)
-{
-    if (n <= 4 * (int64_t)sm_count) return 32;
-    if (n <= 32 * (int64_t)sm_count) return 8;
-    return 0;
-}
-
 template <class CF, int G>
 static int launch_eval_group(ast_ctx* c, const DevModel& dm, const double* d_params, int64_t n, double* d_chi2,
                              double* d_dv, cudaStream_t s)
@@ -362,7 +349,7 @@ static int launch_eval(ast_ctx* c, const DevModel& dm, const double* d_params, i
                        cudaStream_t s, unsigned long long* d_err)
 {
     if (PREC == AST_PREC_FP64) {
-        const int g = eval_group(n, c->sm_count);
+        const int g = group_lanes(n, c->sm_count);
         if (g == 32) return launch_eval_group<CF, 32>(c, dm, d_params, n, d_chi2, d_dv, s);
         if (g == 8) return launch_eval_group<CF, 8>(c, dm, d_params, n, d_chi2, d_dv, s);
     }

@@ -56,6 +56,7 @@ struct FitRun {
     int64_t n_evals = 0, n_fits = 0;
     double kernel_ms = 0;
     int tpb = 256, ctas = 0;
+    int lanes = 1;     // lanes of a slot (fit_group_kernel), 1: a thread each
     size_t smem = 0;   // dynamic shared memory of the launch (the observation block, or 0)
     int minb = 1;      // register budget variant of fit_kernel
 };
@@ -101,6 +102,17 @@ inline int obs_smem_for(K kern, size_t bytes, size_t optin, size_t* smem)
     AST_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     *smem = bytes;
     return AST_OK;
+}
+
+// Lanes an FP64 evaluation by the number that run side by side (1: one thread each).  A warp alone on its
+// quarter of the SM costs its FP64 instructions times 64 cycles, four on an SM 19 each (group64.cuh):
+// eight lanes an evaluation need 2.2 to 3 times fewer, so they win until the SMs hold four such
+// warps twice over; from there the FP64 unit is full either way and threads do the least.
+// Thirty-two lanes share the magnitudes of four times as many observations and win while every
+// evaluation still has a quarter of an SM.
+inline int group_lanes(int64_t n, int sm_count)
+{
+    return n <= 4 * (int64_t)sm_count ? 32 : n <= 32 * (int64_t)sm_count ? 8 : 1;
 }
 
 int build_dev_model(const ast_model* m, const ast_obs_set* obs, DevModel* dm);

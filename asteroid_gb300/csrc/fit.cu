@@ -95,6 +95,95 @@ __global__ void __launch_bounds__(MINB == 3 ? 128 : 256, MINB) fit_kernel(DevMod
     }
     bulk_drain(&bar, staged || !use_smem);
 }
+
+// fit_kernel with G lanes a slot, FP64 (group64.cuh): for fits of too few chains to fill the FP64 unit
+// with a thread each.  The lanes of a group evaluate together; the first one runs the simplex.
+template <class CF, int G>
+__global__ void __launch_bounds__(32, 8) fit_group_kernel(DevModel M, const void* g_obs, ObsLayout L, FitView<CF> V,
+                                                          int64_t budget)
+{
+    const ObsView o = L.view(g_obs, M.n_data);
+    const int64_t s = (blockIdx.x * (int64_t)32 + threadIdx.x) / G;
+    const bool leader = threadIdx.x % G == 0;
+    const bool slot = s < V.n_slots;
+    const int N = M.n_params, NF = M.n_filters;
+    const int64_t S = V.S;
+    SlotState<CF> R;
+    R.chain = -1;
+    R.st = R.l = R.ev = 0;
+    for (int m = 0; m < NF; m++) R.dvl[m] = (CF)0;
+    if (slot) {
+        R.chain = V.chain[s];
+        R.st = V.st[s];
+        R.l = V.it[s];
+        R.ev = V.ev[s];
+        for (int m = 0; m < NF; m++) R.dvl[m] = (CF)V.dv[(int64_t)m * S + s];
+    }
+    bool empty = !slot;  // nothing left for the group
+    unsigned long long n_ev = 0, n_fit = 0, n_done = 0;
+    for (int64_t used = 0; used < budget; used++) {
+        // The group's state on every lane; the simplex itself is in global memory, the first lane's.
+        const bool pull = R.chain < 0 && !empty;
+        unsigned long long c = 0;
+        if (pull && leader) c = atomicAdd(&V.ctr[0], 1ull);
+        c = __shfl_sync(0xffffffffu, c, 0, G);
+        if (pull) {
+            if (c >= (unsigned long long)V.n_chains) {
+                empty = true;
+            } else {
+                R.chain = (int64_t)c;
+                if (leader) start_chain<CF>(M, V, s, R.chain);
+                R.st = PH_INIT;
+                R.l = 0;
+                R.ev = 0;
+                for (int m = 0; m < NF; m++) R.dvl[m] = V.stage > 0 ? (CF)V.chain_dv[R.chain * NF + m] : (CF)0;
+            }
+        }
+        if (__all_sync(0xffffffffu, R.chain < 0)) break;
+        __syncwarp();
+        CF p[AST_MAX_PARAMS], dv[AST_MAX_FILTERS];
+        double params[AST_MAX_PARAMS];
+        for (int i = 0; i < N; i++) params[i] = 0.0;
+        int rej = 1;
+        if (R.chain >= 0) {
+            slot_point<CF>(M, V, s, R, p);
+            rej = x2params<CF>(M, V.reopt, p, params);
+        }
+        for (int m = 0; m < NF; m++) dv[m] = R.dvl[m];
+        __syncwarp();
+        // A group without a point takes part without a result.
+        CF fv = chi2_fp64_group<CF, G>(M, o, params, dv);
+        int finish = 0;
+        if (R.chain >= 0) {
+            if (rej) {
+                fv = (CF)kHuge;
+            } else {
+                for (int m = 0; m < NF; m++) R.dvl[m] = dv[m];
+                R.ev++;
+                n_ev++;
+            }
+            if (leader) finish = slot_apply<CF>(M, V, s, R, p, rej, fv, n_fit);
+        }
+        __syncwarp();
+        finish = __shfl_sync(0xffffffffu, finish, 0, G);
+        R.st = __shfl_sync(0xffffffffu, R.st, 0, G);
+        R.l = __shfl_sync(0xffffffffu, R.l, 0, G);
+        if (finish) {
+            n_done++;
+            R.chain = -1;
+        }
+    }
+    if (!slot || !leader) return;
+    V.chain[s] = R.chain;
+    V.st[s] = R.st;
+    V.it[s] = R.l;
+    V.ev[s] = R.ev;
+    for (int m = 0; m < NF; m++) V.dv[(int64_t)m * S + s] = (double)R.dvl[m];
+    if (n_done) atomicAdd(&V.ctr[1], n_done);
+    if (n_ev) atomicAdd(&V.ctr[2], n_ev);
+    if (n_fit) atomicAdd(&V.ctr[3], n_fit);
+}
+
 // Per-group argmin over the chains' results (lowest chi^2, lowest chain on ties, as the serial
 // loop of cuda.c:1770-1782) and the stage hand-off or the final output (cuda.c:1785-1823).
 template <class CF>
@@ -207,6 +296,22 @@ static decltype(&fit_kernel<CF, PREC, 1>) fit_kernel_ptr(int minb)
     return minb >= 3 ? fit_kernel<CF, PREC, 3> : minb == 2 ? fit_kernel<CF, PREC, 2> : fit_kernel<CF, PREC, 1>;
 }
 
+// The launch of one step: budget evaluations a slot.
+template <class CF, int PREC>
+static cudaError_t fit_launch(const FitRun& r, const DevModel& dm, const void* obs, const ObsLayout& L,
+                              const FitView<CF>& V, int64_t budget, cudaStream_t s)
+{
+    if (PREC == AST_PREC_FP64 && r.lanes == 32)
+        fit_group_kernel<CF, 32><<<r.ctas, r.tpb, 0, s>>>(dm, obs, L, V, budget);
+    else if (PREC == AST_PREC_FP64 && r.lanes == 8)
+        fit_group_kernel<CF, 8><<<r.ctas, r.tpb, 0, s>>>(dm, obs, L, V, budget);
+    else
+        fit_kernel_ptr<CF, PREC>(r.minb)<<<r.ctas, r.tpb, r.smem, s>>>(dm, obs, L, r.smem ? 1 : 0, V, budget);
+    return cudaGetLastError();
+}
+
+static int64_t fit_slots(const FitRun& r) { return (int64_t)r.tpb * r.ctas / r.lanes; }
+
 // Launch geometry: CTA size (tpb), register budget (minb) and whether the CTA stages the
 // observations in shared memory.  Staging is dropped when the block would lower the number of
 // CTAs an SM holds (observations are read once per observation, not per RK4 step, so global
@@ -216,6 +321,18 @@ template <class CF, int PREC>
 static int fit_launch_core(int sm_count, size_t obs_bytes, size_t optin, int tpb_req, int minb_req, int stage_req,
                            int64_t n_chains, FitRun* r)
 {
+    // FP64 with no geometry asked for: lane groups while they are faster (group_lanes).
+    r->lanes = 1;
+    if (PREC == AST_PREC_FP64 && tpb_req <= 0 && minb_req <= 0 && stage_req == 0) {
+        r->lanes = group_lanes(n_chains, sm_count);
+        if (r->lanes > 1) {
+            r->tpb = 32;
+            r->ctas = (int)((n_chains * r->lanes + 31) / 32);
+            r->smem = 0;
+            r->minb = 1;
+            return AST_OK;
+        }
+    }
     // Register budget: 1 (255 registers, CTAs of up to 256), 2 (128), 3 (170, CTAs of up to 128).
     // Unset, the kernel's own shape (KernShape) when the chains fill it -- 3 for the double-float
     // path -- and the full register file when they do not: with fewer chains than three CTAs of
@@ -296,7 +413,7 @@ extern "C" int ast_fit_begin(ast_ctx* c, const ast_fit_cfg* cfg)
              : pr == AST_PREC_MIXED_RHS32 ? fit_launch_cfg<float, AST_PREC_MIXED_RHS32>(c, cfg->tpb, mb, so, cfg->n_chains, &r)
                                         : fit_launch_cfg<float, AST_PREC_MIXED>(c, cfg->tpb, mb, so, cfg->n_chains, &r);
     if (rc) return rc;
-    const int64_t slots = (int64_t)r.tpb * r.ctas;
+    const int64_t slots = fit_slots(r);
     const int64_t groups = cfg->n_chains / cfg->group_size;
     if ((rc = fit_alloc(c, slots, cfg->n_chains, groups, cfb))) return rc;
     FitBuffers& b = c->fb;
@@ -330,8 +447,7 @@ static int fit_step_t(ast_ctx* c, int64_t budget, int32_t* done, cudaStream_t s)
     FitBuffers& b = c->fb;
     FitView<CF> V = make_view<CF>(c);
     AST_CUDA(cudaEventRecord(c->ev0, s));
-    fit_kernel_ptr<CF, PREC>(r.minb)<<<r.ctas, r.tpb, r.smem, s>>>(c->dm, c->d_obs, c->layout, r.smem ? 1 : 0, V, budget);
-    AST_CUDA(cudaGetLastError());
+    AST_CUDA((fit_launch<CF, PREC>(r, c->dm, c->d_obs, c->layout, V, budget, s)));
     AST_CUDA(cudaEventRecord(c->ev1, s));
     unsigned long long h[8];
     AST_CUDA(cudaMemcpyAsync(h, b.ctr, sizeof(h), cudaMemcpyDeviceToHost, s));
@@ -556,7 +672,7 @@ static int noalloc_run(const DevModel& dm, char* base, const int64_t* off, const
                        int64_t S, const FitRun& r, double* d_best_f, double* d_best_params, double* d_best_dv,
                        cudaStream_t s)
 {
-    const int64_t slots = (int64_t)r.tpb * r.ctas;
+    const int64_t slots = fit_slots(r);
     const int N = dm.n_params, NF = dm.n_filters;
     const int64_t C = cfg->n_chains, G = C / cfg->group_size;
     FitView<CF> V;
@@ -584,9 +700,7 @@ static int noalloc_run(const DevModel& dm, char* base, const int64_t* off, const
     for (int32_t stage = 0; stage < cfg->n_stages; stage++) {
         V.stage = stage;
         V.last_stage = stage == cfg->n_stages - 1;
-        fit_kernel_ptr<CF, PREC>(r.minb)<<<r.ctas, r.tpb, r.smem, s>>>(dm, base + off[0], L, r.smem ? 1 : 0, V,
-                                                                       INT64_MAX);
-        AST_CUDA(cudaGetLastError());
+        AST_CUDA((fit_launch<CF, PREC>(r, dm, base + off[0], L, V, INT64_MAX, s)));
         unsigned long long h[8];
         AST_CUDA(cudaMemcpyAsync(h, V.ctr, sizeof(h), cudaMemcpyDeviceToHost, s));
         AST_CUDA(cudaStreamSynchronize(s));
@@ -664,7 +778,7 @@ extern "C" int ast_fit_noalloc(const ast_model* model, const ast_obs_set* obs, c
                  ? fit_launch_core<float, AST_PREC_FP64>(sms, L.bytes, optin, cfg->tpb, cfg->min_ctas_per_sm, cfg->stage_obs, cfg->n_chains, &r)
                  : fit_launch_core<float, AST_PREC_MIXED>(sms, L.bytes, optin, cfg->tpb, cfg->min_ctas_per_sm, cfg->stage_obs, cfg->n_chains, &r);
     if (rc) return rc;
-    const int64_t slots = (int64_t)r.tpb * r.ctas, S = (slots + 31) / 32 * 32;
+    const int64_t slots = fit_slots(r), S = (slots + 31) / 32 * 32;
     int64_t off[20];
     const int64_t bytes = noalloc_layout(S, cfg->n_chains, cfg->n_chains / cfg->group_size, N, NF, cfb, L.bytes, off);
     if (bytes > (int64_t)AST_NOALLOC_SCRATCH_BYTES)

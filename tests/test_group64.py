@@ -64,3 +64,28 @@ def test_lane_groups_equal_threads(gpu, flags, n, filters, span):
         assert np.array_equal(c, chi2[: len(some)], equal_nan=True)
         assert np.array_equal(d, dv[: len(some)], equal_nan=True)
     assert np.isfinite(chi2[np.isfinite(chi2)]).sum() > 0.3 * len(chi2)
+
+
+@pytest.mark.parametrize("flags,chains,group,kw", [
+    ("TORQUE,P_PSI,ACC", 1, 1, {}), ("TORQUE,P_PSI", 33, 33, dict(n_stages=2)), ("BC,INTERP,ACC", 700, 7, {}),
+    ("TORQUE,INTERP,ACC,NUDGE", 640, 64, dict(reopt=True)), ("BW_BALL,ACC", 4000, 250, dict(evals_cap=16))])
+def test_fits_by_lane_groups_equal_threads(gpu, flags, chains, group, kw):
+    """A fit of few chains runs by lane groups unless a geometry is asked for; both give the same chains."""
+    model, obs, P = _object(flags, 48, 2, 5, 1.0)
+    kw = dict(dict(evals_cap=40, n_stages=1), **kw)
+    if kw.get("reopt"):
+        kw["params0"] = P[0]
+    with api.Engine(model, obs) as eng:
+        a = eng.fit(n_chains=chains, group_size=group, seed=9, **kw)
+        lanes_ctas = eng.fit_launch()["ctas"]
+        b = eng.fit(n_chains=chains, group_size=group, seed=9, tpb=32, **kw)
+        assert lanes_ctas > eng.fit_launch()["ctas"] or chains == 1
+        eng.fit_begin(n_chains=chains, group_size=group, seed=9, **kw)  # in bounded steps
+        for _ in range(1000):
+            if eng.fit_step(3):
+                break
+        c = eng.fit_end()
+    for r in (a, c):
+        for k in ("best_f", "best_params", "best_dv", "chain_f"):
+            assert np.array_equal(getattr(r, k), getattr(b, k), equal_nan=True), k
+        assert r.n_evals == b.n_evals and r.n_fits == b.n_fits
