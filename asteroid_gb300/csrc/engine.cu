@@ -352,6 +352,13 @@ static int launch_eval(ast_ctx* c, const DevModel& dm, const double* d_params, i
         const int g = group_lanes(n, c->sm_count);
         if (g == 32) return launch_eval_group<CF, 32>(c, dm, d_params, n, d_chi2, d_dv, s);
         if (g == 8) return launch_eval_group<CF, 8>(c, dm, d_params, n, d_chi2, d_dv, s);
+        // The FP64 unit is the SM's: an SM takes its warps' instructions one after the other, so the
+        // call takes as long as the SM with the most warps.  One-warp CTAs, all in the grid, spread
+        // evenly (20 011 vectors: 5 warps on the fullest SM; CTAs of 128 put 8 on five of them).
+        eval_kernel<CF, PREC, KernShape<PREC>::min_ctas><<<(unsigned)((n + 31) / 32), 32, 0, s>>>(
+            dm, c->d_obs, c->layout, 0, d_params, n, d_chi2, d_dv, d_err);
+        AST_CUDA(cudaGetLastError());
+        return AST_OK;
     }
     // As the fits (fit_launch_core): the precision's own shape when the vectors fill it, the full
     // register file when they do not (1001 vectors of 480 points, mixed: 1.19 ms against 1.33).

@@ -352,9 +352,12 @@ static int fit_launch_core(int sm_count, size_t obs_bytes, size_t optin, int tpb
     if (tpb <= 0) {
         // Enough CTAs to cover every SM before growing the CTA (small chain counts).
         int64_t per_sm = n_chains / (sm_count > 0 ? sm_count : 1);
+        // FP64: one-warp CTAs until the chains fill the SMs -- the SM with the most warps sets the time
+        // (the FP64 unit is the SM's), and small CTAs spread evenly.
         const int tpb_max = minb == 3 ? 128 : 256;
         tpb = 32;
-        while (tpb < tpb_max && tpb * 2 <= per_sm) tpb *= 2;
+        if (PREC != AST_PREC_FP64 || per_sm >= tpb_max)
+            while (tpb < tpb_max && tpb * 2 <= per_sm) tpb *= 2;
     }
     if (tpb < 32 || tpb > 256 || (tpb & 31)) return ast_set_error(AST_E_INVALID, "fit: tpb must be 32..256, multiple of 32");
     int occ_smem = 0, occ_gmem = 0;

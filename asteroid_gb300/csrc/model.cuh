@@ -356,6 +356,7 @@ struct Fp64Setup {
     double M_x, M_y, M_z, XM_x, XM_z, YM_x, YM_y, YM_z;
     double y[6], mu[6];
     double b_ph, c_ph, kappa;
+    double cos_phR, sin_phR, cos_thR, sin_thR;  // BW_BALL's brightness frame
     bool torque, bw;
 };
 
@@ -415,10 +416,12 @@ __device__ __forceinline__ void fp64_setup(const DevModel& M, const double* para
             S.y[2] = psi;
         }
     }
-    S.b_ph = S.c_ph = S.kappa = 0;
+    S.b_ph = S.c_ph = S.kappa = S.cos_phR = S.sin_phR = S.cos_thR = S.sin_thR = 0;
     S.bw = (flags & AST_BW_BALL) != 0;
     if (S.bw) {
         S.kappa = AST_P(kappa);
+        sincos(AST_P(phi_R), &S.sin_phR, &S.cos_phR);
+        sincos(AST_P(theta_R), &S.sin_thR, &S.cos_thR);
     } else {
         S.b_ph = (flags & AST_BC) ? AST_P(b) : bt;
         S.c_ph = (flags & AST_BC) ? AST_P(c) : ct;
@@ -482,9 +485,7 @@ __device__ __forceinline__ double fp64_vmod(const DevModel& M, const double* par
     if (F.bw) {
         // Brightness frame rotated by theta_R, phi_R (cuda.c:475-497), then the
         // black-and-white ball (cuda.c:596-607).
-        double cos_phR, sin_phR, cos_thR, sin_thR;
-        sincos(AST_P(phi_R), &sin_phR, &cos_phR);
-        sincos(AST_P(theta_R), &sin_thR, &cos_thR);
+        const double cos_phR = F.cos_phR, sin_phR = F.sin_phR, cos_thR = F.cos_thR, sin_thR = F.sin_thR;
         N_x = b_x * cos_phR + c_x * sin_phR;
         N_y = b_y * cos_phR + c_y * sin_phR;
         N_z = b_z * cos_phR + c_z * sin_phR;
@@ -643,8 +644,8 @@ __device__ CF chi2_fp64(const DevModel& M, const ObsView& o, const double* param
 {
     const int flags = M.flags;
     const int N_data = M.n_data, N_filters = M.n_filters;
-    double sum_y2[AST_MAX_FILTERS], sum_y[AST_MAX_FILTERS], sum_w[AST_MAX_FILTERS];
-    for (int m = 0; m < N_filters; m++) { sum_y2[m] = 0.0; sum_y[m] = 0.0; sum_w[m] = 0.0; }
+    double sum_y2[AST_MAX_FILTERS], sum_y[AST_MAX_FILTERS];
+    for (int m = 0; m < N_filters; m++) { sum_y2[m] = 0.0; sum_y[m] = 0.0; }
     Fp64Minima Q;
     Fp64Setup S;
     fp64_setup(M, params, S);
@@ -669,12 +670,11 @@ __device__ CF chi2_fp64(const DevModel& M, const ObsView& o, const double* param
             const double yv = o.v[i] - Vmod;
             const float wi = o.w[i];
             sum_y2[m] = sum_y2[m] + yv * yv * wi;
-            sum_y[m] = sum_y[m] + yv * wi;
-            sum_w[m] = sum_w[m] + wi;
+            sum_y[m] = sum_y[m] + yv * wi;  // (the weights' own sums are the object's, prep_obs_sums)
         }
         if ((flags & AST_NUDGE) && !fp64_minima(M, Q, i, o.t[i], Vmod)) return (CF)kHuge;
     }
-    return fp64_finish<CF>(M, sum_y2, sum_y, sum_w, Q, delta_V);
+    return fp64_finish<CF>(M, sum_y2, sum_y, o.sum_w, Q, delta_V);
 }
 
 }  // namespace ast
