@@ -148,6 +148,40 @@ __global__ void __launch_bounds__(128, MINB) eval_kernel(DevModel M, const void*
     bulk_drain(&bar, staged || !use_smem);
 }
 
+// The mixed evaluation by integrator and photometer warps (mixed.cuh): K = blockDim / (32 (1 + PW))
+// integrators, then PW photometers of each; dynamic shared memory: K PairTiles.
+template <class CF, int PREC, int PW>
+__global__ void __launch_bounds__(PW == 1 ? 256 : 96, 1) eval_pair_kernel(DevModel M, const void* g_obs, ObsLayout L,
+                                                                          const double* __restrict__ params, int64_t n,
+                                                                          double* __restrict__ chi2, double* __restrict__ dv)
+{
+    __shared__ float4 trig[kTrigEntries<PREC>];
+    extern __shared__ __align__(16) unsigned char pair_smem[];
+    trig_table_fill(trig, kTrigEntries<PREC>);
+    __syncthreads();
+    const ObsView o = L.view(g_obs, M.n_data);
+    const int N = M.n_params;
+    const int K = blockDim.x / (32 * (1 + PW)), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool integrator = warp < K;
+    const int pair = integrator ? warp : (warp - K) / PW;
+    const int chain = integrator ? lane : (warp - K) % PW * (32 / PW) + lane / PW;
+    PairTile& B = reinterpret_cast<PairTile*>(pair_smem)[pair];
+    const int64_t k = ((int64_t)blockIdx.x * K + pair) * 32 + chain;
+    double p[AST_MAX_PARAMS];
+    for (int i = 0; i < N; i++) p[i] = params[(k < n ? k : n - 1) * N + i];
+    if (integrator) {
+        pair_integrate<PREC == AST_PREC_MIXED_RHS32>(M, o, p, trig, B, 1 + pair, 32 * (1 + PW));
+        return;
+    }
+    CF d[AST_MAX_FILTERS];
+    for (int m = 0; m < M.n_filters; m++) d[m] = 0;
+    const CF r = pair_observe<CF, PW>(M, o, p, d, trig, B, chain, 1 + pair, 32 * (1 + PW));
+    if (k >= n || lane % PW) return;
+    chi2[k] = (double)r;
+    if (dv)
+        for (int m = 0; m < M.n_filters; m++) dv[k * M.n_filters + m] = (double)d[m];
+}
+
 // The FP64 evaluation by groups of G lanes (group64.cuh), one warp a CTA: few vectors take as many SMs
 // as there are warps.
 template <class CF, int G>
@@ -344,6 +378,20 @@ static int launch_eval_group(ast_ctx* c, const DevModel& dm, const double* d_par
     return AST_OK;
 }
 
+template <class CF, int PREC, int PW>
+static int launch_eval_pair(ast_ctx* c, const DevModel& dm, int integrators, const double* d_params, int64_t n,
+                            double* d_chi2, double* d_dv, cudaStream_t s)
+{
+    auto kern = eval_pair_kernel<CF, PREC, PW>;
+    const size_t smem = sizeof(PairTile) * integrators;
+    AST_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int64_t per_cta = 32 * integrators;
+    kern<<<(unsigned)((n + per_cta - 1) / per_cta), 32 * integrators * (1 + PW), smem, s>>>(dm, c->d_obs, c->layout, d_params,
+                                                                                            n, d_chi2, d_dv);
+    AST_CUDA(cudaGetLastError());
+    return AST_OK;
+}
+
 template <class CF, int PREC>
 static int launch_eval(ast_ctx* c, const DevModel& dm, const double* d_params, int64_t n, double* d_chi2, double* d_dv,
                        cudaStream_t s, unsigned long long* d_err)
@@ -359,6 +407,14 @@ static int launch_eval(ast_ctx* c, const DevModel& dm, const double* d_params, i
             dm, c->d_obs, c->layout, 0, d_params, n, d_chi2, d_dv, d_err);
         AST_CUDA(cudaGetLastError());
         return AST_OK;
+    }
+    if (PREC != AST_PREC_FP64) {
+        const PairShape q = pair_shape(n, c->sm_count);
+        if (q.integrators)
+            return q.photometers == 2 ? launch_eval_pair<CF, PREC == AST_PREC_FP64 ? AST_PREC_MIXED : PREC, 2>(
+                                            c, dm, q.integrators, d_params, n, d_chi2, d_dv, s)
+                                      : launch_eval_pair<CF, PREC == AST_PREC_FP64 ? AST_PREC_MIXED : PREC, 1>(
+                                            c, dm, q.integrators, d_params, n, d_chi2, d_dv, s);
     }
     // As the fits (fit_launch_core): the precision's own shape when the vectors fill it, the full
     // register file when they do not (1001 vectors of 480 points, mixed: 1.19 ms against 1.33).

@@ -115,6 +115,22 @@ inline int group_lanes(int64_t n, int sm_count)
     return n <= 4 * (int64_t)sm_count ? 32 : n <= 32 * (int64_t)sm_count ? 8 : 1;
 }
 
+// Integrator warps of a CTA of the paired mixed kernels (mixed.cuh) and photometer warps of each, by the
+// number of evaluations that run side by side; 0 integrators: one thread an evaluation, both parts.
+// Pairs win while an SM holds at most four integrators (a warp's integration alone keeps 81% of the
+// FP32 pipe of its quarter busy, its magnitudes a third); two photometers an integrator while an
+// SM holds one.
+struct PairShape {
+    int integrators, photometers;
+};
+inline PairShape pair_shape(int64_t n, int sm_count)
+{
+    const int64_t warps = (n + 31) / 32;
+    if (warps > 4 * (int64_t)sm_count) return {0, 0};
+    if (warps <= sm_count) return {1, 2};
+    return {(int)((warps + sm_count - 1) / sm_count), 1};
+}
+
 int build_dev_model(const ast_model* m, const ast_obs_set* obs, DevModel* dm);
 int set_device(int device);
 void obs_image(const ast_model* model, const ast_obs_set* obs, const ObsLayout& L, std::vector<unsigned char>& img);

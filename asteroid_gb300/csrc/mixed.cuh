@@ -737,94 +737,99 @@ AST_HD CF mixed_combine(const DevModel& M, const ObsView& o, const df* sum_y, co
     return chi2a;
 }
 
-// Same contract as chi2_fp64 (model.cuh); tab is the shared-memory sin/cos table; ang_out, when
-// non-null, receives the Euler angles at every observation (reduced to [-pi, pi]).  RHS32 selects
-// the FP32 right-hand side of AST_PREC_MIXED_RHS32.
-template <class CF, bool RHS32 = false>
-__host__ __device__ CF chi2_mixed(const DevModel& M, const ObsView& o, const double* params, CF* delta_V, const float4* tab,
-                                  double* ang_out = nullptr)
-{
-    const int flags = M.flags;
-    const int N_data = M.n_data, N_filters = M.n_filters;
+// What the observations of one evaluation add up to: the per-filter residual sums and, under NUDGE, the
+// last two observations, the model minima found so far and the queue of candidates.  (Three
+// variables, since the queue alone has its address taken by a call: the others stay in registers.)
+struct MixedSums {
     df sum_y2[AST_MAX_FILTERS], sum_y[AST_MAX_FILTERS];
-    for (int m = 0; m < N_filters; m++) { sum_y2[m] = df{0.0f, 0.0f}; sum_y[m] = df{0.0f, 0.0f}; }
+};
+struct MixedLast {
+    float t[2] = {0.f, 0.f}, V[2] = {0.f, 0.f};
+    df ang[2][3] = {};
+};
+struct MixedQueue {
     int Mmin = 0;
     float t_mod[AST_M_MAX], V_mod[AST_M_MAX];
-    float t_old[2] = {0.f, 0.f}, V_old[2] = {0.f, 0.f};
-    df ang_old[2][3] = {};
     NudgeCand cand[kNudgeQueue];
     int n_cand = 0;
-    MixedState S;
-    mixed_setup(M, params, S);
-    if (!RHS32) mixed_begin(S);
-    DfFrame F;
-    if (flags & AST_NUDGE) F = make_df_frame(M, params);
-    for (int i = 0; i < N_data; i++) {
-        df ang[3];
-        mixed_advance<RHS32>(S, o, i, tab, ang);
-        if (ang_out)
-            for (int k = 0; k < 3; k++) ang_out[3 * i + k] = df_to_double(ang[k]);
-        const float Vmod = mixed_vmod(S.F, S.bw, DF_ADD(ang[0].hi, ang[0].lo), DF_ADD(ang[1].hi, ang[1].lo),
-                                      DF_ADD(ang[2].hi, ang[2].lo), o, i);
-        {
-            // Residual and weighted sums as double-floats: v - Vmod exactly (TwoSum), products
-            // to ~u^2, sums with the sloppy double-float add (absolute error ~u^2 of the sum).
-            const int m = o.f[i];
-            const df yv = two_sum(o.v[i], -Vmod);
-            const df wy = df_mul_f(yv, o.w[i]);
-            sum_y[m] = df_add_fast(sum_y[m], wy);
-            sum_y2[m] = df_add_fast(sum_y2[m], df_mul_fast(wy, yv));
-        }
-        if (flags & AST_NUDGE) {
-            // Model minima near observed minima (cuda.c:716-760).  The detection and the parabola
-            // are discontinuous in the magnitudes (the reference even rounds them to float), so an
-            // FP32 magnitude is used only to rule a triple out with a margin far above its error;
-            // a candidate triple is queued with its double-float angles and re-evaluated with
-            // double-float magnitudes (nudge_flush), in order, exactly as the reference tests it.
-            const df ang_i[3] = {ang[0], ang[1], ang[2]};
-            if (i >= 2) {
-                bool local = false;
-                for (int ii = 0; ii < M.n_min; ii++)
-                    if (fabsf(t_old[1] - M.t_min[ii]) < AST_DT_MAX2) local = true;
-                const float margin = 1e-4f;
-                if (local && V_old[1] > V_old[0] - margin && V_old[1] >= Vmod - margin) {
-                    NudgeCand& q = cand[n_cand];
-                    q.i = i;
-                    for (int k = 0; k < 3; k++) {
-                        q.a[0][k] = ang_old[0][k];
-                        q.a[1][k] = ang_old[1][k];
-                        q.a[2][k] = ang_i[k];
-                    }
-                    if (++n_cand == kNudgeQueue && !nudge_flush(M, o, F, tab, cand, &n_cand, &Mmin, t_mod, V_mod))
-                        return (CF)kHuge;
-                }
+};
+
+AST_HD void mixed_sums_begin(const DevModel& M, MixedSums& Q)
+{
+    for (int m = 0; m < M.n_filters; m++) { Q.sum_y2[m] = df{0.0f, 0.0f}; Q.sum_y[m] = df{0.0f, 0.0f}; }
+}
+
+// Observation i with model magnitude Vmod and Euler angles ang.  Returns false once there are more than
+// M_MAX minima.
+AST_HD bool mixed_observe(const DevModel& M, const ObsView& o, const DfFrame& F, const float4* tab, MixedSums& Q, MixedLast& E,
+                          MixedQueue& W, int i, float Vmod, const df* ang)
+{
+    {
+        // Residual and weighted sums as double-floats: v - Vmod exactly (TwoSum), products
+        // to ~u^2, sums with the sloppy double-float add (absolute error ~u^2 of the sum).
+        const int m = o.f[i];
+        const df yv = two_sum(o.v[i], -Vmod);
+        const df wy = df_mul_f(yv, o.w[i]);
+        Q.sum_y[m] = df_add_fast(Q.sum_y[m], wy);
+        Q.sum_y2[m] = df_add_fast(Q.sum_y2[m], df_mul_fast(wy, yv));
+    }
+    if (!(M.flags & AST_NUDGE)) return true;
+    // Model minima near observed minima (cuda.c:716-760).  The detection and the parabola
+    // are discontinuous in the magnitudes (the reference even rounds them to float), so an
+    // FP32 magnitude is used only to rule a triple out with a margin far above its error;
+    // a candidate triple is queued with its double-float angles and re-evaluated with
+    // double-float magnitudes (nudge_flush), in order, exactly as the reference tests it.
+    const df ang_i[3] = {ang[0], ang[1], ang[2]};
+    if (i >= 2) {
+        bool local = false;
+        for (int ii = 0; ii < M.n_min; ii++)
+            if (fabsf(E.t[1] - M.t_min[ii]) < AST_DT_MAX2) local = true;
+        const float margin = 1e-4f;
+        if (local && E.V[1] > E.V[0] - margin && E.V[1] >= Vmod - margin) {
+            NudgeCand& q = W.cand[W.n_cand];
+            q.i = i;
+            for (int k = 0; k < 3; k++) {
+                q.a[0][k] = E.ang[0][k];
+                q.a[1][k] = E.ang[1][k];
+                q.a[2][k] = ang_i[k];
             }
-            const int slot = i < 2 ? i : 1;
-            if (i >= 2) {
-                t_old[0] = t_old[1];
-                V_old[0] = V_old[1];
-                for (int k = 0; k < 3; k++) ang_old[0][k] = ang_old[1][k];
-            }
-            t_old[slot] = (float)o.t[i];
-            V_old[slot] = Vmod;
-            for (int k = 0; k < 3; k++) ang_old[slot][k] = ang_i[k];
+            if (++W.n_cand == kNudgeQueue && !nudge_flush(M, o, F, tab, W.cand, &W.n_cand, &W.Mmin, W.t_mod, W.V_mod))
+                return false;
         }
     }
-    if ((flags & AST_NUDGE) && !nudge_flush(M, o, F, tab, cand, &n_cand, &Mmin, t_mod, V_mod)) return (CF)kHuge;
+    const int slot = i < 2 ? i : 1;
+    if (i >= 2) {
+        E.t[0] = E.t[1];
+        E.V[0] = E.V[1];
+        for (int k = 0; k < 3; k++) E.ang[0][k] = E.ang[1][k];
+    }
+    E.t[slot] = (float)o.t[i];
+    E.V[slot] = Vmod;
+    for (int k = 0; k < 3; k++) E.ang[slot][k] = ang_i[k];
+    return true;
+}
+
+// chi^2 and delta_V of the sums, with the reward and punishment factors of the minima (cuda.c:887-993).
+template <class CF>
+__host__ __device__ CF mixed_finish(const DevModel& M, const ObsView& o, const DfFrame& F, const float4* tab, const MixedSums& Q,
+                                    MixedQueue& W, CF* delta_V)
+{
+    const int N_filters = M.n_filters;
+    if ((M.flags & AST_NUDGE) && !nudge_flush(M, o, F, tab, W.cand, &W.n_cand, &W.Mmin, W.t_mod, W.V_mod)) return (CF)kHuge;
     CF dv[AST_MAX_FILTERS];
-    CF chi2a = mixed_combine<CF>(M, o, sum_y, sum_y2, dv);
-    if (flags & AST_NUDGE) {
+    CF chi2a = mixed_combine<CF>(M, o, Q.sum_y, Q.sum_y2, dv);
+    if (M.flags & AST_NUDGE) {
         float S_M = 0.0f, P_tot = 1.0f;
-        for (int imod = 0; imod < Mmin; imod++) {
+        for (int imod = 0; imod < W.Mmin; imod++) {
             for (int iobs = 0; iobs < M.n_min; iobs++) {
-                const float dt = fabsf(t_mod[imod] - M.t_min[iobs]);
+                const float dt = fabsf(W.t_mod[imod] - M.t_min[iobs]);
                 if (dt < AST_DT_MAX2) {
                     if (dt > AST_DT_MAX) {
                         const float x = (AST_DT_MAX2 - dt) / (AST_DT_MAX2 - AST_DT_MAX);
                         S_M = (float)DD_ADD(S_M, DD_MUL((double)DF_MUL(x, x), DD_ADD(DD_MUL(-2.0, (double)x), 3.0)));
                     } else {
                         S_M = (float)(S_M + 1.0);
-                        const float dV = (float)(V_mod[imod] + dv[0] - M.v_min[iobs]);
+                        const float dV = (float)(W.V_mod[imod] + dv[0] - M.v_min[iobs]);
                         const float x = sqrtf(DF_ADD(DF_MUL(dt, dt) / AST_DT_MAX / AST_DT_MAX,
                                                      DF_MUL(dV, dV) / AST_DV_MAX / AST_DV_MAX));
                         if (x < 1.0f) {
@@ -857,6 +862,128 @@ __host__ __device__ CF chi2_mixed(const DevModel& M, const ObsView& o, const dou
     for (int m = 0; m < N_filters; m++) delta_V[m] = dv[m];
     return chi2a;
 }
+
+// Same contract as chi2_fp64 (model.cuh); tab is the shared-memory sin/cos table; ang_out, when
+// non-null, receives the Euler angles at every observation (reduced to [-pi, pi]).  RHS32 selects
+// the FP32 right-hand side of AST_PREC_MIXED_RHS32.
+template <class CF, bool RHS32 = false>
+__host__ __device__ CF chi2_mixed(const DevModel& M, const ObsView& o, const double* params, CF* delta_V, const float4* tab,
+                                  double* ang_out = nullptr)
+{
+    MixedSums Q;
+    MixedLast E;
+    MixedQueue W;
+    mixed_sums_begin(M, Q);
+    MixedState S;
+    mixed_setup(M, params, S);
+    if (!RHS32) mixed_begin(S);
+    DfFrame F;
+    if (M.flags & AST_NUDGE) F = make_df_frame(M, params);
+    for (int i = 0; i < M.n_data; i++) {
+        df ang[3];
+        mixed_advance<RHS32>(S, o, i, tab, ang);
+        if (ang_out)
+            for (int k = 0; k < 3; k++) ang_out[3 * i + k] = df_to_double(ang[k]);
+        const float Vmod = mixed_vmod(S.F, S.bw, DF_ADD(ang[0].hi, ang[0].lo), DF_ADD(ang[1].hi, ang[1].lo),
+                                      DF_ADD(ang[2].hi, ang[2].lo), o, i);
+        if (!mixed_observe(M, o, F, tab, Q, E, W, i, Vmod, ang)) return (CF)kHuge;
+    }
+    return mixed_finish<CF>(M, o, F, tab, Q, W, delta_V);
+}
+
+#ifdef __CUDACC__
+// ---------------------------------------------------------------- integrator and photometer warps
+//
+// For fewer evaluations than the SMs' quarters hold warps.  There a warp alone is bound by its own
+// instruction stream: 1490 cycles an RK4 step, of which the FP32 pipe is busy 1211, and then 3100
+// cycles a magnitude (Lommel-Seeliger), a chain of square roots, arctangents and logarithms that
+// leaves the pipe idle.  Two warps share the 32 evaluations instead: one integrates, a tile of
+// observations ahead, the other turns the tile's angles into magnitudes and sums; they run side by
+// side, on two quarters of the SM where there is room.  With PW photometer lanes an evaluation, PW
+// photometer warps take the tile's observations PW at a time.  Operations, operands and summation
+// order are chi2_mixed's, so are the bits.
+constexpr int kPairTile = 8;
+
+// Shared memory of one integrator and its photometers: two tiles of double-float angles, 32 wide.
+struct PairTile {
+    float ang[2][kPairTile][6][32];
+};
+
+// The barrier of one integrator and its photometers (id 1 to 15).
+__device__ __forceinline__ void pair_sync(int id, int threads)
+{
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// The integrator warp's part of an evaluation of params (its lane's).  Ends one barrier after the last
+// tile's.
+template <bool RHS32>
+__device__ void pair_integrate(const DevModel& M, const ObsView& o, const double* params, const float4* tab,
+                               PairTile& B, int id, int threads)
+{
+    const int lane = threadIdx.x & 31;
+    MixedState S;
+    mixed_setup(M, params, S);
+    if (!RHS32) mixed_begin(S);
+    int b = 0;
+    for (int i0 = 0; i0 < M.n_data; i0 += kPairTile, b ^= 1) {
+        const int n = min(kPairTile, M.n_data - i0);
+        for (int j = 0; j < n; j++) {
+            df a[3];
+            mixed_advance<RHS32>(S, o, i0 + j, tab, a);
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                B.ang[b][j][2 * k][lane] = a[k].hi;
+                B.ang[b][j][2 * k + 1][lane] = a[k].lo;
+            }
+        }
+        pair_sync(id, threads);  // this tile is written, the one before it read
+    }
+    pair_sync(id, threads);
+}
+
+// A photometer warp's part: evaluation `chain` (0 to 31) of the integrator's, whose parameters params
+// are, by PW consecutive lanes; chi^2 and delta_V on each of them.
+template <class CF, int PW>
+__device__ CF pair_observe(const DevModel& M, const ObsView& o, const double* params, CF* delta_V, const float4* tab,
+                           const PairTile& B, int chain, int id, int threads)
+{
+    const int sub = threadIdx.x & (PW - 1);
+    MixedSums Q;
+    MixedLast E;
+    MixedQueue W;
+    mixed_sums_begin(M, Q);
+    MixedState S;
+    mixed_setup(M, params, S);
+    DfFrame F;
+    if (M.flags & AST_NUDGE) F = make_df_frame(M, params);
+    bool huge = false;
+    int b = 0;
+    for (int i0 = 0; i0 < M.n_data; i0 += kPairTile, b ^= 1) {
+        pair_sync(id, threads);
+        const int n = min(kPairTile, M.n_data - i0);
+        for (int j0 = 0; j0 < n; j0 += PW) {
+            const int j = min(j0 + sub, n - 1);
+            const float(*a)[32] = B.ang[b][j];
+            const float V = mixed_vmod(S.F, S.bw, DF_ADD(a[0][chain], a[1][chain]), DF_ADD(a[2][chain], a[3][chain]),
+                                       DF_ADD(a[4][chain], a[5][chain]), o, i0 + j);
+#pragma unroll
+            for (int q = 0; q < PW; q++) {
+                const float Vq = PW == 1 ? V : __shfl_sync(0xffffffffu, V, q, PW);
+                if (j0 + q >= n || huge) continue;
+                const float(*c)[32] = B.ang[b][j0 + q];
+                const df ang[3] = {df{c[0][chain], c[1][chain]}, df{c[2][chain], c[3][chain]}, df{c[4][chain], c[5][chain]}};
+                huge = !mixed_observe(M, o, F, tab, Q, E, W, i0 + j0 + q, Vq, ang);
+            }
+        }
+    }
+    CF r = (CF)kHuge;
+    if (!huge) r = mixed_finish<CF>(M, o, F, tab, Q, W, delta_V);
+    pair_sync(id, threads);
+    return r;
+}
+#endif
 
 // ---------------------------------------------------------------- warp-tiled evaluation
 //
