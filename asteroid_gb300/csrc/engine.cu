@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(128, MINB) eval_kernel(DevModel M, const void*
 // The mixed evaluation by integrator and photometer warps (mixed.cuh): K = blockDim / (32 (1 + PW))
 // integrators, then PW photometers of each; dynamic shared memory: K PairTiles.
 template <class CF, int PREC, int PW>
-__global__ void __launch_bounds__(PW == 1 ? 256 : 96, 1) eval_pair_kernel(DevModel M, const void* g_obs, ObsLayout L,
+__global__ void __launch_bounds__(kPairIntegrators * 32 * (1 + PW), 1) eval_pair_kernel(DevModel M, const void* g_obs, ObsLayout L,
                                                                           const double* __restrict__ params, int64_t n,
                                                                           double* __restrict__ chi2, double* __restrict__ dv)
 {
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(PW == 1 ? 256 : 96, 1) eval_pair_kernel(DevMod
     }
     CF d[AST_MAX_FILTERS];
     for (int m = 0; m < M.n_filters; m++) d[m] = 0;
-    const CF r = pair_observe<CF, PW>(M, o, p, d, trig, B, chain, 1 + pair, 32 * (1 + PW));
+    const CF r = pair_observe<CF, PREC == AST_PREC_MIXED_RHS32, PW>(M, o, p, d, trig, B, chain, 1 + pair, 32 * (1 + PW));
     if (k >= n || lane % PW) return;
     chi2[k] = (double)r;
     if (dv)
@@ -378,10 +378,11 @@ static int launch_eval_group(ast_ctx* c, const DevModel& dm, const double* d_par
     return AST_OK;
 }
 
-template <class CF, int PREC, int PW>
+template <class CF, int PREC>
 static int launch_eval_pair(ast_ctx* c, const DevModel& dm, int integrators, const double* d_params, int64_t n,
                             double* d_chi2, double* d_dv, cudaStream_t s)
 {
+    constexpr int PW = kPairPhotometers;
     auto kern = eval_pair_kernel<CF, PREC, PW>;
     const size_t smem = sizeof(PairTile) * integrators;
     AST_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -408,14 +409,9 @@ static int launch_eval(ast_ctx* c, const DevModel& dm, const double* d_params, i
         AST_CUDA(cudaGetLastError());
         return AST_OK;
     }
-    if (PREC != AST_PREC_FP64) {
-        const PairShape q = pair_shape(n, c->sm_count);
-        if (q.integrators)
-            return q.photometers == 2 ? launch_eval_pair<CF, PREC == AST_PREC_FP64 ? AST_PREC_MIXED : PREC, 2>(
-                                            c, dm, q.integrators, d_params, n, d_chi2, d_dv, s)
-                                      : launch_eval_pair<CF, PREC == AST_PREC_FP64 ? AST_PREC_MIXED : PREC, 1>(
-                                            c, dm, q.integrators, d_params, n, d_chi2, d_dv, s);
-    }
+    if (PREC != AST_PREC_FP64)
+        if (const int k = pair_integrators(n, c->sm_count))
+            return launch_eval_pair<CF, PREC == AST_PREC_FP64 ? AST_PREC_MIXED : PREC>(c, dm, k, d_params, n, d_chi2, d_dv, s);
     // As the fits (fit_launch_core): the precision's own shape when the vectors fill it, the full
     // register file when they do not (1001 vectors of 480 points, mixed: 1.19 ms against 1.33).
     constexpr int kFull = KernShape<PREC>::min_ctas;

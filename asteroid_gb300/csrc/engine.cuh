@@ -56,7 +56,8 @@ struct FitRun {
     int64_t n_evals = 0, n_fits = 0;
     double kernel_ms = 0;
     int tpb = 256, ctas = 0;
-    int lanes = 1;     // lanes of a slot (fit_group_kernel), 1: a thread each
+    int lanes = 1;     // threads of a slot (fit_group_kernel, fit_pair_kernel)
+    int pair = 0;      // integrators of a CTA of fit_pair_kernel, 0: another kernel
     size_t smem = 0;   // dynamic shared memory of the launch (the observation block, or 0)
     int minb = 1;      // register budget variant of fit_kernel
 };
@@ -115,20 +116,14 @@ inline int group_lanes(int64_t n, int sm_count)
     return n <= 4 * (int64_t)sm_count ? 32 : n <= 32 * (int64_t)sm_count ? 8 : 1;
 }
 
-// Integrator warps of a CTA of the paired mixed kernels (mixed.cuh) and photometer warps of each, by the
-// number of evaluations that run side by side; 0 integrators: one thread an evaluation, both parts.
-// Pairs win while an SM holds at most four integrators (a warp's integration alone keeps 81% of the
-// FP32 pipe of its quarter busy, its magnitudes a third); two photometers an integrator while an
-// SM holds one.
-struct PairShape {
-    int integrators, photometers;
-};
-inline PairShape pair_shape(int64_t n, int sm_count)
+// Integrator warps of a CTA of the paired mixed kernels (mixed.cuh), by the number of evaluations that run
+// side by side; 0: one thread an evaluation, both parts.  Pairs win while an SM holds at most four
+// integrators, one on each of its quarters.
+constexpr int kPairIntegrators = 4;
+inline int pair_integrators(int64_t n, int sm_count)
 {
-    const int64_t warps = (n + 31) / 32;
-    if (warps > 4 * (int64_t)sm_count) return {0, 0};
-    if (warps <= sm_count) return {1, 2};
-    return {(int)((warps + sm_count - 1) / sm_count), 1};
+    const int64_t k = ((n + 31) / 32 + sm_count - 1) / sm_count;
+    return k <= kPairIntegrators ? (int)k : 0;
 }
 
 int build_dev_model(const ast_model* m, const ast_obs_set* obs, DevModel* dm);

@@ -184,6 +184,91 @@ __global__ void __launch_bounds__(32, 8) fit_group_kernel(DevModel M, const void
     if (n_fit) atomicAdd(&V.ctr[3], n_fit);
 }
 
+// fit_kernel with the evaluation shared by an integrator warp, which runs the chains of its 32 lanes, and
+// kPairPhotometers photometer warps (mixed.cuh), for mixed fits of too few chains to fill the SMs'
+// quarters.  K integrators a CTA, then their photometers; dynamic shared memory: K PairChains.
+template <class CF, int PREC>
+__global__ void __launch_bounds__(kPairIntegrators * 32 * (1 + kPairPhotometers), 1)
+    fit_pair_kernel(DevModel M, const void* g_obs, ObsLayout L, FitView<CF> V, int64_t budget)
+{
+    constexpr int PW = kPairPhotometers, kThreads = 32 * (1 + PW);
+    constexpr bool RHS32 = PREC == AST_PREC_MIXED_RHS32;
+    __shared__ float4 trig[kTrigEntries<PREC>];
+    extern __shared__ __align__(16) unsigned char pair_smem[];
+    trig_table_fill(trig, kTrigEntries<PREC>);
+    __syncthreads();
+    const ObsView o = L.view(g_obs, M.n_data);
+    const int K = blockDim.x / kThreads, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int pair = warp < K ? warp : (warp - K) / PW, id = 1 + pair;
+    PairChain& X = reinterpret_cast<PairChain*>(pair_smem)[pair];
+    if (warp >= K) {
+        const int chain = (warp - K) % PW * (32 / PW) + lane / PW;
+        while (true) {
+            pair_sync(id, kThreads);
+            if (!X.more) return;
+            pair_serve<CF, RHS32, PW>(M, o, trig, X, chain, id, kThreads);
+        }
+    }
+    const int64_t s = ((int64_t)blockIdx.x * K + pair) * 32 + lane;
+    const int N = M.n_params, NF = M.n_filters;
+    const int64_t S = V.S;
+    SlotState<CF> R;
+    R.chain = V.chain[s];
+    R.st = V.st[s];
+    R.l = V.it[s];
+    R.ev = V.ev[s];
+    for (int m = 0; m < NF; m++) R.dvl[m] = (CF)V.dv[(int64_t)m * S + s];
+    bool empty = false;  // no chain left for the lane
+    unsigned long long n_ev = 0, n_fit = 0, n_done = 0;
+    for (int64_t used = 0; used < budget; used++) {
+        if (R.chain < 0 && !empty) {
+            const unsigned long long c = atomicAdd(&V.ctr[0], 1ull);
+            if (c >= (unsigned long long)V.n_chains) {
+                empty = true;
+            } else {
+                R.chain = (int64_t)c;
+                start_chain<CF>(M, V, s, R.chain);
+                R.st = PH_INIT;
+                R.l = 0;
+                R.ev = 0;
+                for (int m = 0; m < NF; m++) R.dvl[m] = V.stage > 0 ? (CF)V.chain_dv[R.chain * NF + m] : (CF)0;
+            }
+        }
+        if (__all_sync(0xffffffffu, R.chain < 0)) break;
+        CF p[AST_MAX_PARAMS];
+        double params[AST_MAX_PARAMS];
+        for (int i = 0; i < N; i++) params[i] = 0.0;
+        int rej = 1;
+        if (R.chain >= 0) {
+            slot_point<CF>(M, V, s, R, p);
+            rej = x2params<CF>(M, V.reopt, p, params);
+        }
+        const unsigned live = __ballot_sync(0xffffffffu, !rej);
+        CF fv = (CF)kHuge;
+        if (live) {
+            const CF f = pair_eval<CF, RHS32>(M, o, params, live, R.dvl, trig, X, id, kThreads);
+            if (!rej) {
+                fv = f;
+                R.ev++;
+                n_ev++;
+            }
+        }
+        if (R.chain >= 0 && slot_apply<CF>(M, V, s, R, p, rej, fv, n_fit)) {
+            n_done++;
+            R.chain = -1;
+        }
+    }
+    pair_stop(X, id, kThreads);
+    V.chain[s] = R.chain;
+    V.st[s] = R.st;
+    V.it[s] = R.l;
+    V.ev[s] = R.ev;
+    for (int m = 0; m < NF; m++) V.dv[(int64_t)m * S + s] = (double)R.dvl[m];
+    if (n_done) atomicAdd(&V.ctr[1], n_done);
+    if (n_ev) atomicAdd(&V.ctr[2], n_ev);
+    if (n_fit) atomicAdd(&V.ctr[3], n_fit);
+}
+
 // Per-group argmin over the chains' results (lowest chi^2, lowest chain on ties, as the serial
 // loop of cuda.c:1770-1782) and the stage hand-off or the final output (cuda.c:1785-1823).
 template <class CF>
@@ -305,6 +390,8 @@ static cudaError_t fit_launch(const FitRun& r, const DevModel& dm, const void* o
         fit_group_kernel<CF, 32><<<r.ctas, r.tpb, 0, s>>>(dm, obs, L, V, budget);
     else if (PREC == AST_PREC_FP64 && r.lanes == 8)
         fit_group_kernel<CF, 8><<<r.ctas, r.tpb, 0, s>>>(dm, obs, L, V, budget);
+    else if (PREC != AST_PREC_FP64 && r.pair)
+        fit_pair_kernel<CF, PREC == AST_PREC_FP64 ? AST_PREC_MIXED : PREC><<<r.ctas, r.tpb, r.smem, s>>>(dm, obs, L, V, budget);
     else
         fit_kernel_ptr<CF, PREC>(r.minb)<<<r.ctas, r.tpb, r.smem, s>>>(dm, obs, L, r.smem ? 1 : 0, V, budget);
     return cudaGetLastError();
@@ -330,6 +417,22 @@ static int fit_launch_core(int sm_count, size_t obs_bytes, size_t optin, int tpb
             r->ctas = (int)((n_chains * r->lanes + 31) / 32);
             r->smem = 0;
             r->minb = 1;
+            return AST_OK;
+        }
+    }
+    // Mixed with no geometry asked for: integrators and photometers while they are faster.
+    r->pair = 0;
+    if (PREC != AST_PREC_FP64 && tpb_req <= 0 && minb_req <= 0 && stage_req == 0) {
+        r->pair = pair_integrators(n_chains, sm_count);
+        if (r->pair) {
+            const int64_t per_cta = 32 * r->pair;
+            r->lanes = 1 + kPairPhotometers;
+            r->tpb = (int)per_cta * r->lanes;
+            r->ctas = (int)((n_chains + per_cta - 1) / per_cta);
+            r->smem = sizeof(PairChain) * r->pair;
+            r->minb = 1;
+            auto kern = fit_pair_kernel<CF, PREC == AST_PREC_FP64 ? AST_PREC_MIXED : PREC>;
+            AST_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r->smem));
             return AST_OK;
         }
     }

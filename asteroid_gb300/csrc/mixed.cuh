@@ -595,13 +595,12 @@ AST_HD void spin_step_beyond(MixedState& S, float4 hq, float4 hw, const float4* 
     S.s = t;
 }
 
-// Integrate from observation i-1 to i (cuda.c:319-372; nothing for i = 0) and return the Euler
-// angles (phi, theta, psi) in [-pi, pi].  They enter the right-hand side and the brightness only
-// through sin and cos, so the state keeps no whole turns.  RHS32: the FP32 right-hand side
-// (AST_PREC_MIXED_RHS32), a separate instantiation so that the double-float kernels carry none of
-// its code.
+// Integrate from observation i-1 to i (cuda.c:319-372; nothing for i = 0).  RHS32: the FP32 right-hand
+// side (AST_PREC_MIXED_RHS32), a separate instantiation so that the double-float kernels carry none
+// of its code.  The angles enter the right-hand side and the brightness only through sin and cos, so
+// the state keeps no whole turns.
 template <bool RHS32>
-AST_HD void mixed_advance(MixedState& S, const ObsView& o, int i, const float4* tab, df* ang)
+AST_HD void mixed_steps(MixedState& S, const ObsView& o, int i, const float4* tab)
 {
     if (RHS32) {
         if (i > 0) {
@@ -616,22 +615,6 @@ AST_HD void mixed_advance(MixedState& S, const ObsView& o, int i, const float4* 
 #pragma unroll 1
                 for (int l = 0; l < N_steps; l++) rk4_step_f32<3>(S.y, hq, hw, S.muf, tab);
             }
-        }
-        // (Constant indices only: an index computed at run time would move y to local memory.)
-        if (S.torque) {
-            S.y[3] = df_reduce_2pi(S.y[3]);
-            S.y[4] = df_reduce_2pi(S.y[4]);
-            S.y[5] = df_reduce_2pi(S.y[5]);
-            ang[0] = S.y[3];
-            ang[1] = S.y[4];
-            ang[2] = S.y[5];
-        } else {
-            S.y[0] = df_reduce_2pi(S.y[0]);
-            S.y[1] = df_reduce_2pi(S.y[1]);
-            S.y[2] = df_reduce_2pi(S.y[2]);
-            ang[0] = S.y[0];
-            ang[1] = S.y[1];
-            ang[2] = S.y[2];
         }
         return;
     }
@@ -661,7 +644,39 @@ AST_HD void mixed_advance(MixedState& S, const ObsView& o, int i, const float4* 
                 if (!turn_step_free(S.s, C, turn)) spin_step_beyond(S, hq, hw, tab);
         }
     }
-    spin_angles(S.s, S.torque, ang);
+}
+
+// The Euler angles (phi, theta, psi) of the state, in [-pi, pi].
+template <bool RHS32>
+AST_HD void mixed_angles(MixedState& S, df* ang)
+{
+    if (!RHS32) {
+        spin_angles(S.s, S.torque, ang);
+        return;
+    }
+    // (Constant indices only: an index computed at run time would move y to local memory.)
+    if (S.torque) {
+        S.y[3] = df_reduce_2pi(S.y[3]);
+        S.y[4] = df_reduce_2pi(S.y[4]);
+        S.y[5] = df_reduce_2pi(S.y[5]);
+        ang[0] = S.y[3];
+        ang[1] = S.y[4];
+        ang[2] = S.y[5];
+    } else {
+        S.y[0] = df_reduce_2pi(S.y[0]);
+        S.y[1] = df_reduce_2pi(S.y[1]);
+        S.y[2] = df_reduce_2pi(S.y[2]);
+        ang[0] = S.y[0];
+        ang[1] = S.y[1];
+        ang[2] = S.y[2];
+    }
+}
+
+template <bool RHS32>
+AST_HD void mixed_advance(MixedState& S, const ObsView& o, int i, const float4* tab, df* ang)
+{
+    mixed_steps<RHS32>(S, o, i, tab);
+    mixed_angles<RHS32>(S, ang);
 }
 
 // FP32 model magnitude at observation i for the Euler angles (phi, theta, psi): the body frame
@@ -759,17 +774,16 @@ AST_HD void mixed_sums_begin(const DevModel& M, MixedSums& Q)
     for (int m = 0; m < M.n_filters; m++) { Q.sum_y2[m] = df{0.0f, 0.0f}; Q.sum_y[m] = df{0.0f, 0.0f}; }
 }
 
-// Observation i with model magnitude Vmod and Euler angles ang.  Returns false once there are more than
-// M_MAX minima.
+// Observation i (magnitude v, weight w, filter m) with model magnitude Vmod and Euler angles ang.  Returns
+// false once there are more than M_MAX minima.
 AST_HD bool mixed_observe(const DevModel& M, const ObsView& o, const DfFrame& F, const float4* tab, MixedSums& Q, MixedLast& E,
-                          MixedQueue& W, int i, float Vmod, const df* ang)
+                          MixedQueue& W, int i, float v, float w, int m, float Vmod, const df* ang)
 {
     {
         // Residual and weighted sums as double-floats: v - Vmod exactly (TwoSum), products
         // to ~u^2, sums with the sloppy double-float add (absolute error ~u^2 of the sum).
-        const int m = o.f[i];
-        const df yv = two_sum(o.v[i], -Vmod);
-        const df wy = df_mul_f(yv, o.w[i]);
+        const df yv = two_sum(v, -Vmod);
+        const df wy = df_mul_f(yv, w);
         Q.sum_y[m] = df_add_fast(Q.sum_y[m], wy);
         Q.sum_y2[m] = df_add_fast(Q.sum_y2[m], df_mul_fast(wy, yv));
     }
@@ -886,7 +900,7 @@ __host__ __device__ CF chi2_mixed(const DevModel& M, const ObsView& o, const dou
             for (int k = 0; k < 3; k++) ang_out[3 * i + k] = df_to_double(ang[k]);
         const float Vmod = mixed_vmod(S.F, S.bw, DF_ADD(ang[0].hi, ang[0].lo), DF_ADD(ang[1].hi, ang[1].lo),
                                       DF_ADD(ang[2].hi, ang[2].lo), o, i);
-        if (!mixed_observe(M, o, F, tab, Q, E, W, i, Vmod, ang)) return (CF)kHuge;
+        if (!mixed_observe(M, o, F, tab, Q, E, W, i, o.v[i], o.w[i], o.f[i], Vmod, ang)) return (CF)kHuge;
     }
     return mixed_finish<CF>(M, o, F, tab, Q, W, delta_V);
 }
@@ -903,10 +917,62 @@ __host__ __device__ CF chi2_mixed(const DevModel& M, const ObsView& o, const dou
 // photometer warps take the tile's observations PW at a time.  Operations, operands and summation
 // order are chi2_mixed's, so are the bits.
 constexpr int kPairTile = 8;
+constexpr int kPairPhotometers = 2;  // photometer warps of an integrator
 
-// Shared memory of one integrator and its photometers: two tiles of double-float angles, 32 wide.
+// Shared memory of one integrator and its photometers: two tiles of angles as the state holds them, 32
+// wide (compact: three words each; RHS32: double-floats).  The photometers turn them into radians.
 struct PairTile {
-    float ang[2][kPairTile][6][32];
+    float ang[2][kPairTile][9][32];
+};
+
+template <bool RHS32>
+__device__ __forceinline__ void pair_write(MixedState& S, float (*a)[32], int lane)
+{
+    if (RHS32) {
+        df g[3];
+        mixed_angles<true>(S, g);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            a[2 * k][lane] = g[k].hi;
+            a[2 * k + 1][lane] = g[k].lo;
+        }
+        return;
+    }
+    const Spin& s = S.s;
+    a[0][lane] = __uint_as_float(s.phi.k);
+    a[1][lane] = s.phi.e;
+    a[2][lane] = s.phi.t;
+    a[3][lane] = __uint_as_float(s.a.k0);
+    a[4][lane] = s.a.e.x;
+    a[5][lane] = s.a.t.x;
+    a[6][lane] = __uint_as_float(s.a.k1);
+    a[7][lane] = s.a.e.y;
+    a[8][lane] = s.a.t.y;
+}
+
+template <bool RHS32>
+__device__ __forceinline__ void pair_read(const float (*a)[32], int lane, bool torque, df* ang)
+{
+    if (RHS32) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) ang[k] = df{a[2 * k][lane], a[2 * k + 1][lane]};
+        return;
+    }
+    Spin s;
+    s.phi = Turn{__float_as_uint(a[0][lane]), a[1][lane], a[2][lane]};
+    s.a = Turn2{__float_as_uint(a[3][lane]), __float_as_uint(a[6][lane]), make_float2(a[4][lane], a[7][lane]),
+                make_float2(a[5][lane], a[8][lane])};
+    spin_angles(s, torque, ang);
+}
+
+// What an integrator that runs chains exchanges with its photometers beside the tiles: the points'
+// parameters, their chi^2 and delta_V (in: the chain's last), whether there is another evaluation.
+struct PairChain {
+    PairTile tile;
+    double par[AST_MAX_PARAMS][32];
+    double dv[AST_MAX_FILTERS][32];
+    double chi2[32];
+    int more;
 };
 
 // The barrier of one integrator and its photometers (id 1 to 15).
@@ -916,8 +982,8 @@ __device__ __forceinline__ void pair_sync(int id, int threads)
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// The integrator warp's part of an evaluation of params (its lane's).  Ends one barrier after the last
-// tile's.
+// The integrator warp's part of an evaluation of params (its lane's): a barrier after each tile.  The next
+// evaluation's first tile may be written once the photometers are past their last.
 template <bool RHS32>
 __device__ void pair_integrate(const DevModel& M, const ObsView& o, const double* params, const float4* tab,
                                PairTile& B, int id, int threads)
@@ -930,22 +996,16 @@ __device__ void pair_integrate(const DevModel& M, const ObsView& o, const double
     for (int i0 = 0; i0 < M.n_data; i0 += kPairTile, b ^= 1) {
         const int n = min(kPairTile, M.n_data - i0);
         for (int j = 0; j < n; j++) {
-            df a[3];
-            mixed_advance<RHS32>(S, o, i0 + j, tab, a);
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                B.ang[b][j][2 * k][lane] = a[k].hi;
-                B.ang[b][j][2 * k + 1][lane] = a[k].lo;
-            }
+            mixed_steps<RHS32>(S, o, i0 + j, tab);
+            pair_write<RHS32>(S, B.ang[b][j], lane);
         }
         pair_sync(id, threads);  // this tile is written, the one before it read
     }
-    pair_sync(id, threads);
 }
 
 // A photometer warp's part: evaluation `chain` (0 to 31) of the integrator's, whose parameters params
 // are, by PW consecutive lanes; chi^2 and delta_V on each of them.
-template <class CF, int PW>
+template <class CF, bool RHS32, int PW>
 __device__ CF pair_observe(const DevModel& M, const ObsView& o, const double* params, CF* delta_V, const float4* tab,
                            const PairTile& B, int chain, int id, int threads)
 {
@@ -964,24 +1024,74 @@ __device__ CF pair_observe(const DevModel& M, const ObsView& o, const double* pa
         pair_sync(id, threads);
         const int n = min(kPairTile, M.n_data - i0);
         for (int j0 = 0; j0 < n; j0 += PW) {
-            const int j = min(j0 + sub, n - 1);
-            const float(*a)[32] = B.ang[b][j];
-            const float V = mixed_vmod(S.F, S.bw, DF_ADD(a[0][chain], a[1][chain]), DF_ADD(a[2][chain], a[3][chain]),
-                                       DF_ADD(a[4][chain], a[5][chain]), o, i0 + j);
+            const int j = min(j0 + sub, n - 1), i = i0 + j;
+            const float v = o.v[i], w = o.w[i];
+            const int m = o.f[i];
+            df ang[3];
+            pair_read<RHS32>(B.ang[b][j], chain, S.torque, ang);
+            const float V = mixed_vmod(S.F, S.bw, DF_ADD(ang[0].hi, ang[0].lo), DF_ADD(ang[1].hi, ang[1].lo),
+                                       DF_ADD(ang[2].hi, ang[2].lo), o, i);
+            if (PW == 1) {
+                if (!huge) huge = !mixed_observe(M, o, F, tab, Q, E, W, i, v, w, m, V, ang);
+                continue;
+            }
 #pragma unroll
             for (int q = 0; q < PW; q++) {
-                const float Vq = PW == 1 ? V : __shfl_sync(0xffffffffu, V, q, PW);
+                const float Vq = __shfl_sync(0xffffffffu, V, q, PW), vq = __shfl_sync(0xffffffffu, v, q, PW),
+                            wq = __shfl_sync(0xffffffffu, w, q, PW);
+                const int mq = __shfl_sync(0xffffffffu, m, q, PW);
                 if (j0 + q >= n || huge) continue;
-                const float(*c)[32] = B.ang[b][j0 + q];
-                const df ang[3] = {df{c[0][chain], c[1][chain]}, df{c[2][chain], c[3][chain]}, df{c[4][chain], c[5][chain]}};
-                huge = !mixed_observe(M, o, F, tab, Q, E, W, i0 + j0 + q, Vq, ang);
+                if (M.flags & AST_NUDGE) pair_read<RHS32>(B.ang[b][j0 + q], chain, S.torque, ang);
+                huge = !mixed_observe(M, o, F, tab, Q, E, W, i0 + j0 + q, vq, wq, mq, Vq, ang);
             }
         }
     }
-    CF r = (CF)kHuge;
-    if (!huge) r = mixed_finish<CF>(M, o, F, tab, Q, W, delta_V);
+    return huge ? (CF)kHuge : mixed_finish<CF>(M, o, F, tab, Q, W, delta_V);
+}
+
+// One evaluation for the integrator of a PairChain: params on the lanes of `live` (not empty; the others
+// take part with the first live lane's), the chains' last delta_V in dvl.  Returns the lane's chi^2, and
+// its delta_V in dvl.
+template <class CF, bool RHS32>
+__device__ CF pair_eval(const DevModel& M, const ObsView& o, double* params, unsigned live, CF* dvl, const float4* tab,
+                        PairChain& X, int id, int threads)
+{
+    const int lane = threadIdx.x & 31, src = __ffs(live) - 1;
+    for (int i = 0; i < M.n_params; i++) {
+        const double a = __shfl_sync(0xffffffffu, params[i], src);
+        if (!(live >> lane & 1u)) params[i] = a;
+        X.par[i][lane] = params[i];
+    }
+    for (int m = 0; m < M.n_filters; m++) X.dv[m][lane] = (double)dvl[m];
+    if (lane == 0) X.more = 1;
     pair_sync(id, threads);
-    return r;
+    pair_integrate<RHS32>(M, o, params, tab, X.tile, id, threads);
+    pair_sync(id, threads);
+    if (live >> lane & 1u)
+        for (int m = 0; m < M.n_filters; m++) dvl[m] = (CF)X.dv[m][lane];
+    return (CF)X.chi2[lane];
+}
+__device__ __forceinline__ void pair_stop(PairChain& X, int id, int threads)
+{
+    if ((threadIdx.x & 31) == 0) X.more = 0;
+    pair_sync(id, threads);
+}
+
+// A photometer warp's part of one pair_eval, after the barrier that announced it.
+template <class CF, bool RHS32, int PW>
+__device__ void pair_serve(const DevModel& M, const ObsView& o, const float4* tab, PairChain& X, int chain, int id,
+                           int threads)
+{
+    double p[AST_MAX_PARAMS];
+    for (int i = 0; i < M.n_params; i++) p[i] = X.par[i][chain];
+    CF d[AST_MAX_FILTERS];
+    for (int m = 0; m < M.n_filters; m++) d[m] = (CF)X.dv[m][chain];
+    const CF r = pair_observe<CF, RHS32, PW>(M, o, p, d, tab, X.tile, chain, id, threads);
+    if ((threadIdx.x & (PW - 1)) == 0) {
+        X.chi2[chain] = (double)r;
+        for (int m = 0; m < M.n_filters; m++) X.dv[m][chain] = (double)d[m];
+    }
+    pair_sync(id, threads);
 }
 #endif
 

@@ -25,3 +25,28 @@ def test_pairs_equal_threads(gpu, flags, n, filters, span, precision):
             assert np.array_equal(c, chi2[:count], equal_nan=True), count
             assert np.array_equal(d, dv[:count], equal_nan=True), count
     assert np.isfinite(chi2).mean() > 0.3
+
+
+@pytest.mark.parametrize("flags,chains,group,kw", [
+    ("TORQUE,P_PSI,ACC", 1, 1, {}), ("TORQUE,P_PSI", 33, 33, dict(n_stages=2)), ("BC,INTERP,ACC", 700, 7, {}),
+    ("TORQUE,INTERP,ACC,NUDGE", 640, 64, dict(reopt=True)), ("BW_BALL,ACC", 6000, 250, dict(evals_cap=16)),
+    ("TORQUE,ACC", 14336, 256, dict(evals_cap=14, precision=api.PREC_MIXED_RHS32))])
+def test_fits_by_pairs_equal_threads(gpu, flags, chains, group, kw):
+    """A mixed fit of few chains runs by pairs unless a geometry is asked for; both give the same chains."""
+    model, obs, P = _object(flags, 48, 2, 5, 1.0)
+    kw = dict(dict(evals_cap=40, n_stages=1, precision=api.PREC_MIXED), **kw)
+    if kw.get("reopt"):
+        kw["params0"] = P[0]
+    with api.Engine(model, obs) as eng:
+        a = eng.fit(n_chains=chains, group_size=group, seed=9, **kw)
+        assert eng.fit_launch()["tpb"] % 96 == 0
+        b = eng.fit(n_chains=chains, group_size=group, seed=9, tpb=32, **kw)
+        eng.fit_begin(n_chains=chains, group_size=group, seed=9, **kw)  # in bounded steps
+        for _ in range(1000):
+            if eng.fit_step(3):
+                break
+        c = eng.fit_end()
+    for r in (a, c):
+        for k in ("best_f", "best_params", "best_dv", "chain_f"):
+            assert np.array_equal(getattr(r, k), getattr(b, k), equal_nan=True), k
+        assert r.n_evals == b.n_evals and r.n_fits == b.n_fits
