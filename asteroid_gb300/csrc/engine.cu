@@ -148,20 +148,22 @@ __global__ void __launch_bounds__(128, MINB) eval_kernel(DevModel M, const void*
     bulk_drain(&bar, staged || !use_smem);
 }
 
-// The mixed evaluation by integrator and photometer warps (mixed.cuh): K = blockDim / (32 (1 + PW))
-// integrators, then PW photometers of each; dynamic shared memory: K PairTiles.
-template <class CF, int PREC, int PW>
-__global__ void __launch_bounds__(kPairIntegrators * 32 * (1 + PW), 1) eval_pair_kernel(DevModel M, const void* g_obs, ObsLayout L,
-                                                                          const double* __restrict__ params, int64_t n,
-                                                                          double* __restrict__ chi2, double* __restrict__ dv)
+// The mixed evaluation by integrator and photometer warps (mixed.cuh), K integrators a CTA; dynamic shared
+// memory: K PairTiles.
+template <class CF, int PREC>
+__global__ void __launch_bounds__(32 * pair_warps(kPairIntegrators), 1)
+    eval_pair_kernel(DevModel M, const void* g_obs, ObsLayout L, int K, const double* __restrict__ params, int64_t n,
+                     double* __restrict__ chi2, double* __restrict__ dv)
 {
+    constexpr int PW = kPairPhotometers, kThreads = 32 * (1 + PW);
     __shared__ float4 trig[kTrigEntries<PREC>];
     extern __shared__ __align__(16) unsigned char pair_smem[];
     trig_table_fill(trig, kTrigEntries<PREC>);
     __syncthreads();
     const ObsView o = L.view(g_obs, M.n_data);
     const int N = M.n_params;
-    const int K = blockDim.x / (32 * (1 + PW)), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = pair_place(K, threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (warp < 0) return;
     const bool integrator = warp < K;
     const int pair = integrator ? warp : (warp - K) / PW;
     const int chain = integrator ? lane : (warp - K) % PW * (32 / PW) + lane / PW;
@@ -170,12 +172,12 @@ __global__ void __launch_bounds__(kPairIntegrators * 32 * (1 + PW), 1) eval_pair
     double p[AST_MAX_PARAMS];
     for (int i = 0; i < N; i++) p[i] = params[(k < n ? k : n - 1) * N + i];
     if (integrator) {
-        pair_integrate<PREC == AST_PREC_MIXED_RHS32>(M, o, p, trig, B, 1 + pair, 32 * (1 + PW));
+        pair_integrate<PREC == AST_PREC_MIXED_RHS32>(M, o, p, trig, B, 1 + pair, kThreads);
         return;
     }
     CF d[AST_MAX_FILTERS];
     for (int m = 0; m < M.n_filters; m++) d[m] = 0;
-    const CF r = pair_observe<CF, PREC == AST_PREC_MIXED_RHS32, PW>(M, o, p, d, trig, B, chain, 1 + pair, 32 * (1 + PW));
+    const CF r = pair_observe<CF, PREC == AST_PREC_MIXED_RHS32, PW>(M, o, p, d, trig, B, chain, 1 + pair, kThreads);
     if (k >= n || lane % PW) return;
     chi2[k] = (double)r;
     if (dv)
@@ -382,13 +384,12 @@ template <class CF, int PREC>
 static int launch_eval_pair(ast_ctx* c, const DevModel& dm, int integrators, const double* d_params, int64_t n,
                             double* d_chi2, double* d_dv, cudaStream_t s)
 {
-    constexpr int PW = kPairPhotometers;
-    auto kern = eval_pair_kernel<CF, PREC, PW>;
+    auto kern = eval_pair_kernel<CF, PREC>;
     const size_t smem = sizeof(PairTile) * integrators;
     AST_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int64_t per_cta = 32 * integrators;
-    kern<<<(unsigned)((n + per_cta - 1) / per_cta), 32 * integrators * (1 + PW), smem, s>>>(dm, c->d_obs, c->layout, d_params,
-                                                                                            n, d_chi2, d_dv);
+    kern<<<(unsigned)((n + per_cta - 1) / per_cta), 32 * pair_warps(integrators), smem, s>>>(
+        dm, c->d_obs, c->layout, integrators, d_params, n, d_chi2, d_dv);
     AST_CUDA(cudaGetLastError());
     return AST_OK;
 }

@@ -56,7 +56,7 @@ struct FitRun {
     int64_t n_evals = 0, n_fits = 0;
     double kernel_ms = 0;
     int tpb = 256, ctas = 0;
-    int lanes = 1;     // threads of a slot (fit_group_kernel, fit_pair_kernel)
+    int lanes = 1;     // threads of a slot (fit_group_kernel)
     int pair = 0;      // integrators of a CTA of fit_pair_kernel, 0: another kernel
     size_t smem = 0;   // dynamic shared memory of the launch (the observation block, or 0)
     int minb = 1;      // register budget variant of fit_kernel

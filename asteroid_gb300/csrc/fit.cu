@@ -186,10 +186,10 @@ __global__ void __launch_bounds__(32, 8) fit_group_kernel(DevModel M, const void
 
 // fit_kernel with the evaluation shared by an integrator warp, which runs the chains of its 32 lanes, and
 // kPairPhotometers photometer warps (mixed.cuh), for mixed fits of too few chains to fill the SMs'
-// quarters.  K integrators a CTA, then their photometers; dynamic shared memory: K PairChains.
+// quarters.  K integrators a CTA; dynamic shared memory: K PairChains.
 template <class CF, int PREC>
-__global__ void __launch_bounds__(kPairIntegrators * 32 * (1 + kPairPhotometers), 1)
-    fit_pair_kernel(DevModel M, const void* g_obs, ObsLayout L, FitView<CF> V, int64_t budget)
+__global__ void __launch_bounds__(32 * pair_warps(kPairIntegrators), 1)
+    fit_pair_kernel(DevModel M, const void* g_obs, ObsLayout L, int K, FitView<CF> V, int64_t budget)
 {
     constexpr int PW = kPairPhotometers, kThreads = 32 * (1 + PW);
     constexpr bool RHS32 = PREC == AST_PREC_MIXED_RHS32;
@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(kPairIntegrators * 32 * (1 + kPairPhotometers)
     trig_table_fill(trig, kTrigEntries<PREC>);
     __syncthreads();
     const ObsView o = L.view(g_obs, M.n_data);
-    const int K = blockDim.x / kThreads, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = pair_place(K, threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (warp < 0) return;
     const int pair = warp < K ? warp : (warp - K) / PW, id = 1 + pair;
     PairChain& X = reinterpret_cast<PairChain*>(pair_smem)[pair];
     if (warp >= K) {
@@ -391,13 +392,17 @@ static cudaError_t fit_launch(const FitRun& r, const DevModel& dm, const void* o
     else if (PREC == AST_PREC_FP64 && r.lanes == 8)
         fit_group_kernel<CF, 8><<<r.ctas, r.tpb, 0, s>>>(dm, obs, L, V, budget);
     else if (PREC != AST_PREC_FP64 && r.pair)
-        fit_pair_kernel<CF, PREC == AST_PREC_FP64 ? AST_PREC_MIXED : PREC><<<r.ctas, r.tpb, r.smem, s>>>(dm, obs, L, V, budget);
+        fit_pair_kernel<CF, PREC == AST_PREC_FP64 ? AST_PREC_MIXED : PREC><<<r.ctas, r.tpb, r.smem, s>>>(dm, obs, L, r.pair, V,
+                                                                                                        budget);
     else
         fit_kernel_ptr<CF, PREC>(r.minb)<<<r.ctas, r.tpb, r.smem, s>>>(dm, obs, L, r.smem ? 1 : 0, V, budget);
     return cudaGetLastError();
 }
 
-static int64_t fit_slots(const FitRun& r) { return (int64_t)r.tpb * r.ctas / r.lanes; }
+static int64_t fit_slots(const FitRun& r)
+{
+    return r.pair ? (int64_t)32 * r.pair * r.ctas : (int64_t)r.tpb * r.ctas / r.lanes;
+}
 
 // Launch geometry: CTA size (tpb), register budget (minb) and whether the CTA stages the
 // observations in shared memory.  Staging is dropped when the block would lower the number of
@@ -426,8 +431,7 @@ static int fit_launch_core(int sm_count, size_t obs_bytes, size_t optin, int tpb
         r->pair = pair_integrators(n_chains, sm_count);
         if (r->pair) {
             const int64_t per_cta = 32 * r->pair;
-            r->lanes = 1 + kPairPhotometers;
-            r->tpb = (int)per_cta * r->lanes;
+            r->tpb = 32 * pair_warps(r->pair);
             r->ctas = (int)((n_chains + per_cta - 1) / per_cta);
             r->smem = sizeof(PairChain) * r->pair;
             r->minb = 1;

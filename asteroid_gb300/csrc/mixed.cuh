@@ -906,6 +906,23 @@ __host__ __device__ CF chi2_mixed(const DevModel& M, const ObsView& o, const dou
 }
 
 #ifdef __CUDACC__
+// The magnitude frames of a warp's 32 evaluations in shared memory, [kMixedFrameFloats][32].
+__device__ __forceinline__ void frame_store(float* fr, int lane, const MixedFrame& F)
+{
+    const float* f = &F.M_x;
+#pragma unroll
+    for (int k = 0; k < kMixedFrameFloats; k++) fr[k * 32 + lane] = f[k];
+}
+
+__device__ __forceinline__ MixedFrame frame_load(const float* fr, int lane)
+{
+    MixedFrame F;
+    float* f = &F.M_x;
+#pragma unroll
+    for (int k = 0; k < kMixedFrameFloats; k++) f[k] = fr[k * 32 + lane];
+    return F;
+}
+
 // ---------------------------------------------------------------- integrator and photometer warps
 //
 // For fewer evaluations than the SMs' quarters hold warps.  There a warp alone is bound by its own
@@ -919,10 +936,23 @@ __host__ __device__ CF chi2_mixed(const DevModel& M, const ObsView& o, const dou
 constexpr int kPairTile = 8;
 constexpr int kPairPhotometers = 2;  // photometer warps of an integrator
 
+// The warps of a CTA of K integrators.  A warp runs on the quarter of the SM that its number modulo 4
+// names, and an integrator keeps most of its quarter busy: the integrators are the first K warps,
+// their photometers go to the quarters without one first, with warps that leave at once in between.
+//   K = 1: I P P      K = 2: I I P P . . P P      K = 3: I I I P P P P P . . . P      K = 4: 4 I, 8 P
+__host__ __device__ constexpr int pair_warps(int K) { return K == 1 ? 3 : K == 2 ? 8 : 12; }
+// The warp's place: K integrators 0 to K - 1, photometers K to 3 K - 1 (two consecutive ones the same
+// integrator's), -1 none.
+__host__ __device__ constexpr int pair_place(int K, int warp)
+{
+    return K == 2 ? (warp < 4 ? warp : warp < 6 ? -1 : warp - 2) : K == 3 ? (warp < 8 ? warp : warp < 11 ? -1 : 8) : warp;
+}
+
 // Shared memory of one integrator and its photometers: two tiles of angles as the state holds them, 32
 // wide (compact: three words each; RHS32: double-floats).  The photometers turn them into radians.
 struct PairTile {
     float ang[2][kPairTile][9][32];
+    float frame[kMixedFrameFloats][32];  // the evaluations' magnitude frames
 };
 
 template <bool RHS32>
@@ -969,7 +999,7 @@ __device__ __forceinline__ void pair_read(const float (*a)[32], int lane, bool t
 // parameters, their chi^2 and delta_V (in: the chain's last), whether there is another evaluation.
 struct PairChain {
     PairTile tile;
-    double par[AST_MAX_PARAMS][32];
+    double par[AST_MAX_PARAMS][32];  // under NUDGE
     double dv[AST_MAX_FILTERS][32];
     double chi2[32];
     int more;
@@ -991,6 +1021,7 @@ __device__ void pair_integrate(const DevModel& M, const ObsView& o, const double
     const int lane = threadIdx.x & 31;
     MixedState S;
     mixed_setup(M, params, S);
+    frame_store(&B.frame[0][0], lane, S.F);  // read after the first tile's barrier
     if (!RHS32) mixed_begin(S);
     int b = 0;
     for (int i0 = 0; i0 < M.n_data; i0 += kPairTile, b ^= 1) {
@@ -1003,8 +1034,8 @@ __device__ void pair_integrate(const DevModel& M, const ObsView& o, const double
     }
 }
 
-// A photometer warp's part: evaluation `chain` (0 to 31) of the integrator's, whose parameters params
-// are, by PW consecutive lanes; chi^2 and delta_V on each of them.
+// A photometer warp's part: evaluation `chain` (0 to 31) of the integrator's by PW consecutive lanes;
+// params (read under NUDGE only) are its parameters.  chi^2 and delta_V on each of the lanes.
 template <class CF, bool RHS32, int PW>
 __device__ CF pair_observe(const DevModel& M, const ObsView& o, const double* params, CF* delta_V, const float4* tab,
                            const PairTile& B, int chain, int id, int threads)
@@ -1014,22 +1045,23 @@ __device__ CF pair_observe(const DevModel& M, const ObsView& o, const double* pa
     MixedLast E;
     MixedQueue W;
     mixed_sums_begin(M, Q);
-    MixedState S;
-    mixed_setup(M, params, S);
+    MixedFrame S;
+    const bool torque = (M.flags & AST_TORQUE) != 0, bw = (M.flags & AST_BW_BALL) != 0;
     DfFrame F;
     if (M.flags & AST_NUDGE) F = make_df_frame(M, params);
     bool huge = false;
     int b = 0;
     for (int i0 = 0; i0 < M.n_data; i0 += kPairTile, b ^= 1) {
         pair_sync(id, threads);
+        if (i0 == 0) S = frame_load(&B.frame[0][0], chain);
         const int n = min(kPairTile, M.n_data - i0);
         for (int j0 = 0; j0 < n; j0 += PW) {
             const int j = min(j0 + sub, n - 1), i = i0 + j;
             const float v = o.v[i], w = o.w[i];
             const int m = o.f[i];
             df ang[3];
-            pair_read<RHS32>(B.ang[b][j], chain, S.torque, ang);
-            const float V = mixed_vmod(S.F, S.bw, DF_ADD(ang[0].hi, ang[0].lo), DF_ADD(ang[1].hi, ang[1].lo),
+            pair_read<RHS32>(B.ang[b][j], chain, torque, ang);
+            const float V = mixed_vmod(S, bw, DF_ADD(ang[0].hi, ang[0].lo), DF_ADD(ang[1].hi, ang[1].lo),
                                        DF_ADD(ang[2].hi, ang[2].lo), o, i);
             if (PW == 1) {
                 if (!huge) huge = !mixed_observe(M, o, F, tab, Q, E, W, i, v, w, m, V, ang);
@@ -1041,7 +1073,7 @@ __device__ CF pair_observe(const DevModel& M, const ObsView& o, const double* pa
                             wq = __shfl_sync(0xffffffffu, w, q, PW);
                 const int mq = __shfl_sync(0xffffffffu, m, q, PW);
                 if (j0 + q >= n || huge) continue;
-                if (M.flags & AST_NUDGE) pair_read<RHS32>(B.ang[b][j0 + q], chain, S.torque, ang);
+                if (M.flags & AST_NUDGE) pair_read<RHS32>(B.ang[b][j0 + q], chain, torque, ang);
                 huge = !mixed_observe(M, o, F, tab, Q, E, W, i0 + j0 + q, vq, wq, mq, Vq, ang);
             }
         }
@@ -1060,7 +1092,7 @@ __device__ CF pair_eval(const DevModel& M, const ObsView& o, double* params, uns
     for (int i = 0; i < M.n_params; i++) {
         const double a = __shfl_sync(0xffffffffu, params[i], src);
         if (!(live >> lane & 1u)) params[i] = a;
-        X.par[i][lane] = params[i];
+        if (M.flags & AST_NUDGE) X.par[i][lane] = params[i];
     }
     for (int m = 0; m < M.n_filters; m++) X.dv[m][lane] = (double)dvl[m];
     if (lane == 0) X.more = 1;
@@ -1083,7 +1115,8 @@ __device__ void pair_serve(const DevModel& M, const ObsView& o, const float4* ta
                            int threads)
 {
     double p[AST_MAX_PARAMS];
-    for (int i = 0; i < M.n_params; i++) p[i] = X.par[i][chain];
+    if (M.flags & AST_NUDGE)
+        for (int i = 0; i < M.n_params; i++) p[i] = X.par[i][chain];
     CF d[AST_MAX_FILTERS];
     for (int m = 0; m < M.n_filters; m++) d[m] = (CF)X.dv[m][chain];
     const CF r = pair_observe<CF, RHS32, PW>(M, o, p, d, tab, X.tile, chain, id, threads);
@@ -1114,22 +1147,6 @@ __device__ void pair_serve(const DevModel& M, const ObsView& o, const float4* ta
 __host__ __device__ constexpr int tile_warp_bytes(int T)
 {
     return 4 * (kMixedFrameFloats * 32 + 3 * 32 * (T + 1)) + 8 * 32 * (T + 1);
-}
-
-__device__ __forceinline__ void frame_store(float* fr, int lane, const MixedFrame& F)
-{
-    const float* f = &F.M_x;
-#pragma unroll
-    for (int k = 0; k < kMixedFrameFloats; k++) fr[k * 32 + lane] = f[k];
-}
-
-__device__ __forceinline__ MixedFrame frame_load(const float* fr, int lane)
-{
-    MixedFrame F;
-    float* f = &F.M_x;
-#pragma unroll
-    for (int k = 0; k < kMixedFrameFloats; k++) f[k] = fr[k * 32 + lane];
-    return F;
 }
 
 // Called by all 32 lanes of a warp at once (uniform control flow), each with its own params;
