@@ -292,6 +292,117 @@ __global__ void __launch_bounds__(KernShape<AST_PREC_MIXED>::tpb, KernShape<AST_
     if (n_fit) atomicAdd(&V.ctr[3], n_fit);
 }
 
+// ---------------------------------------------------------------- integrators and photometers
+//
+// Batches of too few chains to fill the SMs' quarters, mixed precision: fit_pair_kernel's pairing, each
+// integrator taking 32 consecutive chains at once (REFILL 32).  An integrator whose live chains belong
+// to different objects evaluates lane by lane as batch_kernel does.  Results are batch_kernel's bit for
+// bit.
+template <class CF>
+__global__ void __launch_bounds__(32 * pair_warps(kPairIntegrators), 1)
+    batch_pair_kernel(const BatchObj<CF>* objs, int n_objs, int K, FitView<CF> V, int64_t budget)
+{
+    constexpr int PW = kPairPhotometers, kThreads = 32 * (1 + PW);
+    __shared__ float4 trig[kTrigTable];
+    extern __shared__ __align__(16) unsigned char pair_smem[];
+    trig_table_fill(trig);
+    __syncthreads();
+    const int warp = pair_place(K, threadIdx.x >> 5);
+    const unsigned lane = threadIdx.x & 31u;
+    if (warp < 0) return;
+    const int pair = warp < K ? warp : (warp - K) / PW, id = 1 + pair;
+    PairChain& X = reinterpret_cast<PairChain*>(pair_smem)[pair];
+    if (warp >= K) {
+        const int chain = (warp - K) % PW * (32 / PW) + (int)lane / PW;
+        while (true) {
+            pair_sync(id, kThreads);
+            if (!X.more) return;
+            const BatchObj<CF>& B = objs[X.obj];
+            pair_serve<CF, false, PW>(B.M, B.L.view(B.obs, B.M.n_data), trig, X, chain, id, kThreads);
+        }
+    }
+    const int64_t s = ((int64_t)blockIdx.x * K + pair) * 32 + lane;
+    const int64_t S = V.S;
+    int64_t gchain = V.chain[s];
+    int k = 0;
+    SlotState<CF> R;
+    R.chain = -1;
+    R.st = V.st[s];
+    R.l = V.it[s];
+    R.ev = V.ev[s];
+    for (int m = 0; m < AST_MAX_FILTERS; m++) R.dvl[m] = (CF)0;
+    if (gchain >= 0) {
+        k = find_obj(objs, n_objs, gchain);
+        R.chain = gchain - objs[k].chain0;
+        for (int m = 0; m < objs[k].M.n_filters; m++) R.dvl[m] = (CF)V.dv[(int64_t)m * S + s];
+    }
+    unsigned long long n_ev = 0, n_fit = 0, n_done = 0;
+    for (int64_t used = 0; used < budget; used++) {
+        if (__all_sync(0xffffffffu, gchain < 0)) {
+            unsigned long long base = 0;
+            if (lane == 0) base = atomicAdd(&V.ctr[0], 32ull);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (base >= (unsigned long long)V.n_chains) break;
+            const unsigned long long c = base + lane;
+            if (c < (unsigned long long)V.n_chains) {
+                gchain = (int64_t)c;
+                batch_start<CF>(objs, n_objs, V, s, gchain, k, R);
+            }
+        }
+        // Cancelled objects drop their chains (counted as finished) without an evaluation.
+        if (gchain >= 0 && objs[k].cancelled) {
+            atomicAdd(objs[k].done, 1ull);
+            n_done++;
+            gchain = -1;
+            R.chain = -1;
+        }
+        CF p[AST_MAX_PARAMS];
+        double params[AST_MAX_PARAMS];
+        for (int i = 0; i < AST_MAX_PARAMS; i++) params[i] = 0.0;
+        int rej = 1;
+        if (gchain >= 0) {
+            const BatchObj<CF>& B = objs[k];
+            slot_point<CF>(B.M, obj_view(V, B), s, R, p);
+            rej = x2params<CF>(B.M, B.reopt, p, params);
+        }
+        const unsigned live = __ballot_sync(0xffffffffu, !rej);
+        const int k0 = __shfl_sync(0xffffffffu, k, live ? __ffs(live) - 1 : 0);
+        const bool same = __all_sync(0xffffffffu, rej || k == k0);
+        CF fv = (CF)kHuge;
+        if (live && same) {
+            const BatchObj<CF>& B = objs[k0];
+            if (lane == 0) X.obj = k0;
+            fv = pair_eval<CF, false>(B.M, B.L.view(B.obs, B.M.n_data), params, live, R.dvl, trig, X, id, kThreads);
+        } else if (!rej) {
+            const BatchObj<CF>& B = objs[k];
+            fv = eval_point<CF, AST_PREC_MIXED>(B.M, B.L.view(B.obs, B.M.n_data), params, R.dvl, trig);
+        }
+        if (gchain >= 0) {
+            const BatchObj<CF>& B = objs[k];
+            if (!rej) {
+                R.ev++;
+                n_ev++;
+            }
+            if (slot_apply<CF>(B.M, obj_view(V, B), s, R, p, rej, rej ? (CF)kHuge : fv, n_fit)) {
+                atomicAdd(B.done, 1ull);
+                n_done++;
+                gchain = -1;
+                R.chain = -1;
+            }
+        }
+    }
+    pair_stop(X, id, kThreads);
+    V.chain[s] = gchain;
+    V.st[s] = R.st;
+    V.it[s] = R.l;
+    V.ev[s] = R.ev;
+    if (gchain >= 0)
+        for (int m = 0; m < objs[k].M.n_filters; m++) V.dv[(int64_t)m * S + s] = (double)R.dvl[m];
+    if (n_done) atomicAdd(&V.ctr[1], n_done);
+    if (n_ev) atomicAdd(&V.ctr[2], n_ev);
+    if (n_fit) atomicAdd(&V.ctr[3], n_fit);
+}
+
 // ---------------------------------------------------------------- cooperative chains
 //
 // For a lightly loaded server (few chains in flight, each 5000 sequential evaluations), a chain
@@ -646,6 +757,7 @@ struct ast_pool {
     // launch geometry
     int tpb = 256, refill = 1, ctas = 0;
     int tile = 0;       // warp-tiled evaluation with tiles of this many observations (0: none)
+    int pair = 0;       // integrators of a CTA of batch_pair_kernel (0: another kernel)
     int lanes = 1;      // lanes per chain: 1, or kCoopLanes (cooperative chains, servers only)
     size_t smem = 0;    // dynamic shared memory of the launch
     // entries
@@ -888,7 +1000,7 @@ static FitView<CF> pool_view(const ast_pool& P)
     V.x = (CF*)P.x; V.f = (CF*)P.f; V.ind = P.ind; V.x0 = (CF*)P.x0; V.xr = (CF*)P.xr; V.fr = (CF*)P.fr;
     V.st = P.st; V.it = P.it; V.ev = P.ev; V.chain = P.chain; V.dv = P.dv; V.ctr = P.ctr;
     V.S = P.S;
-    V.n_slots = (int64_t)P.ctas * P.tpb / P.lanes;
+    V.n_slots = P.pair ? (int64_t)P.ctas * P.pair * 32 : (int64_t)P.ctas * P.tpb / P.lanes;
     V.n_chains = P.chain_end;
     V.last_stage = 1;
     return V;
@@ -931,6 +1043,7 @@ static decltype(&batch_tile_kernel<double, 16>) batch_tile_ptr(int T)
 template <class CF, int PREC>
 static int pool_geometry(ast_pool& P, int tpb, int refill, int tile = 0)
 {
+    P.pair = 0;
     if (P.lanes > 1) return coop_geometry<CF, PREC>(P, 128);
     if (tpb < 32 || tpb > 256 || (tpb & 31)) return ast_set_error(AST_E_INVALID, "batch: tpb must be 32..256, x32");
     tpb = std::min(tpb, KernShape<PREC>::tpb);  // the kernel's launch bounds
@@ -964,11 +1077,39 @@ static int pool_geometry(ast_pool& P, int tpb, int refill, int tile = 0)
     return AST_OK;
 }
 
-// One launch of the pool's kernel (thread per chain or warp per object, or the warp-tiled
-// evaluation) on its stream.
+// Threads per CTA as reported: of a paired launch those that run chains, a size that can be asked for.
+static int pool_tpb(const ast_pool& P) { return P.pair ? 32 * P.pair : P.tpb; }
+
+// The geometry of a batch when none is asked for: integrators and photometers where the batch's chains are
+// few (pair_integrators) and the slot pool holds them, else thread per chain.
+template <class CF, int PREC>
+static int batch_geometry_default(ast_pool& P)
+{
+    const int k = PREC == AST_PREC_MIXED ? pair_integrators(P.chain_end, P.sm_count) : 0;
+    const int64_t ctas = k ? (P.chain_end + 32 * k - 1) / (32 * k) : 0;
+    if (!k || P.chain_end <= 0 || ctas * 32 * k > P.n_slots) return pool_geometry<CF, PREC>(P, 256, 1);
+    P.pair = k;
+    P.tpb = 32 * pair_warps(k);
+    P.refill = 32;
+    P.tile = 0;
+    P.smem = sizeof(PairChain) * k;
+    P.ctas = (int)ctas;
+    AST_CUDA(cudaFuncSetAttribute(batch_pair_kernel<CF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
+    return AST_OK;
+}
+
+// One launch of the pool's kernel (thread per chain or warp per object, the warp-tiled evaluation, or
+// integrators and photometers) on its stream.
 template <class CF, int PREC>
 static void launch_pool(ast_pool& P, const FitView<CF>& V, int64_t budget)
 {
+    if constexpr (PREC == AST_PREC_MIXED) {
+        if (P.pair) {
+            batch_pair_kernel<CF><<<P.ctas, P.tpb, P.smem, P.stream>>>((const BatchObj<CF>*)P.d_objs, (int)P.active.size(),
+                                                                       P.pair, V, budget);
+            return;
+        }
+    }
     if constexpr (std::is_same<CF, double>::value && PREC == AST_PREC_MIXED) {
         if (P.tile) {  // pool_geometry allows tiles for mixed-precision ACC pools only
             batch_tile_ptr(P.tile)<<<P.ctas, P.tpb, P.smem, P.stream>>>((const BatchObj<double>*)P.d_objs,
@@ -1079,7 +1220,7 @@ static int batch_run_t(ast_batch* B, const ast_batch_launch* tune, double* kerne
     if (tune) {
         if ((rc = pool_geometry<CF, PREC>(P, tune->tpb, tune->refill, tune->tile))) return rc;
     } else if (!P.ctas) {
-        if ((rc = pool_geometry<CF, PREC>(P, 256, 1))) return rc;
+        if ((rc = batch_geometry_default<CF, PREC>(P))) return rc;
     }
     if ((rc = batch_capture<CF, PREC>(B))) return rc;
     AST_CUDA(cudaEventRecord(P.ev0, P.stream));
@@ -1189,7 +1330,7 @@ static int batch_step_t(ast_batch* B, int64_t evals_per_slot, int32_t* done, dou
     ast_pool& P = B->P;
     batch_order(B);
     int rc;
-    if (!P.ctas && (rc = pool_geometry<CF, PREC>(P, 256, 1))) return rc;
+    if (!P.ctas && (rc = batch_geometry_default<CF, PREC>(P))) return rc;
     if ((rc = upload_table<CF>(P))) return rc;
     const FitView<CF> V = pool_view<CF>(P);
     AST_CUDA(cudaEventRecord(P.ev0, P.stream));
@@ -1309,7 +1450,7 @@ extern "C" int ast_batch_set_geometry(ast_batch* B, const ast_batch_launch* g)
 extern "C" int ast_batch_geometry(ast_batch* B, ast_batch_launch* out)
 {
     if (!B || !out) return ast_set_error(AST_E_INVALID, "ast_batch_geometry: NULL argument");
-    out->tpb = B->P.tpb;
+    out->tpb = pool_tpb(B->P);
     out->refill = B->P.refill;
     out->ctas = B->P.ctas;
     out->tile = B->P.tile;
@@ -1323,7 +1464,7 @@ extern "C" int ast_batch_counters(ast_batch* B, int64_t* n_evals, int64_t* n_fit
     if (!B) return ast_set_error(AST_E_INVALID, "ast_batch_counters: NULL batch");
     if (n_evals) *n_evals = (int64_t)B->P.evals;
     if (n_fits) *n_fits = (int64_t)B->P.fits;
-    if (tpb) *tpb = B->P.tpb;
+    if (tpb) *tpb = pool_tpb(B->P);
     if (refill) *refill = B->P.refill;
     if (ctas) *ctas = B->P.ctas;
     return AST_OK;

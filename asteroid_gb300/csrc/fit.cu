@@ -641,7 +641,7 @@ extern "C" int ast_set_stage_wait(ast_ctx* c, int32_t polls)
 extern "C" int ast_fit_launch(ast_ctx* c, int32_t* tpb, int32_t* ctas, int32_t* minb, int32_t* smem)
 {
     if (!c || !c->fb.ctr) return ast_set_error(AST_E_INVALID, "ast_fit_launch: no fit");
-    if (tpb) *tpb = c->run.tpb;
+    if (tpb) *tpb = c->run.pair ? 32 * c->run.pair : c->run.tpb;  // threads that run chains
     if (ctas) *ctas = c->run.ctas;
     if (minb) *minb = c->run.minb;
     if (smem) *smem = (int32_t)c->run.smem;

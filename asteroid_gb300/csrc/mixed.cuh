@@ -1003,6 +1003,7 @@ struct PairChain {
     double dv[AST_MAX_FILTERS][32];
     double chi2[32];
     int more;
+    int obj;  // of a batch, the evaluations' object
 };
 
 // The barrier of one integrator and its photometers (id 1 to 15).

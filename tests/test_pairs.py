@@ -39,7 +39,7 @@ def test_fits_by_pairs_equal_threads(gpu, flags, chains, group, kw):
         kw["params0"] = P[0]
     with api.Engine(model, obs) as eng:
         a = eng.fit(n_chains=chains, group_size=group, seed=9, **kw)
-        assert eng.fit_launch()["tpb"] in (96, 256, 384)
+        assert eng.fit_launch()["tpb"] <= 128 and eng.fit_launch()["smem"] > 18000  # a PairChain
         b = eng.fit(n_chains=chains, group_size=group, seed=9, tpb=32, **kw)
         eng.fit_begin(n_chains=chains, group_size=group, seed=9, **kw)  # in bounded steps
         for _ in range(1000):
@@ -50,3 +50,32 @@ def test_fits_by_pairs_equal_threads(gpu, flags, chains, group, kw):
         for k in ("best_f", "best_params", "best_dv", "chain_f"):
             assert np.array_equal(getattr(r, k), getattr(b, k), equal_nan=True), k
         assert r.n_evals == b.n_evals and r.n_fits == b.n_fits
+
+
+@pytest.mark.parametrize("acc", [True, False])
+def test_batches_by_pairs_equal_threads(gpu, acc):
+    """A batch of few chains runs by pairs unless a geometry is asked for: objects of uneven size, a warp that
+    straddles two of them, one with NUDGE, run whole and in bounded steps."""
+    end = ",ACC" if acc else ""
+    objects = [_object(f + end, n, nf, n, span) for f, n, nf, span in
+               (("TORQUE", 60, 2, 1.0), ("BC,INTERP", 33, 1, 2.0), ("BW_BALL", 29, 4, 0.5), ("INTERP,NUDGE", 41, 1, 1.0))]
+    chains = (64, 48, 16, 33)  # the second and third share a warp
+
+    def batch(steps=0, **geometry):
+        with api.Batch(precision=api.PREC_MIXED, acc=acc) as b:
+            for (model, obs, P), c in zip(objects, chains):
+                b.add(model, obs, n_chains=c, group_size=c, seed=4, evals_cap=30)
+            if steps:
+                while not b.step(steps)[0]:
+                    pass
+            else:
+                b.run(**geometry)
+            c = b.counters()
+            return [b.result(i) for i in range(len(objects))], c
+
+    ref, c0 = batch(tpb=128, refill=1)
+    for got, c in (batch(), batch(steps=5)):
+        assert c["refill"] == 32 and c["tpb"] == 32 and c["n_evals"] == c0["n_evals"]
+        for r, g in zip(ref, got):
+            for k in ("best_f", "best_params", "best_dv"):
+                assert np.array_equal(getattr(r, k), getattr(g, k), equal_nan=True)
