@@ -41,6 +41,10 @@ constexpr int kPeriodTpb = 256;
 constexpr int kFreqs = 8;                       // frequencies per thread
 constexpr int kFreqTile = kPeriodTpb * kFreqs;  // frequencies per CTA
 constexpr int kChunk = 2048;                    // intervals per shared-memory pass (16 KB)
+// Least intervals of a CTA's slice: enough to be worth its 2048 atomic additions, few enough to fill the
+// SMs with the intervals of a curve of some hundred minima (5 801 distinct: 41 us, with 512 88; 24 538:
+// 99 us, with 512 118).
+constexpr int kSlice = 128;
 constexpr float kMarginBase = 1e-7f;            // rounding of x_hi - r + x_lo (<= 2^-25) and 0.1f vs 0.1
 // Periodogram constants of misc.c:131-135.
 constexpr double kSgm = 0.1, kDt0 = 1.0 / 24.0, kDt2 = 80.0 / 24.0, kS0 = 3;
@@ -224,23 +228,23 @@ __global__ void __launch_bounds__(kPeriodTpb) interval_count_kernel(const double
         if (f0 + k < nn && cnt[k]) atomicAdd(&counts[f0 + k], (unsigned int)cnt[k]);
 }
 
-// Device buffers of one call, freed on every return.
+// Trial frequencies and their periods (misc.c:137-144), in the reference's operations.
+__global__ void frequencies_kernel(double* fr, double* dt1, double fr2, double range)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= kBins) return;
+    fr[i] = __dadd_rn(fr2, __dmul_rn((double)i / (double)(kBins - 1), range));
+    dt1[i] = 1 / fr[i];
+}
+
+// Device memory of one call, one allocation, freed on every return.
 struct PeriodScratch {
-    double* tm = nullptr;
-    unsigned long long* keys = nullptr;  // hash table of distinct intervals
-    unsigned int* mult = nullptr;        // their multiplicities
-    double* dt = nullptr;                // distinct intervals, packed
-    unsigned int* wt = nullptr;          // their multiplicities, packed
-    unsigned int* misc = nullptr;        // [0] distinct intervals, [1] table full
-    double* fr = nullptr;
-    double* dt1 = nullptr;
-    unsigned int* counts = nullptr;
+    char* base = nullptr;
     cudaStream_t s = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr, em = nullptr;
     ~PeriodScratch()
     {
-        cudaFree(tm); cudaFree(keys); cudaFree(mult); cudaFree(dt); cudaFree(wt); cudaFree(misc);
-        cudaFree(fr); cudaFree(dt1); cudaFree(counts);
+        cudaFree(base);
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
         if (em) cudaEventDestroy(em);
@@ -274,11 +278,8 @@ extern "C" int ast_minima(int32_t device, int32_t n_plot, const double* t, const
     out->n_intervals = m;
     // Trial frequencies (misc.c:137-144).
     const double fr0 = 1 / kDt0, fr2 = 1 / kDt2;
-    std::vector<double> fr(kBins), dt1(kBins);
-    for (int i = 0; i < kBins; i++) {
-        fr[i] = fr2 + (double)i / (double)(kBins - 1) * (fr0 - fr2);
-        dt1[i] = 1 / fr[i];
-    }
+    std::vector<double> fr(kBins);
+    for (int i = 0; i < kBins; i++) fr[i] = fr2 + (double)i / (double)(kBins - 1) * (fr0 - fr2);
     std::vector<unsigned int> cnt(kBins, 0);
     if (m > 0) {
         // x = dt * fr must stay below 2^21 for the rounding of the count kernel.
@@ -290,59 +291,61 @@ extern "C" int ast_minima(int32_t device, int32_t n_plot, const double* t, const
         PeriodScratch d;
         uint64_t table = 1024;
         while (table < 2 * (uint64_t)m) table <<= 1;
-        if (cudaMalloc(&d.tm, sizeof(double) * n) != cudaSuccess ||
-            cudaMalloc(&d.keys, sizeof(unsigned long long) * table) != cudaSuccess ||
-            cudaMalloc(&d.mult, sizeof(unsigned int) * table) != cudaSuccess ||
-            cudaMalloc(&d.dt, sizeof(double) * m) != cudaSuccess || cudaMalloc(&d.wt, sizeof(unsigned int) * m) != cudaSuccess ||
-            cudaMalloc(&d.misc, sizeof(unsigned int) * 2) != cudaSuccess ||
-            cudaMalloc(&d.fr, sizeof(double) * kBins) != cudaSuccess ||
-            cudaMalloc(&d.dt1, sizeof(double) * kBins) != cudaSuccess ||
-            cudaMalloc(&d.counts, sizeof(unsigned int) * kBins) != cudaSuccess) {
+        // What starts at zero first: the hash table of distinct intervals and their multiplicities, the
+        // counts, [0] the number of distinct intervals and [1] table full; then the minima, the distinct
+        // intervals packed with their multiplicities, the frequencies and periods.
+        auto up = [](size_t v) { return (v + 255) / 256 * 256; };
+        const size_t o_keys = 0, o_mult = o_keys + up(8 * table), o_counts = o_mult + up(4 * table),
+                     o_misc = o_counts + up(4 * kBins), zero = o_misc + 256, o_tm = zero, o_dt = o_tm + up(8 * (size_t)n),
+                     o_wt = o_dt + up(8 * (size_t)m), o_fr = o_wt + up(4 * (size_t)m), o_dt1 = o_fr + up(8 * kBins);
+        if (cudaMalloc(&d.base, o_dt1 + up(8 * kBins)) != cudaSuccess) {
             cudaGetLastError();
             return ast_set_error(AST_E_NOMEM, "ast_minima: cudaMalloc failed (%lld intervals)", (long long)m);
         }
+        unsigned long long* d_keys = (unsigned long long*)(d.base + o_keys);
+        unsigned int *d_mult = (unsigned int*)(d.base + o_mult), *d_counts = (unsigned int*)(d.base + o_counts),
+                     *d_misc = (unsigned int*)(d.base + o_misc), *d_wt = (unsigned int*)(d.base + o_wt);
+        double *d_tm = (double*)(d.base + o_tm), *d_dt = (double*)(d.base + o_dt), *d_fr = (double*)(d.base + o_fr),
+               *d_dt1 = (double*)(d.base + o_dt1);
         AST_CUDA(cudaStreamCreateWithFlags(&d.s, cudaStreamNonBlocking));
         AST_CUDA(cudaEventCreate(&d.e0));
         AST_CUDA(cudaEventCreate(&d.e1));
         AST_CUDA(cudaEventCreate(&d.em));
-        AST_CUDA(cudaMemcpyAsync(d.tm, tm.data(), sizeof(double) * n, cudaMemcpyHostToDevice, d.s));
-        AST_CUDA(cudaMemcpyAsync(d.fr, fr.data(), sizeof(double) * kBins, cudaMemcpyHostToDevice, d.s));
-        AST_CUDA(cudaMemcpyAsync(d.dt1, dt1.data(), sizeof(double) * kBins, cudaMemcpyHostToDevice, d.s));
-        AST_CUDA(cudaMemsetAsync(d.counts, 0, sizeof(unsigned int) * kBins, d.s));
-        AST_CUDA(cudaMemsetAsync(d.keys, 0, sizeof(unsigned long long) * table, d.s));
-        AST_CUDA(cudaMemsetAsync(d.mult, 0, sizeof(unsigned int) * table, d.s));
-        AST_CUDA(cudaMemsetAsync(d.misc, 0, sizeof(unsigned int) * 2, d.s));
+        AST_CUDA(cudaMemsetAsync(d.base, 0, zero, d.s));
+        frequencies_kernel<<<(kBins + 255) / 256, 256, 0, d.s>>>(d_fr, d_dt1, fr2, fr0 - fr2);
+        AST_CUDA(cudaGetLastError());
+        AST_CUDA(cudaMemcpyAsync(d_tm, tm.data(), sizeof(double) * n, cudaMemcpyHostToDevice, d.s));
         int cur = 0, sms = 0;
         AST_CUDA(cudaGetDevice(&cur));
         AST_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cur));
         AST_CUDA(cudaEventRecord(d.e0, d.s));
-        pair_hash_kernel<<<n - 1, 256, 0, d.s>>>(d.tm, n, d.keys, d.mult, table - 1, d.misc + 1);
+        pair_hash_kernel<<<n - 1, 256, 0, d.s>>>(d_tm, n, d_keys, d_mult, table - 1, d_misc + 1);
         AST_CUDA(cudaGetLastError());
         compact_kernel<<<(unsigned)std::min<uint64_t>((table + 255) / 256, (uint64_t)sms * 8), 256, 0, d.s>>>(
-            d.keys, d.mult, table, d.dt, d.wt, d.misc);
+            d_keys, d_mult, table, d_dt, d_wt, d_misc);
         AST_CUDA(cudaGetLastError());
         unsigned int misc[2] = {0, 0};
-        AST_CUDA(cudaMemcpyAsync(misc, d.misc, sizeof(misc), cudaMemcpyDeviceToHost, d.s));
+        AST_CUDA(cudaMemcpyAsync(misc, d_misc, sizeof(misc), cudaMemcpyDeviceToHost, d.s));
         AST_CUDA(cudaStreamSynchronize(d.s));
         if (misc[1]) return ast_set_error(AST_E_INVALID, "ast_minima: interval table full");
         const int64_t mu = misc[0];  // distinct intervals
         out->n_distinct = mu;
         const int tiles = (kBins + kFreqTile - 1) / kFreqTile;
         // One wave: as many (tile, slice) CTAs as are resident at once, all with the same work
-        // (each slice at least 512 intervals).
+        // (each slice at least kSlice intervals).
         int occ = 0;
         AST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, interval_count_kernel, kPeriodTpb, 0));
         int64_t slices = std::max<int64_t>(1, (int64_t)sms * std::max(occ, 1) / tiles);
-        slices = std::max<int64_t>(1, std::min<int64_t>(slices, (mu + 511) / 512));
+        slices = std::max<int64_t>(1, std::min<int64_t>(slices, (mu + kSlice - 1) / kSlice));
         const int64_t per_slice = (mu + slices - 1) / slices;
         slices = (mu + per_slice - 1) / per_slice;
         const float margin = kMarginBase + (float)(1e-13 * x_max);
         AST_CUDA(cudaEventRecord(d.em, d.s));
-        interval_count_kernel<<<dim3(tiles, (unsigned)slices), kPeriodTpb, 0, d.s>>>(d.dt, d.wt, mu, per_slice, d.fr,
-                                                                                     d.dt1, kBins, margin, d.counts);
+        interval_count_kernel<<<dim3(tiles, (unsigned)slices), kPeriodTpb, 0, d.s>>>(d_dt, d_wt, mu, per_slice, d_fr,
+                                                                                     d_dt1, kBins, margin, d_counts);
         AST_CUDA(cudaGetLastError());
         AST_CUDA(cudaEventRecord(d.e1, d.s));
-        AST_CUDA(cudaMemcpyAsync(cnt.data(), d.counts, sizeof(unsigned int) * kBins, cudaMemcpyDeviceToHost, d.s));
+        AST_CUDA(cudaMemcpyAsync(cnt.data(), d_counts, sizeof(unsigned int) * kBins, cudaMemcpyDeviceToHost, d.s));
         AST_CUDA(cudaStreamSynchronize(d.s));
         float ms = 0, cms = 0;
         AST_CUDA(cudaEventElapsedTime(&ms, d.e0, d.e1));
