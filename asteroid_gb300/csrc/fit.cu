@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(32, 8) fit_group_kernel(DevModel M, const void
         for (int m = 0; m < NF; m++) dv[m] = R.dvl[m];
         __syncwarp();
         // A group without a point takes part without a result.
-        CF fv = chi2_fp64_group<CF, G>(M, o, params, dv);
+        CF fv = chi2_fp64_group<CF, G, TrigLibrary>(M, o, params, dv);
         int finish = 0;
         if (R.chain >= 0) {
             if (rej) {

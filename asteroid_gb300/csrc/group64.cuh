@@ -6,8 +6,9 @@
 // its warp to itself takes the number of its FP64 instructions times 64 cycles, and spreading its
 // components over idle lanes divides that number: eight lanes hold the six components of the state,
 // one stage's two sin/cos pairs are one call, its products two instructions, its update one; the
-// magnitudes of G observations, one on each lane of the group, are one evaluation.  159 instructions
-// an RK4 step and 467 / G + 2 an observation, against 340 and 467 on one lane (torque).
+// magnitudes of G observations, one on each lane of the group, are one evaluation.  123 instructions
+// an RK4 step and 440 / G + 2 an observation, against 268 and 440 on one lane (torque, the table's
+// sine and cosine of trig64.cuh; 159 and 467 against 340 and 467 with the library's).
 //
 // Every operation is the thread path's (chi2_fp64) on the same operands, sums in observation order,
 // so the results are its results bit for bit.  All 32 lanes of the warp call together, each group
@@ -21,11 +22,12 @@ __device__ __forceinline__ double shfl8(double v, int src) { return __shfl_sync(
 
 // Derivative of the lane's component at the stage value f of every lane: roles 0..2 the angular
 // velocity (mu_a = mu[role], mu_b = mu[3 + role]), 3 phi, 4 theta, 5 to 7 psi.
+template <class TRIG>
 __device__ __forceinline__ double group_rhs_torque(int role, double f, double mu_a, double mu_b)
 {
     const double th = shfl8(f, 4), ps = shfl8(f, 5);
     double s, c;
-    sincos(role & 1 ? ps : th, &s, &c);
+    TRIG::sincos(role & 1 ? ps : th, &s, &c);
     const double s4 = shfl8(s, 0), c4 = shfl8(c, 0), s5 = shfl8(s, 1), c5 = shfl8(c, 1);
     const double y0 = shfl8(f, 0), y1 = shfl8(f, 1), y2 = shfl8(f, 2);
     // mu_a y' y'' + mu_b; (phi's numerator) y0 s5 + y1 c5; (theta) y0 c5 - y1 s5
@@ -46,12 +48,12 @@ __device__ __forceinline__ double group_rhs_torque(int role, double f, double mu
 // it does there -- as a value of its own in the first three stages, in a fused multiply-add in the
 // last, where nothing but the step's sum needs it beside (the compiler's choice there; the tests
 // compare the two paths bit for bit).
-template <bool LAST>
+template <bool LAST, class TRIG>
 __device__ __forceinline__ double group_rhs_free(int role, double f, const double* mu, double mu_a)
 {
     const double th = shfl8(f, 4), ps = shfl8(f, 5);
     double s, c;
-    sincos(role & 1 ? 2.0 * ps : th, &s, &c);
+    TRIG::sincos(role & 1 ? 2.0 * ps : th, &s, &c);
     const double s1 = shfl8(s, 0), c1 = shfl8(c, 0), s2 = shfl8(s, 1), c2 = shfl8(c, 1);
     // (phi) mu1 - mu2 c2; (theta) mu0 mu2 s1, whose sum with -0 is itself
     const double x = role == 4 ? mu_a : -mu[2];
@@ -66,16 +68,16 @@ __device__ __forceinline__ double group_rhs_free(int role, double f, const doubl
 }
 
 // One RK4 step of the lane's component (rk4_step).
-template <bool TORQUE>
+template <bool TORQUE, class TRIG>
 __device__ __forceinline__ double group_step(int role, double y, double h, const double* mu, double mu_a, double mu_b)
 {
     auto rhs = [&](double f) {
-        return TORQUE ? group_rhs_torque(role, f, mu_a, mu_b) : group_rhs_free<false>(role, f, mu, mu_a);
+        return TORQUE ? group_rhs_torque<TRIG>(role, f, mu_a, mu_b) : group_rhs_free<false, TRIG>(role, f, mu, mu_a);
     };
     const double K1 = rhs(y);
     const double K2 = rhs(y + 0.5 * h * K1);
     const double K3 = rhs(y + 0.5 * h * K2);
-    const double K4 = TORQUE ? rhs(y + h * K3) : group_rhs_free<true>(role, y + h * K3, mu, mu_a);
+    const double K4 = TORQUE ? rhs(y + h * K3) : group_rhs_free<true, TRIG>(role, y + h * K3, mu, mu_a);
     return y + 1 / 6.0 * h * (K1 + 2 * K2 + 2 * K3 + K4);
 }
 
@@ -83,7 +85,7 @@ __device__ __forceinline__ double group_step(int role, double y, double h, const
 // and delta_V on every lane.  vmod_out, when non-null, receives the model magnitude of every
 // observation (the reference's Nplot > 0 mode, cuda.c:699-704, without the delta_V shift); ang_out
 // the Euler angles (phi, theta, psi); geo_out the renderer's geometry.
-template <class CF, int G>
+template <class CF, int G, class TRIG>
 __device__ CF chi2_fp64_group(const DevModel& M, const ObsView& o, const double* params, CF* delta_V,
                               double* vmod_out = nullptr, double* ang_out = nullptr, double* geo_out = nullptr)
 {
@@ -114,10 +116,10 @@ __device__ CF chi2_fp64_group(const DevModel& M, const ObsView& o, const double*
             const double h = o.h[i];
             if (S.torque) {
 #pragma unroll 1
-                for (int l = 0; l < N_steps; l++) y = group_step<true>(role, y, h, S.mu, mu_a, mu_b);
+                for (int l = 0; l < N_steps; l++) y = group_step<true, TRIG>(role, y, h, S.mu, mu_a, mu_b);
             } else {
 #pragma unroll 1
-                for (int l = 0; l < N_steps; l++) y = group_step<false>(role, y, h, S.mu, mu_a, mu_b);
+                for (int l = 0; l < N_steps; l++) y = group_step<false, TRIG>(role, y, h, S.mu, mu_a, mu_b);
             }
         }
         {
@@ -133,7 +135,7 @@ __device__ CF chi2_fp64_group(const DevModel& M, const ObsView& o, const double*
         const int i0 = i & ~(G - 1), n = i - i0 + 1;
         const bool own = lane < n;
         const int k = own ? i0 + lane : i;
-        const double Vmod = fp64_vmod(M, params, S, phi, theta, psi, o, k,
+        const double Vmod = fp64_vmod<TRIG>(M, params, S, phi, theta, psi, o, k,
                                       geo_out && own ? geo_out + (int64_t)kAstGeo * k : nullptr);
         if (own && vmod_out) vmod_out[k] = Vmod;
         if (own && ang_out) {

@@ -12,6 +12,7 @@
 #include <math.h>
 #include <stdint.h>
 #include "asteroid_gb300.h"
+#include "trig64.cuh"
 
 #ifndef AST_HD
 #define AST_HD __host__ __device__ __forceinline__
@@ -306,11 +307,12 @@ AST_HD void params2x(const DevModel& M, const double* params, CF* x)
 // Euler equations with constant body-frame torque + Euler-angle kinematics (cuda.c:44-58).
 // y = (Omega_i, Omega_s, Omega_l, phi, theta, psi); mu = ((Is-Il)/Ii, (Il-Ii)/Is, (Ii-Is)/Il,
 // Ki/Ii, Ks/Is, Kl/Il) with Il = 1.
+template <class TRIG>
 __device__ __forceinline__ void ode_torque(const double* y, double* f, const double* mu)
 {
     double s5, c5, s4, c4;
-    sincos(y[5], &s5, &c5);
-    sincos(y[4], &s4, &c4);
+    TRIG::sincos(y[5], &s5, &c5);
+    TRIG::sincos(y[4], &s4, &c4);
     f[0] = mu[0] * y[1] * y[2] + mu[3];
     f[1] = mu[1] * y[2] * y[0] + mu[4];
     f[2] = mu[2] * y[0] * y[1] + mu[5];
@@ -320,31 +322,32 @@ __device__ __forceinline__ void ode_torque(const double* y, double* f, const dou
 }
 
 // Torque-free Euler angles (cuda.c:68-75): y = (phi, theta, psi), mu = (L, Ip, Im).
+template <class TRIG>
 __device__ __forceinline__ void ode_free(const double* y, double* f, const double* mu)
 {
     double s2, c2, s1, c1;
-    sincos(2.0 * y[2], &s2, &c2);
-    sincos(y[1], &s1, &c1);
+    TRIG::sincos(2.0 * y[2], &s2, &c2);
+    TRIG::sincos(y[1], &s1, &c1);
     f[0] = mu[0] * (mu[1] - mu[2] * c2);
     f[1] = mu[0] * mu[2] * s1 * s2;
     f[2] = c1 * (mu[0] - f[0]);
 }
 
 // One classic RK4 step of size h (cuda.c:348-372), in the reference's operation order.
-template <int NODE>
+template <int NODE, class TRIG>
 __device__ __forceinline__ void rk4_step(double* y, double h, const double* mu)
 {
     double f[NODE], K1[NODE], K2[NODE], K3[NODE], K4[NODE];
-    if (NODE == 6) ode_torque(y, K1, mu); else ode_free(y, K1, mu);
+    if (NODE == 6) ode_torque<TRIG>(y, K1, mu); else ode_free<TRIG>(y, K1, mu);
 #pragma unroll
     for (int j = 0; j < NODE; j++) f[j] = y[j] + 0.5 * h * K1[j];
-    if (NODE == 6) ode_torque(f, K2, mu); else ode_free(f, K2, mu);
+    if (NODE == 6) ode_torque<TRIG>(f, K2, mu); else ode_free<TRIG>(f, K2, mu);
 #pragma unroll
     for (int j = 0; j < NODE; j++) f[j] = y[j] + 0.5 * h * K2[j];
-    if (NODE == 6) ode_torque(f, K3, mu); else ode_free(f, K3, mu);
+    if (NODE == 6) ode_torque<TRIG>(f, K3, mu); else ode_free<TRIG>(f, K3, mu);
 #pragma unroll
     for (int j = 0; j < NODE; j++) f[j] = y[j] + h * K3[j];
-    if (NODE == 6) ode_torque(f, K4, mu); else ode_free(f, K4, mu);
+    if (NODE == 6) ode_torque<TRIG>(f, K4, mu); else ode_free<TRIG>(f, K4, mu);
 #pragma unroll
     for (int j = 0; j < NODE; j++) y[j] = y[j] + 1 / 6.0 * h * (K1[j] + 2 * K2[j] + 2 * K3[j] + K4[j]);
 }
@@ -448,6 +451,7 @@ __device__ __forceinline__ void write_geo(double* g, double b, double c, double 
 // Model magnitude at observation i for the Euler angles (phi, theta, psi): the body axes
 // (cuda.c:432-473), then the brightness (cuda.c:475-689).  geo, when non-null, receives the kAstGeo
 // inputs of the renderer.
+template <class TRIG>
 __device__ __forceinline__ double fp64_vmod(const DevModel& M, const double* params, const Fp64Setup& F, double phi,
                                             double theta, double psi, const ObsView& o, int i, double* geo)
 {
@@ -455,7 +459,7 @@ __device__ __forceinline__ double fp64_vmod(const DevModel& M, const double* par
     const double M_x = F.M_x, M_y = F.M_y, M_z = F.M_z;
     const double XM_x = F.XM_x, XM_z = F.XM_z, YM_x = F.YM_x, YM_y = F.YM_y, YM_z = F.YM_z;
     double cos_phi, sin_phi;
-    sincos(phi, &sin_phi, &cos_phi);
+    TRIG::sincos(phi, &sin_phi, &cos_phi);
     double N_x = XM_x * cos_phi + YM_x * sin_phi;
     double N_y = YM_y * sin_phi;
     double N_z = XM_z * cos_phi + YM_z * sin_phi;
@@ -463,7 +467,7 @@ __device__ __forceinline__ double fp64_vmod(const DevModel& M, const double* par
     double p_y = N_z * M_x - N_x * M_z;
     double p_z = N_x * M_y - N_y * M_x;
     double cos_theta, sin_theta;
-    sincos(theta, &sin_theta, &cos_theta);
+    TRIG::sincos(theta, &sin_theta, &cos_theta);
     double a_x = M_x * cos_theta + p_x * sin_theta;
     double a_y = M_y * cos_theta + p_y * sin_theta;
     double a_z = M_z * cos_theta + p_z * sin_theta;
@@ -471,7 +475,7 @@ __device__ __forceinline__ double fp64_vmod(const DevModel& M, const double* par
     const double w_y = a_z * N_x - a_x * N_z;
     const double w_z = a_x * N_y - a_y * N_x;
     double sin_psi, cos_psi;
-    sincos(psi, &sin_psi, &cos_psi);
+    TRIG::sincos(psi, &sin_psi, &cos_psi);
     const double b_x = N_x * cos_psi + w_x * sin_psi;
     const double b_y = N_y * cos_psi + w_y * sin_psi;
     const double b_z = N_z * cos_psi + w_z * sin_psi;
@@ -639,7 +643,7 @@ __device__ __forceinline__ CF fp64_finish(const DevModel& M, const double* sum_y
 // chi2one (cuda.c:81-1011) for one parameter vector over the object's observations.
 // Returns CHI_FLOAT; delta_V is written only when the evaluation runs to the end (the NUDGE
 // "more than M_MAX minima" exit returns 1e30 and leaves it, as the reference does).
-template <class CF>
+template <class CF, class TRIG>
 __device__ CF chi2_fp64(const DevModel& M, const ObsView& o, const double* params, CF* delta_V)
 {
     const int flags = M.flags;
@@ -655,16 +659,16 @@ __device__ CF chi2_fp64(const DevModel& M, const ObsView& o, const double* param
             const double h = o.h[i];
             if (S.torque) {
 #pragma unroll 1
-                for (int l = 0; l < N_steps; l++) rk4_step<6>(S.y, h, S.mu);
+                for (int l = 0; l < N_steps; l++) rk4_step<6, TRIG>(S.y, h, S.mu);
             } else {
 #pragma unroll 1
-                for (int l = 0; l < N_steps; l++) rk4_step<3>(S.y, h, S.mu);
+                for (int l = 0; l < N_steps; l++) rk4_step<3, TRIG>(S.y, h, S.mu);
             }
         }
         const double phi = S.torque ? S.y[3] : S.y[0];
         const double theta = S.torque ? S.y[4] : S.y[1];
         const double psi = S.torque ? S.y[5] : S.y[2];
-        const double Vmod = fp64_vmod(M, params, S, phi, theta, psi, o, i, nullptr);
+        const double Vmod = fp64_vmod<TRIG>(M, params, S, phi, theta, psi, o, i, nullptr);
         {   // Per-filter sums (cuda.c:707-714).
             const int m = o.f[i];
             const double yv = o.v[i] - Vmod;

@@ -75,7 +75,7 @@ __global__ void rmsd_setup_kernel(DevModel M, const void* g_obs, ObsLayout L, co
     CF dv[AST_MAX_FILTERS];
     CF f0;
     if (PREC == AST_PREC_FP64)
-        f0 = chi2_fp64_group<CF, 32>(M, o, p, dv);  // the warp together
+        f0 = chi2_fp64_group<CF, 32, TrigLibrary>(M, o, p, dv);  // the warp together
     else
         f0 = eval_point<CF, PREC>(M, o, p, dv, trig);
     if (threadIdx.x != 0) return;

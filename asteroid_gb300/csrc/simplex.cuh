@@ -137,7 +137,7 @@ template <class CF, int PREC>
 __device__ __forceinline__ CF eval_point(const DevModel& M, const ObsView& o, const double* params, CF* dv,
                                          const float4* trig)
 {
-    if (PREC == AST_PREC_FP64) return chi2_fp64<CF>(M, o, params, dv);
+    if (PREC == AST_PREC_FP64) return chi2_fp64<CF, TrigLibrary>(M, o, params, dv);
     return chi2_mixed<CF, PREC == AST_PREC_MIXED_RHS32>(M, o, params, dv, trig);
 }
 
@@ -414,7 +414,7 @@ __device__ void group_best_body(const DevModel& M, const FitView<CF>& V, int64_t
     if (best < kHuge) x2params<CF>(M, V.reopt, xb, p);
     if (fp64_obs && best < kHuge) {
         double d[AST_MAX_FILTERS];
-        f = chi2_fp64_group<double, 32>(M, *fp64_obs, p, d);
+        f = chi2_fp64_group<double, 32, TrigTable>(M, *fp64_obs, p, d);
     }
     if (threadIdx.x != 0) return;
     out_f[g] = f;
