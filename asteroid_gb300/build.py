@@ -130,14 +130,16 @@ def build_parity_engine(force: bool = False) -> Path:
     build into _build/parity/libasteroid_gb300.so.  Test infrastructure for the FP64 parity
     check against the reference kernel compiled the same way (oracle/build_ref.sh nofma): both
     sides then round every product and sum separately, so only the order of operations and
-    CUDA's libm are left to differ.  Loaded in a child process through AST_ENGINE_LIB."""
+    CUDA's libm are left to differ.  It evaluates with CUDA's sincos in the reference's
+    expressions (AST_LIBRARY_TRIG, as the FP64 simplex search does), not with the table and the
+    rearranged magnitude of the evaluation kernels.  Loaded in a child process through AST_ENGINE_LIB."""
     build_engine()
     PARITY.mkdir(exist_ok=True)
     nvcc = _nvcc()
     src = PKG / "csrc" / "engine.cu"
     obj = PARITY / "engine.o"
     if force or _stale(obj, [src] + _headers()):
-        _run([nvcc, *GENCODE, "-lineinfo", "-O3", "-std=c++17", "-fmad=false", "-Xcompiler",
+        _run([nvcc, *GENCODE, "-lineinfo", "-O3", "-std=c++17", "-fmad=false", "-DAST_LIBRARY_TRIG", "-Xcompiler",
               "-fPIC,-O2,-ffp-contract=off", f"-I{INCLUDE}", f"-I{PKG / 'host'}", "-c", str(src), "-o", str(obj)])
     objs = [obj] + [BUILD / (Path(s).stem + ".o") for s in CU_SOURCES if Path(s).stem != "engine"]
     objs += [BUILD / (Path(s).stem + ".o") for s in C_SOURCES]

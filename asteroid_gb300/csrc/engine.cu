@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(128, MINB) eval_kernel(DevModel M, const void*
         for (int m = 0; m < M.n_filters; m++) d[m] = 0;
         CF r;
         if (PREC == AST_PREC_FP64)
-            r = chi2_fp64<CF, TrigTable>(M, o, p, d);
+            r = chi2_fp64<CF, TrigEval>(M, o, p, d);
         else
             r = chi2_mixed<CF, PREC == AST_PREC_MIXED_RHS32>(M, o, p, d, trig);
         chi2[k] = (double)r;
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(32, 8) eval_group_kernel(DevModel M, const voi
     for (int i = 0; i < M.n_params; i++) p[i] = params[kk * M.n_params + i];
     CF d[AST_MAX_FILTERS];
     for (int m = 0; m < M.n_filters; m++) d[m] = 0;
-    const CF r = chi2_fp64_group<CF, G, TrigTable>(M, o, p, d);
+    const CF r = chi2_fp64_group<CF, G, TrigEval>(M, o, p, d);
     if (k >= n || threadIdx.x % G) return;
     chi2[k] = (double)r;
     if (dv)
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(32, 1) model_curve_kernel(DevModel M, const vo
     double d[AST_MAX_FILTERS];
     DevModel M2 = M;
     M2.flags &= ~AST_NUDGE;  // the curve is the brightness model alone
-    chi2_fp64_group<double, 32, TrigTable>(M2, o, p, d, vmod, nullptr, geo);
+    chi2_fp64_group<double, 32, TrigEval>(M2, o, p, d, vmod, nullptr, geo);
 }
 
 // Euler angles at every observation along the FP64 (one warp) or the mixed-precision integration (one
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(32, 1) model_angles_kernel(DevModel M, const v
     DevModel M2 = M;
     M2.flags &= ~AST_NUDGE;
     if (PREC == AST_PREC_FP64) {
-        chi2_fp64_group<double, 32, TrigTable>(M2, o, p, d, nullptr, ang);
+        chi2_fp64_group<double, 32, TrigEval>(M2, o, p, d, nullptr, ang);
         return;
     }
     trig_table_fill(trig, kTrigEntries<PREC>);

@@ -7,8 +7,8 @@
 // components over idle lanes divides that number: eight lanes hold the six components of the state,
 // one stage's two sin/cos pairs are one call, its products two instructions, its update one; the
 // magnitudes of G observations, one on each lane of the group, are one evaluation.  123 instructions
-// an RK4 step and 440 / G + 2 an observation, against 268 and 440 on one lane (torque, the table's
-// sine and cosine of trig64.cuh; 159 and 467 against 340 and 467 with the library's).
+// an RK4 step and 290 / G + 2 an observation, against 268 and 290 on one lane (torque, evaluations; 159
+// and 467 against 340 and 467 in the simplex search, trig64.cuh).
 //
 // Every operation is the thread path's (chi2_fp64) on the same operands, sums in observation order,
 // so the results are its results bit for bit.  All 32 lanes of the warp call together, each group

@@ -1,10 +1,12 @@
 // model.cuh -- the light-curve model in FP64: device tables, the x <-> params maps, the ODE
 // right-hand sides and the chi^2 of one parameter vector.
 //
-// The plain path must agree with the reference kernel to 1e-12 relative chi^2, so every
-// expression below keeps the operand order and the float/double types of the reference's
+// The plain path must agree with the reference kernel to 1e-12 relative chi^2, so the
+// expressions below keep the operand order and the float/double types of the reference's
 // chi2one (cuda.c:81-1011), x2params (cuda.c:1120-1319) and params2x (cuda.c:1016-1115);
-// nvcc then makes the same multiply-add contractions in both.  What differs is the data
+// nvcc then makes the same multiply-add contractions in both.  The evaluation kernels' sine and
+// cosine (trig64.cuh) and Lommel-Seeliger magnitude (ls_algebraic) are their own: they move a
+// chi^2 by no more than another choice of contractions does.  What differs is the data
 // flow: quantities that do not depend on the parameters (per-interval RK4 step count and
 // size, the ephemeris interpolation of E and S) are computed once per object by
 // prep_obs_kernel with the same expressions, instead of once per evaluation.
@@ -359,6 +361,7 @@ struct Fp64Setup {
     double M_x, M_y, M_z, XM_x, XM_z, YM_x, YM_y, YM_z;
     double y[6], mu[6];
     double b_ph, c_ph, kappa;
+    double ib2, ic2;  // 1 / b_ph^2, 1 / c_ph^2
     double cos_phR, sin_phR, cos_thR, sin_thR;  // BW_BALL's brightness frame
     bool torque, bw;
 };
@@ -429,6 +432,8 @@ __device__ __forceinline__ void fp64_setup(const DevModel& M, const double* para
         S.b_ph = (flags & AST_BC) ? AST_P(b) : bt;
         S.c_ph = (flags & AST_BC) ? AST_P(c) : ct;
     }
+    S.ib2 = 1.0 / (S.b_ph * S.b_ph);
+    S.ic2 = 1.0 / (S.c_ph * S.c_ph);
 }
 
 // Doubles of the renderer's geometry at one observation (compute_rgb's arguments, cuda.c:576-586).
@@ -446,6 +451,33 @@ __device__ __forceinline__ void write_geo(double* g, double b, double c, double 
     g[11] = bx; g[12] = by; g[13] = bz;
     g[14] = cx; g[15] = cy; g[16] = cz;
     g[17] = ax; g[18] = ay; g[19] = az;
+}
+
+// The Lommel-Seeliger magnitude of cuda.c:664-689 without its inverse and half-angle functions.
+// alpha' is the angle between the scaled vectors to the Sun and the Earth, lambda' the one
+// between the first and their sum; nu = alpha' - lambda' is then the one between their sum and the second, and
+// each has its sine and cosine from the same triangle:
+//     cos lambda' = (S + E cos alpha') / |S + E|,  sin lambda' = E sin alpha' / |S + E|,  nu with S and E exchanged,
+// and cot(x/2) = (1 + cos x) / sin x, or sin x / (1 - cos x) where cos x < 0.  290 FP64 instructions an
+// observation against 440: 20 011 evaluations of 480 points 22.6 -> 17.7 ms, a curve of 20 000 points 132 ->
+// 127.  The error is no larger: 1.2e-16 rms of log10 either way for alpha' of 0.1 to 2, against
+// multiprecision, and 70 times smaller close to pi.
+AST_HD double ls_algebraic(double b, double c, double ib2, double ic2, double Sb, double Sc, double Sa, double Eb, double Ec,
+                           double Ea)
+{
+    const double Tb = Sb * ib2, Tc = Sc * ic2;
+    const double S = sqrt(Sb * Tb + Sc * Tc + Sa * Sa);
+    const double E = sqrt(Eb * Eb * ib2 + Ec * Ec * ic2 + Ea * Ea);
+    const double SE = S * E;
+    const double ca = (Eb * Tb + Ec * Tc + Sa * Ea) / SE;
+    const double sa = sqrt(1.0 - ca * ca);
+    const double inv = 1.0 / sqrt(S * S + E * E + 2 * SE * ca);
+    const double cl = (S + E * ca) * inv, sl = E * sa * inv;
+    const double cn = (E + S * ca) * inv, sn = S * sa * inv;
+    const bool pl = !signbit(cl), pn = !signbit(cn);  // (the integer pipe's; a comparison is the FP64 unit's)
+    const double lp = pl ? 1.0 + cl : sl, lq = pl ? sl : 1.0 - cl;
+    const double np = pn ? 1.0 + cn : sn, nq = pn ? sn : 1.0 - cn;
+    return -2.5 * log10(b * c * SE * inv * (cn + cl - sl * sn * log(lp * np / (lq * nq))));
 }
 
 // Model magnitude at observation i for the Euler angles (phi, theta, psi): the body axes
@@ -519,18 +551,22 @@ __device__ __forceinline__ double fp64_vmod(const DevModel& M, const double* par
         if (geo)
             write_geo(geo, b, c, E_x1, E_y1, E_z1, Ep_b, Ep_c, Ep_a, Sp_b, Sp_c, Sp_a,
                       b_x, b_y, b_z, c_x, c_y, c_z, a_x, a_y, a_z);
-        const double scalar_Sun = sqrt(Sp_b * Sp_b / (b * b) + Sp_c * Sp_c / (c * c) + Sp_a * Sp_a);
-        const double scalar_Earth = sqrt(Ep_b * Ep_b / (b * b) + Ep_c * Ep_c / (c * c) + Ep_a * Ep_a);
-        const double cos_alpha_p = (Sp_b * Ep_b / (b * b) + Sp_c * Ep_c / (c * c) + Sp_a * Ep_a) / (scalar_Sun * scalar_Earth);
-        const double sin_alpha_p = sqrt(1.0 - cos_alpha_p * cos_alpha_p);
-        const double alpha_p = atan2(sin_alpha_p, cos_alpha_p);
-        const double scalar = sqrt(scalar_Sun * scalar_Sun + scalar_Earth * scalar_Earth + 2 * scalar_Sun * scalar_Earth * cos_alpha_p);
-        const double cos_lambda_p = (scalar_Sun + scalar_Earth * cos_alpha_p) / scalar;
-        const double sin_lambda_p = scalar_Earth * sin_alpha_p / scalar;
-        const double lambda_p = atan2(sin_lambda_p, cos_lambda_p);
-        Vmod = -2.5 * log10(b * c * scalar_Sun * scalar_Earth / scalar *
-                            (cos(lambda_p - alpha_p) + cos_lambda_p +
-                             sin_lambda_p * sin(lambda_p - alpha_p) * log(1.0 / tan(0.5 * lambda_p) / tan(0.5 * (alpha_p - lambda_p)))));
+        if (TRIG::kAlgebraic) {
+            Vmod = ls_algebraic(b, c, F.ib2, F.ic2, Sp_b, Sp_c, Sp_a, Ep_b, Ep_c, Ep_a);
+        } else {
+            const double scalar_Sun = sqrt(Sp_b * Sp_b / (b * b) + Sp_c * Sp_c / (c * c) + Sp_a * Sp_a);
+            const double scalar_Earth = sqrt(Ep_b * Ep_b / (b * b) + Ep_c * Ep_c / (c * c) + Ep_a * Ep_a);
+            const double cos_alpha_p = (Sp_b * Ep_b / (b * b) + Sp_c * Ep_c / (c * c) + Sp_a * Ep_a) / (scalar_Sun * scalar_Earth);
+            const double sin_alpha_p = sqrt(1.0 - cos_alpha_p * cos_alpha_p);
+            const double alpha_p = atan2(sin_alpha_p, cos_alpha_p);
+            const double scalar = sqrt(scalar_Sun * scalar_Sun + scalar_Earth * scalar_Earth + 2 * scalar_Sun * scalar_Earth * cos_alpha_p);
+            const double cos_lambda_p = (scalar_Sun + scalar_Earth * cos_alpha_p) / scalar;
+            const double sin_lambda_p = scalar_Earth * sin_alpha_p / scalar;
+            const double lambda_p = atan2(sin_lambda_p, cos_lambda_p);
+            Vmod = -2.5 * log10(b * c * scalar_Sun * scalar_Earth / scalar *
+                                (cos(lambda_p - alpha_p) + cos_lambda_p +
+                                 sin_lambda_p * sin(lambda_p - alpha_p) * log(1.0 / tan(0.5 * lambda_p) / tan(0.5 * (alpha_p - lambda_p)))));
+        }
     }
     return Vmod;
 }

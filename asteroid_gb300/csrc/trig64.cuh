@@ -158,10 +158,18 @@ AST_HD void sincos_tab(double x, double* s, double* c)
 // between chi^2 of models from the prior that no step resolves, where a sine's last bit decides (one of
 // 2048 such chains then takes another number of evaluations).
 struct TrigTable {
+    static constexpr bool kAlgebraic = true;  // and ls_algebraic (model.cuh)
     static __device__ __forceinline__ void sincos(double x, double* s, double* c) { sincos_tab(x, s, c); }
 };
 struct TrigLibrary {
+    static constexpr bool kAlgebraic = false;
     static __device__ __forceinline__ void sincos(double x, double* s, double* c) { ::sincos(x, s, c); }
 };
+// The parity build (build_parity_engine) evaluates as the search does, in the reference's expressions.
+#ifdef AST_LIBRARY_TRIG
+using TrigEval = TrigLibrary;
+#else
+using TrigEval = TrigTable;
+#endif
 
 }  // namespace ast

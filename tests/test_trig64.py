@@ -1,4 +1,5 @@
-"""The FP64 table sine and cosine (csrc/trig64.cuh), compiled for the host, against mpmath."""
+"""The FP64 table sine and cosine (csrc/trig64.cuh) and the evaluation kernels' Lommel-Seeliger
+magnitude (csrc/model.cuh), compiled for the host, against mpmath."""
 import ctypes as C
 import subprocess
 from pathlib import Path
@@ -14,13 +15,16 @@ STEP = 2 * np.pi / 1024
 
 
 @pytest.fixture(scope="module")
-def sincos(tmp_path_factory):
+def lib(tmp_path_factory):
     out = tmp_path_factory.mktemp("trig64") / "libtrig64_harness.so"
     subprocess.run([build._nvcc(), "-shared", "-Xcompiler", "-fPIC,-ffp-contract=off", "-O2", "-std=c++17",
                     f"-I{build.PKG / 'csrc'}", f"-I{build.INCLUDE}", str(ROOT / "tests" / "host" / "trig64_harness.cu"),
                     "-o", str(out)], check=True, capture_output=True)
-    lib = C.CDLL(str(out))
+    return C.CDLL(str(out))
 
+
+@pytest.fixture(scope="module")
+def sincos(lib):
     def run(x):
         x = np.ascontiguousarray(x, np.float64)
         r = np.empty((len(x), 2))
@@ -52,3 +56,40 @@ def test_beyond(sincos):
     r = sincos(x)
     with np.errstate(invalid="ignore"):
         np.testing.assert_allclose(r, np.stack([np.sin(x), np.cos(x)], 1), rtol=0, atol=2.3e-16)
+
+
+# Round and flat bodies, the angle between the scaled vectors on both sides of a right angle (each branch of the
+# half-angle quotients).
+@pytest.mark.parametrize("b,c", [(1.0, 1.0), (0.7, 0.4), (0.9, 0.02), (0.1, 0.05)])
+def test_magnitude(lib, b, c):
+    rng = np.random.default_rng(5)
+    n = 300
+    v = np.empty((n, 8))
+    v[:, 0], v[:, 1] = b, c
+    S = rng.normal(size=(n, 3))
+    E = S + rng.normal(size=(n, 3)) * rng.choice([0.1, 1.0, 5.0], (n, 1))
+    v[:, 2:5] = S / np.linalg.norm(S, axis=1, keepdims=True)
+    v[:, 5:8] = E / np.linalg.norm(E, axis=1, keepdims=True)
+    got = np.empty(n)
+    lib.h_ls_algebraic(n, v.ctypes.data_as(C.c_void_p), got.ctypes.data_as(C.c_void_p))
+    with mpmath.workprec(160):
+        compared = 0
+        for vi, g in zip(v, got):
+            sb, sc, sa, eb, ec, ea = (mpmath.mpf(float(x)) for x in vi[2:])
+            B, K = mpmath.mpf(b), mpmath.mpf(c)
+            s = mpmath.sqrt(sb * sb / (B * B) + sc * sc / (K * K) + sa * sa)
+            e = mpmath.sqrt(eb * eb / (B * B) + ec * ec / (K * K) + ea * ea)
+            ca = (sb * eb / (B * B) + sc * ec / (K * K) + sa * ea) / (s * e)
+            al = mpmath.acos(ca)
+            if not 0.05 < al < 2.5:
+                continue
+            compared += 1
+            sc_ = mpmath.sqrt(s * s + e * e + 2 * s * e * ca)
+            la = mpmath.atan2(e * mpmath.sin(al) / sc_, (s + e * ca) / sc_)
+            want = -2.5 * mpmath.log10(B * K * s * e / sc_ * (
+                mpmath.cos(la - al) + mpmath.cos(la) + mpmath.sin(la) * mpmath.sin(la - al) *
+                mpmath.log(1 / mpmath.tan(la / 2) / mpmath.tan((al - la) / 2))))
+            # cos alpha' carries eight roundings, which sin alpha' turns into an angle; a magnitude moves by up to
+            # 2.5 / ln 10 d ln B / d alpha', below 10 up to alpha' = 2.5.  The rest: twenty roundings of the factors.
+            assert abs(g - want) <= (10 * 8 / mpmath.sin(al) + 1.09 * 20) * 2.0 ** -53 + 2.0 ** -52 * abs(want)
+        assert compared > 50
