@@ -5,8 +5,8 @@
 // FMA chains of 1 to 8 independent operations, 1 to 32 active lanes).  So an evaluation that has
 // its warp to itself takes the number of its FP64 instructions times 64 cycles, and spreading its
 // components over idle lanes divides that number: eight lanes hold the six components of the state,
-// one stage's two sin/cos pairs are one call, its products two instructions, its update one; the
-// magnitudes of G observations, one on each lane of the group, are one evaluation.  123 instructions
+// one stage's two sines and two cosines are one call, its products two instructions, its update one; the
+// magnitudes of G observations, one on each lane of the group, are one evaluation.  111 instructions
 // an RK4 step and 290 / G + 2 an observation, against 268 and 290 on one lane (torque, evaluations; 159
 // and 467 against 340 and 467 in the simplex search, trig64.cuh).
 //
@@ -26,9 +26,8 @@ template <class TRIG>
 __device__ __forceinline__ double group_rhs_torque(int role, double f, double mu_a, double mu_b)
 {
     const double th = shfl8(f, 4), ps = shfl8(f, 5);
-    double s, c;
-    TRIG::sincos(role & 1 ? ps : th, &s, &c);
-    const double s4 = shfl8(s, 0), c4 = shfl8(c, 0), s5 = shfl8(s, 1), c5 = shfl8(c, 1);
+    const double v = TRIG::sin_or_cos(role & 1 ? ps : th, role & 2);
+    const double s4 = shfl8(v, 0), s5 = shfl8(v, 1), c4 = shfl8(v, 2), c5 = shfl8(v, 3);
     const double y0 = shfl8(f, 0), y1 = shfl8(f, 1), y2 = shfl8(f, 2);
     // mu_a y' y'' + mu_b; (phi's numerator) y0 s5 + y1 c5; (theta) y0 c5 - y1 s5
     const double p = role < 3 ? mu_a : y1;
@@ -52,9 +51,8 @@ template <bool LAST, class TRIG>
 __device__ __forceinline__ double group_rhs_free(int role, double f, const double* mu, double mu_a)
 {
     const double th = shfl8(f, 4), ps = shfl8(f, 5);
-    double s, c;
-    TRIG::sincos(role & 1 ? 2.0 * ps : th, &s, &c);
-    const double s1 = shfl8(s, 0), c1 = shfl8(c, 0), s2 = shfl8(s, 1), c2 = shfl8(c, 1);
+    const double v = TRIG::sin_or_cos(role & 1 ? 2.0 * ps : th, role & 2);
+    const double s1 = shfl8(v, 0), s2 = shfl8(v, 1), c1 = shfl8(v, 2), c2 = shfl8(v, 3);
     // (phi) mu1 - mu2 c2; (theta) mu0 mu2 s1, whose sum with -0 is itself
     const double x = role == 4 ? mu_a : -mu[2];
     const double y = role == 4 ? s1 : c2;

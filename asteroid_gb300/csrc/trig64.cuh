@@ -4,9 +4,10 @@
 // warp) or 19 (four warps on an SM), and most of an RK4 step's were the sine and cosine of two angles
 // in each stage: sincos() issues 25.  With a point of a table of 1024 angles next to x, at
 // most pi/1024 away, three terms of each series are enough and x's sine and cosine take 16; memory,
-// integer and predicate instructions run beside them.  159 -> 123 instructions an RK4 step on lanes of
-// a group, 340 -> 268 on one lane (torque); 20 011 evaluations of 480 points 27.1 -> 22.6 ms, one of 300
-// points 4.48 -> 3.98, 337 of 611 (black-and-white ball) 8.9 -> 6.9, a curve of 20 000 points 153 -> 132.
+// integer and predicate instructions run beside them.  159 -> 111 instructions an RK4 step on lanes of
+// a group, 340 -> 268 on one lane (torque); 20 011 evaluations of 480 points 27.1 -> 22.6 ms (sine and
+// cosine on one lane); one of 300 points 4.48 -> 3.98 and 3.60 with each on a lane of its own, 337 of 611
+// (black-and-white ball) 8.9 -> 6.9 and 5.9, with the curve of 20 000 points 153 -> 132 and 117 (ls_algebraic in between).
 //
 // The table holds the points' sine and cosine as unevaluated sums of two doubles: the results are
 // within 0.6 ulp of 1 for one rounding of each sum, 1.2 ulp of themselves near the zeros
@@ -126,7 +127,10 @@ static __host__ __device__ __noinline__ void beyond(double x, double* s, double*
 // (both terms are multiples of 2^-62 unless k = 0, and the difference is below 2^-8), and d's rest
 // enters with another; k is within half a step and its own product's rounding, 2^-5 of one at |x| =
 // 2^40.  Infinities and NaN give NaN.  Every rounding explicit: the same bits in every kernel.
-AST_HD void sincos_tab(double x, double* s, double* c)
+//
+// shift: added to the table point, kTrig64 / 4 for (cos x, -sin x); the points a quarter turn on are
+// the same numbers, so the bits are, too.  Without c only the first is computed, in 13 instructions.
+AST_HD void sincos_tab(double x, double* s, double* c, int shift = 0)
 {
     constexpr double kStep = 2.0 * trig64::kPi2.hi / kTrig64, kStepLo = 2.0 * trig64::kPi2.lo / kTrig64;
     const double magic = 6755399441055744.0;  // 1.5 2^52
@@ -142,15 +146,18 @@ AST_HD void sincos_tab(double x, double* s, double* c)
     memcpy(&bits, &kb, 8);
 #endif
     if (((uint32_t)(xb >> 32) & 0x7fffffffu) - 0x42700000u < 0x3d800000u) {  // 2^40 <= |x| < infinity
-        trig64::beyond(x, s, c);
+        double sx, cx;
+        trig64::beyond(x, &sx, &cx);
+        *s = shift ? cx : sx;
+        if (c) *c = shift ? -sx : cx;
         return;
     }
-    const trig64::Point P = trig64::point((int)(bits & (kTrig64 - 1)));
+    const trig64::Point P = trig64::point((int)((bits + (uint32_t)shift) & (kTrig64 - 1)));
     const double r2 = DD_MUL(r, r);
     const double sr = DD_FMA(DD_MUL(r, r2), DD_FMA(r2, 1.0 / 120.0, -1.0 / 6.0), r);  // sin r
     const double v = DD_MUL(r2, DD_FMA(r2, 1.0 / 24.0, -0.5));                        // cos r - 1
     *s = DD_ADD(P.s, DD_FMA(P.c, sr, DD_FMA(P.s, v, P.sl)));
-    *c = DD_ADD(P.c, DD_FMA(-P.s, sr, DD_FMA(P.c, v, P.cl)));
+    if (c) *c = DD_ADD(P.c, DD_FMA(-P.s, sr, DD_FMA(P.c, v, P.cl)));
 }
 
 // The sine and cosine of an FP64 evaluation.  Evaluations proper (ast_eval_batch, curves, the FP64 chi^2
@@ -160,10 +167,22 @@ AST_HD void sincos_tab(double x, double* s, double* c)
 struct TrigTable {
     static constexpr bool kAlgebraic = true;  // and ls_algebraic (model.cuh)
     static __device__ __forceinline__ void sincos(double x, double* s, double* c) { sincos_tab(x, s, c); }
+    static __device__ __forceinline__ double sin_or_cos(double x, bool cosine)
+    {
+        double r;
+        sincos_tab(x, &r, nullptr, cosine ? kTrig64 / 4 : 0);
+        return r;
+    }
 };
 struct TrigLibrary {
     static constexpr bool kAlgebraic = false;
     static __device__ __forceinline__ void sincos(double x, double* s, double* c) { ::sincos(x, s, c); }
+    static __device__ __forceinline__ double sin_or_cos(double x, bool cosine)
+    {
+        double s, c;
+        ::sincos(x, &s, &c);
+        return cosine ? c : s;
+    }
 };
 // The parity build (build_parity_engine) evaluates as the search does, in the reference's expressions.
 #ifdef AST_LIBRARY_TRIG
