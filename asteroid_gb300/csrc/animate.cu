@@ -5,11 +5,13 @@
 // snapshot, shades its own pixel: four lines of sight through the pixel's corners intersected with
 // the triaxial ellipsoid, Lambert-like shading between terminator, shadow and sunlit colours, a
 // red spot around the end of the b axis.  Here the recursion runs once (ast_model_geometry: one
-// thread, the fit's FP64 evaluation) and render_kernel shades every pixel of every frame from
+// warp, the FP64 evaluation) and render_kernel shades every pixel of every frame from
 // that geometry: one CTA per 32 x 8 tile of a frame, frames on the grid's y dimension, the frame's
 // 20 doubles in shared memory, each line of sight through a pixel corner evaluated once and shared
-// by the four pixels that meet there.  The arithmetic is the reference's, in FP64, with every
-// rounding explicit (no contracted multiply-adds) so that the CPU restatement reproduces each byte.
+// by the four pixels that meet there.  The bytes are those of the reference's FP64 arithmetic with
+// every rounding explicit (no contracted multiply-adds), so that the CPU restatement reproduces
+// each one: values are computed in double-float with a bound on their error, and again in that FP64
+// arithmetic where a comparison or a byte's rounding lies within the bound.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>

@@ -16,7 +16,9 @@
 //              are idle, so the lanes of a warp always integrate the same light curve (no
 //              divergence between objects of different lengths, at the cost of idle lanes
 //              while the warp's last chain finishes).
-// ast_batch_tune times both, with several CTA sizes, on the caller's batch.
+// ast_batch_tune times both, with several CTA sizes, on the caller's batch.  A mixed batch of so few
+// chains that they leave quarters of the SMs idle runs integrator and photometer warps
+// (batch_pair_kernel) unless a geometry is set or tuned.
 //
 // Batch (ast_batch_*): all objects are added, then one CUDA graph -- slot reset, the persistent
 // kernel run to completion, the per-group argmin of every object -- is captured once and
@@ -1059,7 +1061,7 @@ static int pool_geometry(ast_pool& P, int tpb, int refill, int tile = 0)
         smem = (size_t)(tpb / 32) * tile_warp_bytes(tile);
         auto kern = batch_tile_ptr(tile);
         // Always raised to the request: without it, dynamic and static shared memory together stay
-        // within 48 KB (the sin/cos table takes 4 KB of that).
+        // within 48 KB (the sin/cos tables take 45 KB of that).
         AST_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         AST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, tpb, smem));
     } else {

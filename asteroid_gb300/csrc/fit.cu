@@ -14,6 +14,9 @@
 //     observation times only), so the hot loop does not diverge;
 //   * a launch runs until every slot has spent its evaluation budget or the pool is empty and
 //     saves its state, so a fit can be advanced in bounded steps (bench, serving);
+//   * a search of fewer chains than fill the SMs gives each chain more of one: a group of 8 or 32
+//     lanes (fit_group_kernel, FP64) or an integrator and two photometer warps for 32 chains
+//     (fit_pair_kernel, mixed);
 //   * stages (-Nstages) are separate pools; between them group_best_kernel takes each group's
 //     best chain (the reference's per-block argmin and hand-off, cuda.c:1769-1805).
 // The chain semantics (random start, initial simplex, sort with ties to the last index,

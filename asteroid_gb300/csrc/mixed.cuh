@@ -4,8 +4,8 @@
 // FP64) is bound by the FP64 pipe.  Here the fixed-step RK4 of the Euler equations and Euler
 // angles (cuda.c:13-77, 319-372) runs entirely on the FP32 pipe: the state, the stage
 // combinations and the right-hand side (including sin/cos of the Euler angles) are double-float
-// values (dfloat.cuh), ~48-bit significands, which keeps the integrated rotation phase (up to
-// ~1e5 rad over a long light curve) accurate to ~1e-10 rad.  The brightness model at each
+// values (dfloat.cuh), ~48-bit significands, with compact angles (turn.cuh), which keeps the
+// integrated rotation phase (up to ~1e5 rad over a long light curve) accurate to ~1e-10 rad.  The brightness model at each
 // observation (cuda.c:432-689) is evaluated in plain FP32 from the double-float angles reduced
 // to [-pi, pi].  FP64 is left for the per-evaluation set-up (initial angles and angular
 // velocity, cuda.c:195-252), the parameter-independent ephemeris interpolation (hoisted per
@@ -74,7 +74,8 @@ AST_HD float ls_magnitude_f(float Sb, float Sc, float Sa, float Eb, float Ec, fl
     return DF_MUL(-2.5f, log10f(DF_MUL(DF_MUL(DF_MUL(bc, sS), sE) / scalar, B)));
 }
 
-// The rotation ODEs (cuda.c:13-77) in double-float, on the state in packed pairs (df2): the
+// The rotation ODEs (cuda.c:13-77) in double-float on the angles themselves, for the steps that
+// turn.cuh declines (spin_step_general), on the state in packed pairs (df2): the
 // sin and cos of the two angles the right-hand side needs are one df2_sincos, its products and
 // quotient are the scalar double-float operations on the pairs' halves.  Pair layout, torque:
 // (y0, y1), (y2, phi), (psi, theta), where y0..y2 are the body-frame angular velocities of

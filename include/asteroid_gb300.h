@@ -405,9 +405,9 @@ int ast_set_stage_wait(ast_ctx* ctx, int32_t polls);
 /* Number of chain slots (persistent threads) the fit kernel of this context runs. */
 int64_t ast_fit_slots(ast_ctx* ctx);
 
-/* Launch geometry ast_fit_begin chose: threads per CTA, CTAs, register budget (CTAs of 256
- * threads per SM the kernel was compiled for) and dynamic shared memory bytes.  Any pointer may
- * be NULL.  No reference counterpart (the reference's geometry is the compile-time
+/* Launch geometry ast_fit_begin chose: threads per CTA (of a launch of integrator and photometer
+ * warps, the integrators', which run the chains), CTAs, register budget (CTAs of 256 threads per SM
+ * the kernel was compiled for) and dynamic shared memory bytes.  Any pointer may be NULL.  No reference counterpart (the reference's geometry is the compile-time
  * N_BLOCKS x BSIZE, asteroid.h:38-48). */
 int ast_fit_launch(ast_ctx* ctx, int32_t* tpb, int32_t* ctas, int32_t* min_ctas_per_sm, int32_t* smem_bytes);
 
@@ -463,7 +463,9 @@ int ast_batch_step(ast_batch* batch, int64_t evals_per_slot, int32_t* done, doub
 int ast_batch_result(ast_batch* batch, int32_t index, ast_fit_out* out);
 int ast_batch_counters(ast_batch* batch, int64_t* n_evals, int64_t* n_fits, int32_t* tpb, int32_t* refill,
                        int32_t* ctas);
-/* The launch geometry the batch runs with (tpb, refill, ctas, tile); evals_per_s is 0. */
+/* The launch geometry the batch runs with (tpb, refill, ctas, tile); evals_per_s is 0.  A batch whose
+ * geometry is neither set nor tuned and whose chains are few runs integrator and photometer warps;
+ * tpb is then the threads that run chains. */
 int ast_batch_geometry(ast_batch* batch, ast_batch_launch* out);
 /* Set the geometry (tpb, refill, tile of *geometry) for the following ast_batch_step calls,
  * instead of the tuned or default one. */
