@@ -37,7 +37,7 @@ __device__ __forceinline__ double group_rhs_torque(int role, double f, double mu
     const double y = role == 0 ? y2 : role == 1 ? y0 : role == 2 ? y1 : role == 3 ? s5 : c5;
     const double z = role < 3 ? mu_b : role == 3 ? t : -t;
     const double r = x * y + z;
-    const double f3 = shfl8(r, 3) / s4;
+    const double f3 = TRIG::div(shfl8(r, 3), s4);
     const double f5 = y2 - f3 * c4;
     return role == 3 ? f3 : role >= 5 ? f5 : r;
 }

@@ -318,7 +318,7 @@ __device__ __forceinline__ void ode_torque(const double* y, double* f, const dou
     f[0] = mu[0] * y[1] * y[2] + mu[3];
     f[1] = mu[1] * y[2] * y[0] + mu[4];
     f[2] = mu[2] * y[0] * y[1] + mu[5];
-    f[3] = (y[0] * s5 + y[1] * c5) / s4;
+    f[3] = TRIG::div(y[0] * s5 + y[1] * c5, s4);
     f[4] = y[0] * c5 - y[1] * s5;
     f[5] = y[2] - f[3] * c4;
 }
@@ -469,15 +469,15 @@ AST_HD double ls_algebraic(double b, double c, double ib2, double ic2, double Sb
     const double S = sqrt(Sb * Tb + Sc * Tc + Sa * Sa);
     const double E = sqrt(Eb * Eb * ib2 + Ec * Ec * ic2 + Ea * Ea);
     const double SE = S * E;
-    const double ca = (Eb * Tb + Ec * Tc + Sa * Ea) / SE;
+    const double ca = quot(Eb * Tb + Ec * Tc + Sa * Ea, SE);
     const double sa = sqrt(1.0 - ca * ca);
-    const double inv = 1.0 / sqrt(S * S + E * E + 2 * SE * ca);
+    const double inv = inv_sqrt(S * S + E * E + 2 * SE * ca);
     const double cl = (S + E * ca) * inv, sl = E * sa * inv;
     const double cn = (E + S * ca) * inv, sn = S * sa * inv;
     const bool pl = !signbit(cl), pn = !signbit(cn);  // (the integer pipe's; a comparison is the FP64 unit's)
     const double lp = pl ? 1.0 + cl : sl, lq = pl ? sl : 1.0 - cl;
     const double np = pn ? 1.0 + cn : sn, nq = pn ? sn : 1.0 - cn;
-    return -2.5 * log10(b * c * SE * inv * (cn + cl - sl * sn * log(lp * np / (lq * nq))));
+    return -2.5 * log10(b * c * SE * inv * (cn + cl - sl * sn * log(quot(lp * np, lq * nq))));
 }
 
 // Model magnitude at observation i for the Euler angles (phi, theta, psi): the body axes

@@ -58,6 +58,25 @@ def test_beyond(sincos):
         np.testing.assert_allclose(r, np.stack([np.sin(x), np.cos(x)], 1), rtol=0, atol=2.3e-16)
 
 
+# The seeds' whole range of significands, both signs, over many binades (within a float's on the host).
+def test_quotients(lib):
+    rng = np.random.default_rng(7)
+    n = 4000
+    s = rng.choice([-1.0, 1.0], n) * rng.uniform(1, 2, n) * 2.0 ** rng.integers(-100, 100, n)
+    s[:4] = 1.0, np.nextafter(2.0, 0), np.nextafter(1.0, 2), -2.0
+    u = rng.normal(size=n) * 2.0 ** rng.integers(-100, 100, n)
+    u[:2] = 0.0, -1.0
+    out = np.empty((n, 2))
+    lib.h_quotients(n, u.ctypes.data_as(C.c_void_p), s.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.c_void_p))
+    with mpmath.workprec(200):
+        for ui, si, (q, r) in zip(u, s, out):
+            want = mpmath.mpf(float(ui)) / mpmath.mpf(float(si))
+            assert abs(mpmath.mpf(float(q)) - want) <= 0.501 * np.spacing(abs(float(want)))
+            want = 1 / mpmath.sqrt(abs(mpmath.mpf(float(si))))
+            # e's own error, one rounding of x y (2^-53), enters by half; the last sum's rounding.
+            assert abs(mpmath.mpf(float(r)) - want) <= 0.5 * np.spacing(float(want)) + 0.51 * 2.0 ** -53 * want
+
+
 # Round and flat bodies, the angle between the scaled vectors on both sides of a right angle (each branch of the
 # half-angle quotients).
 @pytest.mark.parametrize("b,c", [(1.0, 1.0), (0.7, 0.4), (0.9, 0.02), (0.1, 0.05)])
