@@ -6,8 +6,8 @@
 // its warp to itself takes the number of its FP64 instructions times 64 cycles, and spreading its
 // components over idle lanes divides that number: eight lanes hold the six components of the state,
 // one stage's two sines and two cosines are one call, its products two instructions, its update one; the
-// magnitudes of G observations, one on each lane of the group, are one evaluation.  111 instructions
-// an RK4 step and 290 / G + 2 an observation, against 268 and 290 on one lane (torque, evaluations; 159
+// magnitudes of G observations, one on each lane of the group, are one evaluation.  95 instructions
+// an RK4 step and 267 / G + 2 an observation, against 252 and 267 on one lane (torque, evaluations; 159
 // and 467 against 340 and 467 in the simplex search, trig64.cuh).
 //
 // Every operation is the thread path's (chi2_fp64) on the same operands, sums in observation order,

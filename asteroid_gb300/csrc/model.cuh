@@ -5,7 +5,7 @@
 // expressions below keep the operand order and the float/double types of the reference's
 // chi2one (cuda.c:81-1011), x2params (cuda.c:1120-1319) and params2x (cuda.c:1016-1115);
 // nvcc then makes the same multiply-add contractions in both.  The evaluation kernels' sine and
-// cosine (trig64.cuh) and Lommel-Seeliger magnitude (ls_algebraic) are their own: they move a
+// cosine and quotients (trig64.cuh) and Lommel-Seeliger magnitude (ls_algebraic) are their own: they move a
 // chi^2 by no more than another choice of contractions does.  What differs is the data
 // flow: quantities that do not depend on the parameters (per-interval RK4 step count and
 // size, the ephemeris interpolation of E and S) are computed once per object by
@@ -458,8 +458,8 @@ __device__ __forceinline__ void write_geo(double* g, double b, double c, double 
 // between the first and their sum; nu = alpha' - lambda' is then the one between their sum and the second, and
 // each has its sine and cosine from the same triangle:
 //     cos lambda' = (S + E cos alpha') / |S + E|,  sin lambda' = E sin alpha' / |S + E|,  nu with S and E exchanged,
-// and cot(x/2) = (1 + cos x) / sin x, or sin x / (1 - cos x) where cos x < 0.  290 FP64 instructions an
-// observation against 440: 20 011 evaluations of 480 points 22.6 -> 17.7 ms, a curve of 20 000 points 132 ->
+// and cot(x/2) = (1 + cos x) / sin x, or sin x / (1 - cos x) where cos x < 0.  267 FP64 instructions an
+// observation (290 before quot and inv_sqrt) against 440: 20 011 evaluations of 480 points 22.6 -> 17.7 ms, a curve of 20 000 points 132 ->
 // 127.  The error is no larger: 1.2e-16 rms of log10 either way for alpha' of 0.1 to 2, against
 // multiprecision, and 70 times smaller close to pi.
 AST_HD double ls_algebraic(double b, double c, double ib2, double ic2, double Sb, double Sc, double Sa, double Eb, double Ec,

@@ -5,14 +5,14 @@
 // in each stage: sincos() issues 25.  With a point of a table of 1024 angles next to x, at
 // most pi/1024 away, three terms of each series are enough and x's sine and cosine take 16; memory,
 // integer and predicate instructions run beside them.  159 -> 111 instructions an RK4 step on lanes of
-// a group, 340 -> 268 on one lane (torque); 20 011 evaluations of 480 points 27.1 -> 22.6 ms (sine and
-// cosine on one lane); one of 300 points 4.48 -> 3.98 and 3.60 with each on a lane of its own, 337 of 611
-// (black-and-white ball) 8.9 -> 6.9 and 5.9, with the curve of 20 000 points 153 -> 132 and 117 (ls_algebraic in between).
+// a group, 340 -> 268 on one lane (torque); 20 011 evaluations of 480 points 27.1 -> 22.6 ms, one of 300
+// points 4.48 -> 3.98, 337 of 611 (black-and-white ball) 8.9 -> 6.9, a curve of 20 000 points 153 -> 132; with
+// each function on a lane of its own 3.86 -> 3.60, 6.9 -> 5.9 and 127 -> 117.
 //
 // The table holds the points' sine and cosine as unevaluated sums of two doubles: the results are
 // within 0.6 ulp of 1 for one rounding of each sum, 1.2 ulp of themselves near the zeros
-// (tests/test_trig64.py).  1024 points: with 512 each
-// series needs one term more, with 4096 none less, and 32 KB stay in the L1.
+// (tests/test_trig64.py).  1024 points: with 512 each series needs one term more, with 4096 none less, and
+// 32 KB stay in the L1.
 #pragma once
 #include <stdint.h>
 #include <string.h>
@@ -184,7 +184,8 @@ AST_HD double rsqrt_seed(double x)
 
 // u / s in six instructions, against ten of the division: one cubic step of the reciprocal
 // (Householder's method of order 2: y + y (e + e^2), e = 1 - s y, leaves e^3 < 2^-66) and the quotient's
-// remainder, whose correction leaves 0.5 ulp and a 2^-52th of one.  No zero, infinite or denormal s, where the
+// remainder, whose correction leaves 0.5 ulp and a 2^-52th of one.  One evaluation of 300 points 3.60 -> 3.36 ms,
+// the curve of 20 000 points 117 -> 112, 20 011 evaluations of 480 points 17.7 -> 17.3.  No zero, infinite or denormal s, where the
 // quotient is infinite and this NaN: an evaluation's chi^2 is NaN either way.
 AST_HD double quot(double u, double s)
 {
