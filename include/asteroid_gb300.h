@@ -193,7 +193,8 @@ int ast_format_result(char* buf, int64_t cap, double chi2, const double* dv, int
 
 typedef struct ast_ctx ast_ctx;
 
-#define AST_PREC_FP64   0   /* plain path: the reference's double arithmetic */
+#define AST_PREC_FP64   0   /* plain path: double arithmetic throughout (simplex search: the reference's
+                               expressions; evaluations: the same model to the same accuracy) */
 #define AST_PREC_MIXED  1   /* double-FP32 state and right-hand side, FP32 brightness */
 #define AST_PREC_MIXED_RHS32 2 /* AST_PREC_MIXED with the ODE right-hand side in FP32 (the state
                                   still double-FP32): faster, but outside 1e-6 relative chi^2 on
