@@ -58,10 +58,12 @@ AST_HD void prep_obs_point(const DevModel& M, char* base, const ObsLayout& L, in
         ef[k * n + i] = (float)ex[k * n + i];
         sf[k * n + i] = (float)sx[k * n + i];
     }
-    // h, h/6; and of the step counted in compact angles' table points, q = h T/2pi: q, 1/(6q).
+    // h, h/6; and of the step counted in compact angles' table points, q = h T/2pi: q, 1/(6q).  For equal
+    // times, or times so close that 1/(6q) leaves a float's range, 0: what it multiplies, the advance of
+    // the angular velocity counted in such steps (of order q^2), is 0 in floats too.
     const double q = hi / kTurnStep;
     const df H = df_from_double(hi), H6 = df_from_double(hi / 6.0);
-    const df Q = df_from_double(q), C6 = df_from_double(i == 0 ? 0.0 : 1.0 / (6.0 * q));
+    const df Q = df_from_double(q), C6 = df_from_double(fabs(q) < 1e-30 ? 0.0 : 1.0 / (6.0 * q));
     float4* hq = (float4*)(base + L.off_hq);
     float4* hw = (float4*)(base + L.off_hw);
     hq[i] = float4{H.hi, H.lo, Q.hi, Q.lo};

@@ -2,6 +2,7 @@
 // floating-point contraction, as mixed_harness.cu).
 #include <vector>
 #include "mixed.cuh"
+#include "prep.cuh"
 
 using namespace ast;
 
@@ -58,6 +59,35 @@ void h_turn_steps(int torque, int n, double h, const double* mu, double* y)
     o.nst = nst;
     o.hq = hq;
     o.hw = hw;
+    df a[3];
+    mixed_advance<false>(S, o, 1, tab.data(), a);
+    for (int k = 0; k < 3; k++) {
+        if (torque) y[k] = df_to_double(S.s.w[k]) + (double)S.s.r[k];
+        y[3 + k] = df_to_double(a[k]);
+    }
+}
+
+// From y at time 0 to time t, with the step constants of prep_obs_point.
+void h_turn_interval(int torque, double t, double time_step, const double* mu, double* y)
+{
+    const std::vector<float4> tab = table();
+    const ObsLayout L = ObsLayout::make(2);
+    std::vector<char> block((size_t)L.bytes + 256);
+    char* base = block.data() + (256 - (uintptr_t)block.data() % 256);
+    DevModel M{};
+    M.time_step = time_step;
+    M.n_data = 2;
+    ((double*)(base + L.off_t))[1] = t;
+    for (int i = 0; i < 2; i++) prep_obs_point(M, base, L, 2, i);
+    const ObsView o = L.view(base, 2);
+    MixedState S;
+    S.torque = torque != 0;
+    S.bw = false;
+    for (int k = 0; k < (torque ? 6 : 3); k++) {
+        S.mu[k] = df_from_double(mu[k]);
+        S.y[k] = df_from_double(torque ? y[k] : y[3 + k]);
+    }
+    mixed_begin(S);
     df a[3];
     mixed_advance<false>(S, o, 1, tab.data(), a);
     for (int k = 0; k < 3; k++) {

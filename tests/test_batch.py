@@ -210,3 +210,21 @@ def test_warp_tiled_mapping_equals_single_fits(gpu, synth_objects, tile):
         got = [b.result(i) for i in range(len(objs))]
     for k, s in enumerate(objs):
         same(got[k], single(s, api.PREC_MIXED, 90 + k))
+
+
+@pytest.mark.parametrize("chains", [32, 152 * 160])
+def test_a_repeated_time(gpu, oracle_mod, synth_objects, chains):
+    """A batch does not check its objects' times: an interval of no length leaves the state as it is, by
+    pairs and by threads."""
+    from dataclasses import replace
+
+    s = synth_objects("c0acc")
+    t = s.obs.mjd.copy()
+    t[10], t[200] = t[9], t[199]
+    obs = replace(s.obs, mjd=t)
+    with api.Batch(precision=api.PREC_MIXED, acc=True) as b:
+        b.add(s.model, obs, n_chains=chains, group_size=chains, seed=5, evals_cap=20, reopt=True, params0=s.params_true)
+        b.run()
+        r = b.result(0)
+    ref, _ = oracle_mod.chi2_batch(s.model, obs, r.best_params)
+    assert np.allclose(r.best_f, ref, rtol=1e-6, atol=0), (r.best_f, ref)

@@ -112,3 +112,20 @@ def test_a_thousand_steps_keep_the_phase(lib, torque):
     d = (got[3:] - ref[3:] + math.pi) % (2 * math.pi) - math.pi
     # 300 rad at u^2 systematically (the constants' own rounding), ten times that for the random part.
     assert np.max(np.abs(d)) <= 10 * 300 * 2.0 ** -48
+
+
+# From the same time twice to the shortest and an ordinary interval: where the step's size in table points, or its
+# inverse, leaves a float's range the state stays as it is.
+@pytest.mark.parametrize("torque", [1, 0])
+@pytest.mark.parametrize("t", [0.0, 5e-324, 1e-45, 1e-40, 1e-30, 1e-18, 1e-12, 1e-3])
+def test_intervals_down_to_nothing(lib, torque, t):
+    lib.h_turn_interval.argtypes = [C.c_int, C.c_double, C.c_double, C.c_void_p, C.c_void_p]
+    y = np.array([9.0, -14.0, 25.0, 0.25, 1.25, -0.75])
+    mu = np.array([0.31, -0.22, -0.09, 0.01, -0.02, 0.015]) if torque else np.array([28.0, 0.75, 0.11])
+    got = y.copy()
+    lib.h_turn_interval(torque, t, 1e-2, P(mu), P(got))
+    ref = _rk4(torque, t, mu, y)
+    tol = 2.0 ** -48 * (40 * 11.5 * (1 + 30 * t) ** 2 + 16 * math.pi)  # as a step's above
+    assert np.max(np.abs((got[3:] - ref[3:] + math.pi) % (2 * math.pi) - math.pi)) <= tol
+    if torque:
+        assert np.max(np.abs(got[:3] - ref[:3])) <= (tol * 31 if t > 1e-17 else 0.0)

@@ -101,6 +101,22 @@ def test_noalloc_fit_matches_fit_on_two_calls(gpu, synth_objects, case):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("precision", [api.PREC_FP64, api.PREC_MIXED])
+def test_noalloc_takes_a_repeated_time(gpu, oracle_mod, synth_objects, precision):
+    """The device arrays' times are not checked: an interval of no length leaves the state as it is."""
+    from dataclasses import replace
+    from types import SimpleNamespace
+
+    c = synth_objects("c0acc")
+    t = c.obs.mjd.copy()
+    t[10], t[200] = t[9], t[199]
+    s = SimpleNamespace(model=c.model, obs=replace(c.obs, mjd=t), params_true=c.params_true)
+    f, p, _ = _noalloc(s, 64, 32, 1, 41, 40, precision, True)
+    ref, _ = oracle_mod.chi2_batch(s.model, s.obs, p)
+    assert np.allclose(f, ref, rtol=1e-9 if precision == api.PREC_FP64 else 1e-6, atol=0), (f, ref)
+
+
+@pytest.mark.gpu
 def test_noalloc_first_call_in_a_fresh_process(gpu):
     """480 points (block staged in shared memory, 65 KB), 2000 points with INTERP + NUDGE (read
     through L1) and 4096 points (the array's maximum): ast_fit_noalloc is the process's first fit."""
