@@ -1020,7 +1020,7 @@ static int coop_geometry(ast_pool& P, int tpb)
 {
     const size_t smem = (size_t)(tpb / kCoopLanes) * sizeof(CoopXchg<CF>);
     auto kern = coop_kernel<CF, PREC>;
-    AST_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_smem(kern, smem)) return rc;  // one CTA size for every server
     int occ = 0;
     AST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, tpb, smem));
     if (occ < 1) return ast_set_error(AST_E_TOO_LARGE, "server: cooperative kernel does not fit on an SM");
@@ -1060,9 +1060,9 @@ static int pool_geometry(ast_pool& P, int tpb, int refill, int tile = 0)
         refill = 32;
         smem = (size_t)(tpb / 32) * tile_warp_bytes(tile);
         auto kern = batch_tile_ptr(tile);
-        // Always raised to the request: without it, dynamic and static shared memory together stay
-        // within 48 KB (the sin/cos tables take 45 KB of that).
-        AST_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        // Always raised, to the largest CTA's need: without it, dynamic and static shared memory together
+        // stay within 48 KB (the sin/cos tables take 45 KB of that).
+        if (int rc = allow_smem(kern, (size_t)(KernShape<AST_PREC_MIXED>::tpb / 32) * tile_warp_bytes(tile))) return rc;
         AST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, tpb, smem));
     } else {
         AST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel_ptr<CF, PREC>(refill), tpb, 0));
@@ -1096,8 +1096,7 @@ static int batch_geometry_default(ast_pool& P)
     P.tile = 0;
     P.smem = sizeof(PairChain) * k;
     P.ctas = (int)ctas;
-    AST_CUDA(cudaFuncSetAttribute(batch_pair_kernel<CF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
-    return AST_OK;
+    return allow_smem(batch_pair_kernel<CF>, sizeof(PairChain) * kPairIntegrators);
 }
 
 // One launch of the pool's kernel (thread per chain or warp per object, the warp-tiled evaluation, or

@@ -386,7 +386,7 @@ static int launch_eval_pair(ast_ctx* c, const DevModel& dm, int integrators, con
 {
     auto kern = eval_pair_kernel<CF, PREC>;
     const size_t smem = sizeof(PairTile) * integrators;
-    AST_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_smem(kern, sizeof(PairTile) * kPairIntegrators)) return rc;
     const int64_t per_cta = 32 * integrators;
     kern<<<(unsigned)((n + per_cta - 1) / per_cta), 32 * pair_warps(integrators), smem, s>>>(
         dm, c->d_obs, c->layout, integrators, d_params, n, d_chi2, d_dv);

@@ -87,11 +87,22 @@ struct ast_ctx {
 };
 
 namespace ast {
+// Lets launches of `kern` ask for up to `bytes` of dynamic shared memory (needed above 48 KB; allocates
+// nothing).  The limit belongs to the kernel on its device, not to a context or a call: one caller's
+// value holds for the launches of every other context and thread.  So `bytes` is the most that any call
+// asks of the kernel, the same from every caller, never what this call needs.
+template <class K>
+inline int allow_smem(K kern, size_t bytes)
+{
+    AST_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return AST_OK;
+}
+
 // Dynamic shared memory for staging an observation block of `bytes` in one CTA of `kern`: the
 // block's size when it fits beside the kernel's static shared memory (the double-float trig
 // table, the staging barrier) under the per-CTA opt-in limit `optin`, else 0 -- the kernel then
-// reads the block from global memory through L1.  When it is staged, the kernel's dynamic
-// shared-memory limit is raised to the block's size (needed above 48 KB; allocates nothing).
+// reads the block from global memory through L1.  When it is staged, the kernel may ask for all
+// that the device has beside its static shared memory.
 template <class K>
 inline int obs_smem_for(K kern, size_t bytes, size_t optin, size_t* smem)
 {
@@ -100,7 +111,7 @@ inline int obs_smem_for(K kern, size_t bytes, size_t optin, size_t* smem)
     cudaFuncAttributes a;
     AST_CUDA(cudaFuncGetAttributes(&a, kern));
     if (bytes + a.sharedSizeBytes > optin) return AST_OK;
-    AST_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    if (int rc = allow_smem(kern, optin - a.sharedSizeBytes)) return rc;
     *smem = bytes;
     return AST_OK;
 }

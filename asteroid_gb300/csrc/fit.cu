@@ -438,9 +438,8 @@ static int fit_launch_core(int sm_count, size_t obs_bytes, size_t optin, int tpb
             r->ctas = (int)((n_chains + per_cta - 1) / per_cta);
             r->smem = sizeof(PairChain) * r->pair;
             r->minb = 1;
-            auto kern = fit_pair_kernel<CF, PREC == AST_PREC_FP64 ? AST_PREC_MIXED : PREC>;
-            AST_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r->smem));
-            return AST_OK;
+            return allow_smem(fit_pair_kernel<CF, PREC == AST_PREC_FP64 ? AST_PREC_MIXED : PREC>,
+                              sizeof(PairChain) * kPairIntegrators);
         }
     }
     // Register budget: 1 (255 registers, CTAs of up to 256), 2 (128), 3 (170, CTAs of up to 128).
