@@ -776,7 +776,7 @@ struct ast_pool {
 struct ast_batch {
     ast_pool P;
     cudaGraphExec_t graph = nullptr;
-    int g_tpb = 0, g_refill = 0, g_ctas = 0, g_tile = 0;
+    int g_tpb = 0, g_refill = 0, g_ctas = 0, g_tile = 0, g_pair = 0;  // the graph's geometry
     bool ordered = false;
     bool ran = false;
 };
@@ -1183,7 +1183,8 @@ template <class CF, int PREC>
 static int batch_capture(ast_batch* B)
 {
     ast_pool& P = B->P;
-    if (B->graph && B->g_tpb == P.tpb && B->g_refill == P.refill && B->g_ctas == P.ctas && B->g_tile == P.tile)
+    if (B->graph && B->g_tpb == P.tpb && B->g_refill == P.refill && B->g_ctas == P.ctas && B->g_tile == P.tile &&
+        B->g_pair == P.pair)
         return AST_OK;
     if (B->graph) { cudaGraphExecDestroy(B->graph); B->graph = nullptr; }
     std::vector<std::pair<int, Entry*>> all;
@@ -1209,6 +1210,7 @@ static int batch_capture(ast_batch* B)
     B->g_refill = P.refill;
     B->g_ctas = P.ctas;
     B->g_tile = P.tile;
+    B->g_pair = P.pair;
     return AST_OK;
 }
 

@@ -79,3 +79,30 @@ def test_batches_by_pairs_equal_threads(gpu, acc):
         for r, g in zip(ref, got):
             for k in ("best_f", "best_params", "best_dv"):
                 assert np.array_equal(getattr(r, k), getattr(g, k), equal_nan=True)
+
+
+def test_a_requested_geometry_is_not_run_by_the_paired_graph(gpu):
+    """Three warps a CTA, refill 32, two CTAs: a paired launch of one integrator a CTA and a launch of one thread
+    a chain alike.  The batch's graph is recorded again for the second, whose time tells which kernel ran."""
+    model, obs, P = _object("TORQUE,ACC", 300, 2, 3, 0.05)
+
+    def batch():
+        b = api.Batch(precision=api.PREC_MIXED, acc=True, n_slots=192)
+        b.add(model, obs, n_chains=64, group_size=32, seed=4, evals_cap=60, reopt=True, params0=P[0])
+        return b
+
+    def ms(b, **geometry):
+        t = min(b.run(**geometry) for _ in range(3))
+        return t, b.result(0)
+
+    with batch() as b:
+        threads, ref = ms(b, tpb=96, refill=32)
+    with batch() as b:
+        pairs, r = ms(b)
+        after, g = ms(b, tpb=96, refill=32)
+        assert b.counters()["tpb"] == 96 and b.counters()["ctas"] == 2
+    assert pairs < 0.85 * threads  # the two kernels' times are told apart
+    assert after > 0.92 * threads, (pairs, threads, after)
+    for k in ("best_f", "best_params", "best_dv"):
+        assert np.array_equal(getattr(r, k), getattr(ref, k), equal_nan=True)
+        assert np.array_equal(getattr(g, k), getattr(ref, k), equal_nan=True)
