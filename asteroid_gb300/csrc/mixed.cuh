@@ -297,13 +297,13 @@ AST_HD df ls_magnitude_df(const df* Sp, const df* Ep, df ib, df ic, df bc, const
     df cr[3];
     df_cross3(sv, ev, cr);
     const df cn = df_sqrt(df_dot3(cr, cr));
-    const df mu = df_atan2(cn, df_dot3(sv, hv), tab);
-    const df nu = df_atan2(cn, df_dot3(hv, ev), tab);
-    const df eps = df_atan2(cn, df_neg(df_dot3(sv, ev)), tab);
-    df sd, D, s, cd;
-    const df hmn = df_sub(mu, nu);
-    df_sincos(df{0.5f * hmn.hi, 0.5f * hmn.lo}, tab, &sd, &D);
-    df_sincos(df{0.5f * eps.hi, 0.5f * eps.lo}, tab, &s, &cd);
+    df x[3] = {df_dot3(sv, hv), df_dot3(hv, ev), df_neg(df_dot3(sv, ev))};  // to mu, nu, eps
+#pragma unroll 1
+    for (int k = 0; k < 3; k++) x[k] = df_atan2(cn, x[k], tab);
+    df h[2] = {df_sub(x[0], x[1]), x[2]}, sn[2], cs[2];
+#pragma unroll 1
+    for (int k = 0; k < 2; k++) df_sincos(df{0.5f * h[k].hi, 0.5f * h[k].lo}, tab, &sn[k], &cs[k]);
+    const df D = cs[0], s = sn[1];
     const df B = df_mul(df_mul(df{2.0f * D.hi, 2.0f * D.lo}, D), ls_f_df(df_div(s, D)));
     const df arg = df_mul(df_div(df_mul(df_mul(bc, sS), sE), scalar), B);
     const df INV_LN10{0.4342945f, -1.010305e-08f};
@@ -357,10 +357,10 @@ AST_HD DfFrame make_df_frame(const DevModel& M, const double* params)
 // the body frame as in cuda.c:432-473, then ls_magnitude_df or the BW_BALL law (cuda.c:568-580).
 AST_HD double vmod_df(const DevModel& M, const ObsView& o, const DfFrame& F, const df* ang, int i, const float4* tab)
 {
-    df sph, cph, sth, cth, sps, cps;
-    df_sincos(ang[0], tab, &sph, &cph);
-    df_sincos(ang[1], tab, &sth, &cth);
-    df_sincos(ang[2], tab, &sps, &cps);
+    df sn[3], cs[3];
+#pragma unroll 1
+    for (int k = 0; k < 3; k++) df_sincos(ang[k], tab, &sn[k], &cs[k]);
+    const df sph = sn[0], cph = cs[0], sth = sn[1], cth = cs[1], sps = sn[2], cps = cs[2];
     const df N[3] = {df_add(df_mul(F.XM_x, cph), df_mul(F.YM[0], sph)), df_mul(F.YM[1], sph),
                      df_add(df_mul(F.XM_z, cph), df_mul(F.YM[2], sph))};
     df p[3];
@@ -404,16 +404,20 @@ struct NudgeCand {
 // The reference's test and parabola (cuda.c:716-760) on each queued triple, with double-float
 // magnitudes.  Returns false as soon as more than AST_M_MAX minima are found (the model is then
 // rejected exactly as the reference rejects it, only after a few more observations).
-// Not inlined: the magnitude code is cold and large, and one copy serves both call sites.
+// Not inlined: the magnitude code is cold and large, and one copy serves both call sites.  One copy of the
+// magnitude, too, and of its sines and arctangents: 80 KB instead of 278, which with the step did not fit the
+// instruction cache (torqued NUDGE fits from the prior, 19 456 chains of 60 points: 45 ms against 92).
 static __host__ __device__ __noinline__ bool nudge_flush(const DevModel& M, const ObsView& o, const DfFrame& F,
                                                          const float4* tab, NudgeCand* cand, int* n_cand, int* Mmin,
                                                          float* t_mod, float* V_mod)
 {
     for (int q = 0; q < *n_cand; q++) {
         const int ic = cand[q].i;
-        const float f0 = (float)vmod_df(M, o, F, cand[q].a[0], ic - 2, tab);
-        const float f1 = (float)vmod_df(M, o, F, cand[q].a[1], ic - 1, tab);
-        const double v2 = vmod_df(M, o, F, cand[q].a[2], ic, tab);
+        double v[3];
+#pragma unroll 1
+        for (int j = 0; j < 3; j++) v[j] = vmod_df(M, o, F, cand[q].a[j], ic - 2 + j, tab);
+        const float f0 = (float)v[0], f1 = (float)v[1];
+        const double v2 = v[2];
         if (f1 > f0 && f1 >= v2) {
             if (++*Mmin > AST_M_MAX) return false;
             const float t0 = (float)o.t[ic - 2], t1 = (float)o.t[ic - 1];
@@ -553,7 +557,8 @@ AST_HD void spin_angles(const Spin& s, bool torque, df* ang)
 
 // The step for a state that turn_step_* declines, an angle that advances by more than 1000 turns in
 // one step: rk4_step_df2 on the angles themselves (a rotation the fixed step does not resolve; any
-// finite or non-finite outcome, as long as it is the model's).  Cold: one copy, not inlined.
+// finite or non-finite outcome, as long as it is the model's).  Cold: one copy, not inlined, loops rolled
+// (the instruction cache holds it beside the step and the magnitude).
 static __host__ __device__ __noinline__ void spin_step_general(Spin* s, bool torque, const df* mu, float4 hq, float4 hw,
                                                                const float4* tab)
 {
@@ -562,6 +567,7 @@ static __host__ __device__ __noinline__ void spin_step_general(Spin* s, bool tor
     const float4 gq = make_float4(hq.x, hq.y, 0.5f * hq.x, 0.5f * hq.y);
     const float4 gw = make_float4(hw.x, hw.y, 2.0f * hw.x, 2.0f * hw.y);
     df m[6];
+#pragma unroll 1
     for (int k = 0; k < (torque ? 6 : 3); k++)
         m[k] = torque && k < 3 ? df_from_double(df_to_double(mu[k]) / kTurnStep) : mu[k];
     if (torque) {
@@ -581,9 +587,11 @@ static __host__ __device__ __noinline__ void spin_step_general(Spin* s, bool tor
         ang[1] = df2_y(Y[0]);
         ang[0] = df2_x(Y[1]);
     }
-    const Turn th = turn_from(ang[1]), ps = turn_from(ang[2], torque ? 1 : 2);
-    s->phi = turn_from(ang[0]);
-    s->a = Turn2{ps.k, th.k, make_float2(ps.e, th.e), make_float2(ps.t, th.t)};
+    Turn t[3];
+#pragma unroll 1
+    for (int k = 0; k < 3; k++) t[k] = turn_from(ang[k], k == 2 && !torque ? 2 : 1);
+    s->phi = t[0];
+    s->a = Turn2{t[2].k, t[1].k, make_float2(t[2].e, t[1].e), make_float2(t[2].t, t[1].t)};
 }
 
 // Called on copies, so that the state itself stays in registers.

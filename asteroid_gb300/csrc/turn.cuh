@@ -111,7 +111,8 @@ AST_HD df turn_value(uint32_t k, float e, float t, int turns)
 // An angle in radians as a compact one (turns = 1), or twice it (turns = 2, its k/4 modulo 2 T).
 AST_HD Turn turn_from(df a, int turns = 1)
 {
-    const df r = df_mul(df_reduce_2pi(a), df_from_double(turns / kTurnStep));
+    const df one = df_from_double(1.0 / kTurnStep), two = df_from_double(2.0 / kTurnStep);
+    const df r = df_mul(df_reduce_2pi(a), turns == 1 ? one : two);
     return turn_reduce(r, 0);
 }
 
