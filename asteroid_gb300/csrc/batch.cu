@@ -1087,7 +1087,7 @@ static int pool_tpb(const ast_pool& P) { return P.pair ? 32 * P.pair : P.tpb; }
 template <class CF, int PREC>
 static int batch_geometry_default(ast_pool& P)
 {
-    const int k = PREC == AST_PREC_MIXED ? pair_integrators(P.chain_end, P.sm_count) : 0;
+    const int k = PREC == AST_PREC_MIXED ? pair_integrators(P.chain_end, P.sm_count, kPairIntegrators) : 0;
     const int64_t ctas = k ? (P.chain_end + 32 * k - 1) / (32 * k) : 0;
     if (!k || P.chain_end <= 0 || ctas * 32 * k > P.n_slots) return pool_geometry<CF, PREC>(P, 256, 1);
     P.pair = k;

@@ -316,6 +316,7 @@ extern "C" int ast_prepare(const ast_model* model, const ast_obs_set* obs, int32
     if ((rc = build_dev_model(model, obs, &c->dm))) { ast_destroy(c); return rc; }
     c->n_data = obs->n_data;
     c->n_filters = obs->n_filters;
+    c->span = obs->mjd[obs->n_data - 1] - obs->mjd[0];
     const int64_t n = obs->n_data;
     c->layout = ObsLayout::make(n);
     std::vector<unsigned char> img;
@@ -411,7 +412,7 @@ static int launch_eval(ast_ctx* c, const DevModel& dm, const double* d_params, i
         return AST_OK;
     }
     if (PREC != AST_PREC_FP64)
-        if (const int k = pair_integrators(n, c->sm_count))
+        if (const int k = pair_integrators(n, c->sm_count, pair_most_eval(dm.flags)))
             return launch_eval_pair<CF, PREC == AST_PREC_FP64 ? AST_PREC_MIXED : PREC>(c, dm, k, d_params, n, d_chi2, d_dv, s);
     // As the fits (fit_launch_core): the precision's own shape when the vectors fill it, the full
     // register file when they do not (1001 vectors of 480 points, mixed: 1.19 ms against 1.33).

@@ -73,6 +73,7 @@ struct ast_ctx {
     ast_model model{};
     ast::DevModel dm{};
     int32_t n_data = 0, n_filters = 0;
+    double span = 0;  // days from the first observation to the last
     ast::ObsLayout layout{};
     void* d_obs = nullptr;
     // evaluation scratch
@@ -128,13 +129,41 @@ inline int group_lanes(int64_t n, int sm_count)
 }
 
 // Integrator warps of a CTA of the paired mixed kernels (mixed.cuh), by the number of evaluations that run
-// side by side; 0: one thread an evaluation, both parts.  Pairs win while an SM holds at most four
-// integrators, one on each of its quarters.
+// side by side; 0: one thread an evaluation, both parts.  At most `most` (pair_most_eval, pair_most_fit).
 constexpr int kPairIntegrators = 4;
-inline int pair_integrators(int64_t n, int sm_count)
+inline int pair_integrators(int64_t n, int sm_count, int most)
 {
     const int64_t k = ((n + 31) / 32 + sm_count - 1) / sm_count;
-    return k <= kPairIntegrators ? (int)k : 0;
+    return k <= most ? (int)k : 0;
+}
+
+// The most integrators a CTA with which pairs are faster than threads.  Beside its step an integrator has
+// the general step's code (models that the step declines) and a photometer the NUDGE candidates'; an SM whose
+// warps run all of them at once waits for instructions, the more warps the more.  Pairs against threads,
+// ms, with 2, 3 and 4 integrators a CTA on 152 SMs; steps: the curve's span in RK4 steps an observation.
+//   evaluations, 150 points, steps 2.1: near a model       0.37/0.53    0.39/0.53    0.42/0.53
+//                                       from the prior     0.57/0.69    0.77/0.70    0.94/0.71
+//                torque, NUDGE: near a model               0.73/0.93    0.86/0.93    0.85/0.94
+//                               from the prior             1.18/1.11    1.58/1.14    1.87/1.20
+//   fits, 60 points, steps 2.1: free, 16 evaluations a chain  3.4/4.8    4.0/4.9      4.4/4.8
+//     100 evaluations:
+//                torque, from a model                      21.7/30.0    25.9/30.6    38.6/29.3
+//                        from the prior                    45.1/46.0    66.7/52.4    88.3/58.6
+//                                        steps 9.1         75.3/88.0    84.7/88.4    98.4/89.0
+//                torque, NUDGE, from the prior              143/138      206/183      274/205
+//                FP32 right-hand side, from a model        21.9/27.2    24.7/29.0    31.7/28.2
+// Evaluations are taken for those of models near a solution.  A batch's objects share a launch and its thread kernel keeps three CTAs of 128
+// an SM: pairs up to four (six objects of three variants, 30 evaluations a chain: 26/67, 29/68, 36/67).
+inline int pair_most_eval(int flags)
+{
+    return (flags & AST_TORQUE) && (flags & AST_NUDGE) ? 2 : kPairIntegrators;
+}
+inline int pair_most_fit(int precision, int flags, bool from_model, double steps)
+{
+    if (flags & AST_NUDGE) return 2;
+    if (precision == AST_PREC_MIXED_RHS32) return 3;
+    if (!(flags & AST_TORQUE)) return kPairIntegrators;
+    return from_model || steps >= 6 ? 3 : 2;
 }
 
 int build_dev_model(const ast_model* m, const ast_obs_set* obs, DevModel* dm);

@@ -414,7 +414,7 @@ static int64_t fit_slots(const FitRun& r)
 // `obs_bytes` is the observation block's size, `optin` the device's per-CTA shared-memory limit.
 template <class CF, int PREC>
 static int fit_launch_core(int sm_count, size_t obs_bytes, size_t optin, int tpb_req, int minb_req, int stage_req,
-                           int64_t n_chains, FitRun* r)
+                           int64_t n_chains, int pair_most, FitRun* r)
 {
     // FP64 with no geometry asked for: lane groups while they are faster (group_lanes).
     r->lanes = 1;
@@ -431,7 +431,7 @@ static int fit_launch_core(int sm_count, size_t obs_bytes, size_t optin, int tpb
     // Mixed with no geometry asked for: integrators and photometers while they are faster.
     r->pair = 0;
     if (PREC != AST_PREC_FP64 && tpb_req <= 0 && minb_req <= 0 && stage_req == 0) {
-        r->pair = pair_integrators(n_chains, sm_count);
+        r->pair = pair_integrators(n_chains, sm_count, pair_most);
         if (r->pair) {
             const int64_t per_cta = 32 * r->pair;
             r->tpb = 32 * pair_warps(r->pair);
@@ -488,10 +488,11 @@ static int fit_launch_core(int sm_count, size_t obs_bytes, size_t optin, int tpb
 }
 
 template <class CF, int PREC>
-static int fit_launch_cfg(ast_ctx* c, int tpb_req, int minb_req, int stage_req, int64_t n_chains, FitRun* r)
+static int fit_launch_cfg(ast_ctx* c, const ast_fit_cfg* cfg, FitRun* r)
 {
-    return fit_launch_core<CF, PREC>(c->sm_count, (size_t)c->layout.bytes, c->smem_optin, tpb_req, minb_req, stage_req,
-                                     n_chains, r);
+    const int most = pair_most_fit(PREC, c->dm.flags, cfg->reopt != 0, c->span / c->dm.time_step / c->n_data);
+    return fit_launch_core<CF, PREC>(c->sm_count, (size_t)c->layout.bytes, c->smem_optin, cfg->tpb, cfg->min_ctas_per_sm,
+                                     cfg->stage_obs, cfg->n_chains, most, r);
 }
 
 extern "C" int ast_fit_begin(ast_ctx* c, const ast_fit_cfg* cfg)
@@ -514,16 +515,15 @@ extern "C" int ast_fit_begin(ast_ctx* c, const ast_fit_cfg* cfg)
     r.reopt = cfg->reopt ? 1 : 0;
     const bool acc = (c->model.flags & AST_ACC) != 0;
     const int cfb = acc ? 8 : 4;
-    const int mb = cfg->min_ctas_per_sm, so = cfg->stage_obs;
     const int32_t pr = cfg->precision;
     if (acc)
-        rc = pr == AST_PREC_FP64        ? fit_launch_cfg<double, AST_PREC_FP64>(c, cfg->tpb, mb, so, cfg->n_chains, &r)
-             : pr == AST_PREC_MIXED_RHS32 ? fit_launch_cfg<double, AST_PREC_MIXED_RHS32>(c, cfg->tpb, mb, so, cfg->n_chains, &r)
-                                        : fit_launch_cfg<double, AST_PREC_MIXED>(c, cfg->tpb, mb, so, cfg->n_chains, &r);
+        rc = pr == AST_PREC_FP64        ? fit_launch_cfg<double, AST_PREC_FP64>(c, cfg, &r)
+             : pr == AST_PREC_MIXED_RHS32 ? fit_launch_cfg<double, AST_PREC_MIXED_RHS32>(c, cfg, &r)
+                                        : fit_launch_cfg<double, AST_PREC_MIXED>(c, cfg, &r);
     else
-        rc = pr == AST_PREC_FP64        ? fit_launch_cfg<float, AST_PREC_FP64>(c, cfg->tpb, mb, so, cfg->n_chains, &r)
-             : pr == AST_PREC_MIXED_RHS32 ? fit_launch_cfg<float, AST_PREC_MIXED_RHS32>(c, cfg->tpb, mb, so, cfg->n_chains, &r)
-                                        : fit_launch_cfg<float, AST_PREC_MIXED>(c, cfg->tpb, mb, so, cfg->n_chains, &r);
+        rc = pr == AST_PREC_FP64        ? fit_launch_cfg<float, AST_PREC_FP64>(c, cfg, &r)
+             : pr == AST_PREC_MIXED_RHS32 ? fit_launch_cfg<float, AST_PREC_MIXED_RHS32>(c, cfg, &r)
+                                        : fit_launch_cfg<float, AST_PREC_MIXED>(c, cfg, &r);
     if (rc) return rc;
     const int64_t slots = fit_slots(r);
     const int64_t groups = cfg->n_chains / cfg->group_size;
@@ -883,12 +883,12 @@ extern "C" int ast_fit_noalloc(const ast_model* model, const ast_obs_set* obs, c
     FitRun r;
     if (acc)
         rc = cfg->precision == AST_PREC_FP64
-                 ? fit_launch_core<double, AST_PREC_FP64>(sms, L.bytes, optin, cfg->tpb, cfg->min_ctas_per_sm, cfg->stage_obs, cfg->n_chains, &r)
-                 : fit_launch_core<double, AST_PREC_MIXED>(sms, L.bytes, optin, cfg->tpb, cfg->min_ctas_per_sm, cfg->stage_obs, cfg->n_chains, &r);
+                 ? fit_launch_core<double, AST_PREC_FP64>(sms, L.bytes, optin, cfg->tpb, cfg->min_ctas_per_sm, cfg->stage_obs, cfg->n_chains, kPairIntegrators, &r)
+                 : fit_launch_core<double, AST_PREC_MIXED>(sms, L.bytes, optin, cfg->tpb, cfg->min_ctas_per_sm, cfg->stage_obs, cfg->n_chains, kPairIntegrators, &r);
     else
         rc = cfg->precision == AST_PREC_FP64
-                 ? fit_launch_core<float, AST_PREC_FP64>(sms, L.bytes, optin, cfg->tpb, cfg->min_ctas_per_sm, cfg->stage_obs, cfg->n_chains, &r)
-                 : fit_launch_core<float, AST_PREC_MIXED>(sms, L.bytes, optin, cfg->tpb, cfg->min_ctas_per_sm, cfg->stage_obs, cfg->n_chains, &r);
+                 ? fit_launch_core<float, AST_PREC_FP64>(sms, L.bytes, optin, cfg->tpb, cfg->min_ctas_per_sm, cfg->stage_obs, cfg->n_chains, kPairIntegrators, &r)
+                 : fit_launch_core<float, AST_PREC_MIXED>(sms, L.bytes, optin, cfg->tpb, cfg->min_ctas_per_sm, cfg->stage_obs, cfg->n_chains, kPairIntegrators, &r);
     if (rc) return rc;
     const int64_t slots = fit_slots(r), S = (slots + 31) / 32 * 32;
     int64_t off[20];

@@ -106,3 +106,26 @@ def test_a_requested_geometry_is_not_run_by_the_paired_graph(gpu):
     for k in ("best_f", "best_params", "best_dv"):
         assert np.array_equal(getattr(r, k), getattr(ref, k), equal_nan=True)
         assert np.array_equal(getattr(g, k), getattr(ref, k), equal_nan=True)
+
+
+# One integrator to four, and where threads take over: with torque at the third or fourth (a start from the prior
+# or from a model, a sparse or a dense curve), with NUDGE at the third, with the FP32 right-hand side at the fourth.
+@pytest.mark.parametrize("flags,chains,span,precision,reopt,integrators", [
+    ("ACC", 4864, 1.0, api.PREC_MIXED, False, 1), ("ACC", 19456, 1.0, api.PREC_MIXED, False, 4), ("ACC", 19488, 1.0, api.PREC_MIXED, False, 0),
+    ("TORQUE,ACC", 9728, 1.0, api.PREC_MIXED, False, 2), ("TORQUE,ACC", 9760, 1.0, api.PREC_MIXED, False, 0),
+    ("TORQUE,ACC", 9760, 5.0, api.PREC_MIXED, False, 3), ("TORQUE,ACC", 14592, 1.0, api.PREC_MIXED, True, 3),
+    ("TORQUE", 14624, 5.0, api.PREC_MIXED, True, 0), ("NUDGE", 9728, 1.0, api.PREC_MIXED, True, 2), ("NUDGE", 9760, 5.0, api.PREC_MIXED, True, 0),
+    ("TORQUE,ACC", 14592, 1.0, api.PREC_MIXED_RHS32, False, 3), ("ACC", 14624, 1.0, api.PREC_MIXED_RHS32, True, 0)])
+def test_where_fits_by_pairs_end(gpu, flags, chains, span, precision, reopt, integrators):
+    if _sms() != 152:
+        pytest.skip("the chain counts are those of 152 SMs")
+    model, obs, P = _object(flags, 48, 2, 5, span)
+    kw = dict(reopt=True, params0=P[0]) if reopt else {}
+    with api.Engine(model, obs) as eng:
+        a = eng.fit(n_chains=chains, group_size=32, seed=2, evals_cap=13, precision=precision, **kw)
+        g = eng.fit_launch()
+        # A PairChain is some 27 KB; the block of 48 points is 8.
+        assert (g["tpb"] // 32 if g["smem"] > 18000 else 0) == integrators, g
+        b = eng.fit(n_chains=chains, group_size=32, seed=2, evals_cap=13, precision=precision, tpb=128, **kw)
+    for k in ("best_f", "best_params", "best_dv", "chain_f"):
+        assert np.array_equal(getattr(a, k), getattr(b, k), equal_nan=True), k

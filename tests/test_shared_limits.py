@@ -29,7 +29,7 @@ def test_fits_in_turn_equal_fits_alone(gpu, precision, large, small, kw):
     def begin(eng, chains):
         eng.fit_begin(n_chains=chains, group_size=32, seed=3, evals_cap=14, precision=precision, **kw)
 
-    objects = [_object("TORQUE,ACC", n, 2, 5, 1.0)[:2] for n, _ in (large, small)]
+    objects = [_object("ACC", n, 2, 5, 1.0)[:2] for n, _ in (large, small)]
     chains = (large[1], small[1])
     ref = []
     for (model, obs), c in zip(objects, chains):
