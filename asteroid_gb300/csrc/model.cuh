@@ -453,31 +453,59 @@ __device__ __forceinline__ void write_geo(double* g, double b, double c, double 
     g[17] = ax; g[18] = ay; g[19] = az;
 }
 
-// The Lommel-Seeliger magnitude of cuda.c:664-689 without its inverse and half-angle functions.
-// alpha' is the angle between the scaled vectors to the Sun and the Earth, lambda' the one
-// between the first and their sum; nu = alpha' - lambda' is then the one between their sum and the second, and
-// each has its sine and cosine from the same triangle:
-//     cos lambda' = (S + E cos alpha') / |S + E|,  sin lambda' = E sin alpha' / |S + E|,  nu with S and E exchanged,
-// and cot(x/2) = (1 + cos x) / sin x, or sin x / (1 - cos x) where cos x < 0.  267 FP64 instructions an
-// observation (290 before quot and inv_sqrt) against 440: 20 011 evaluations of 480 points 22.6 -> 17.7 ms, a curve of 20 000 points 132 ->
-// 127.  The error is no larger: 1.2e-16 rms of log10 either way for alpha' of 0.1 to 2, against
-// multiprecision, and 70 times smaller close to pi.
+// The Lommel-Seeliger magnitude of cuda.c:664-689 without its inverse and half-angle functions and without
+// their cancellation near alpha' = pi.  alpha' is the angle between the scaled vectors to the Sun and the Earth (lengths
+// S and E), lambda' the one between the first and their sum, nu = alpha' - lambda'.  With t = |S + E| / (S + E),
+//     cos lambda' + cos nu = 2 cos(alpha'/2) D,  D = cos((lambda' - nu)/2) = cos(alpha'/2) / t,
+//     sin lambda' sin nu = 2 (1 - t^2) D^2,  cot(lambda'/2) cot(nu/2) = (1 + t) / (1 - t)
+// (sums to products and the law of tangents), and the bracket of cuda.c:686 becomes
+//     2 D^2 (t - (1 - t^2) atanh t) = (1 + cos alpha') t g(t),  g(t) = sum of 2 t^(2k-2) / (4k^2 - 1), k = 1, 2, ...
+// The closed form from t = 1/2 on, where the difference loses less than three bits, and 25 terms of the series below
+// (the rest is under 2^-56 of the sum).  1 - t^2 = 2SE (1 - cos alpha') / (S + E)^2,
+// t^2 = ((S - E)^2 + 2SE (1 + cos alpha')) / (S + E)^2: no difference of nearly equal sums.  Every rounding explicit:
+// the same bits in every kernel.  Rms error against multiprecision, cuda.c's expressions in the second place:
+// 2.5e-16 mag (3.0e-16) for alpha' below 0.3, 4.8e-16 (7.2e-16) from 1.6 to 2.2, 6.9e-16 (6.8e-15) to 2.8 and
+// 1.4e-13 (1.6e-10) up to pi.  20 011 evaluations of 480 points take as long as with each angle's own sine and cosine
+// and their half-angle quotients (17.36 ms), whose error from 2.2 on was up to three times cuda.c's.
+struct LsSeries {
+    double c[25];
+};
+constexpr LsSeries make_ls_series()
+{
+    LsSeries s{};
+    for (int k = 1; k <= 25; k++) s.c[k - 1] = 2.0 / (4.0 * k * k - 1.0);
+    return s;
+}
+constexpr LsSeries kLsSeries = make_ls_series();
 AST_HD double ls_algebraic(double b, double c, double ib2, double ic2, double Sb, double Sc, double Sa, double Eb, double Ec,
                            double Ea)
 {
-    const double Tb = Sb * ib2, Tc = Sc * ic2;
-    const double S = sqrt(Sb * Tb + Sc * Tc + Sa * Sa);
-    const double E = sqrt(Eb * Eb * ib2 + Ec * Ec * ic2 + Ea * Ea);
-    const double SE = S * E;
-    const double ca = quot(Eb * Tb + Ec * Tc + Sa * Ea, SE);
-    const double sa = sqrt(1.0 - ca * ca);
-    const double inv = inv_sqrt(S * S + E * E + 2 * SE * ca);
-    const double cl = (S + E * ca) * inv, sl = E * sa * inv;
-    const double cn = (E + S * ca) * inv, sn = S * sa * inv;
-    const bool pl = !signbit(cl), pn = !signbit(cn);  // (the integer pipe's; a comparison is the FP64 unit's)
-    const double lp = pl ? 1.0 + cl : sl, lq = pl ? sl : 1.0 - cl;
-    const double np = pn ? 1.0 + cn : sn, nq = pn ? sn : 1.0 - cn;
-    return -2.5 * log10(b * c * SE * inv * (cn + cl - sl * sn * log(quot(lp * np, lq * nq))));
+    constexpr LsSeries series = kLsSeries;
+    const double Tb = DD_MUL(Sb, ib2), Tc = DD_MUL(Sc, ic2);
+    const double S = sqrt(DD_FMA(Sb, Tb, DD_FMA(Sc, Tc, DD_MUL(Sa, Sa))));
+    const double E = sqrt(DD_FMA(DD_MUL(Eb, Eb), ib2, DD_FMA(DD_MUL(Ec, Ec), ic2, DD_MUL(Ea, Ea))));
+    const double SE = DD_MUL(S, E), SE2 = DD_ADD(SE, SE);
+    const double ca = quot(DD_FMA(Eb, Tb, DD_FMA(Ec, Tc, DD_MUL(Sa, Ea))), SE);
+    const double p = DD_ADD(1.0, ca), a = DD_SUB(1.0, ca), d = DD_SUB(S, E);
+    const double iz = recip(DD_ADD(S, E)), iz2 = DD_MUL(iz, iz);
+    const double m = DD_MUL(DD_MUL(SE2, a), iz2);  // 1 - t^2
+    const double scale = DD_MUL(DD_MUL(DD_MUL(b, c), SE), iz);
+    double g;
+    if (m > 0.75) {
+        const double t2 = DD_MUL(DD_FMA(d, d, DD_MUL(SE2, p)), iz2);
+        g = series.c[24];
+#pragma unroll
+        for (int k = 23; k >= 0; k--) g = DD_FMA(g, t2, series.c[k]);
+        g = DD_MUL(g, p);
+    } else {
+        const double t2 = DD_SUB(1.0, m), rt = inv_sqrt(t2), q = DD_FMA(t2, rt, 1.0);
+        const double L = log(DD_MUL(DD_MUL(q, q), recip(m)));  // 2 atanh t
+        const double r2 = DD_MUL(rt, rt);
+        // 2 cos^2((lambda' - nu)/2): p / t^2, below a right angle 2 - 2 sin^2.
+        const double C = signbit(ca) ? DD_MUL(p, r2) : DD_FMA(-DD_MUL(DD_MUL(d, d), iz2), DD_MUL(a, r2), 2.0);
+        g = DD_MUL(C, DD_FMA(DD_MUL(-0.5, m), DD_MUL(rt, L), 1.0));
+    }
+    return DD_MUL(-2.5, log10(DD_MUL(scale, g)));
 }
 
 // Model magnitude at observation i for the Euler angles (phi, theta, psi): the body axes

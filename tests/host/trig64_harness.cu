@@ -22,3 +22,9 @@ extern "C" void h_quotients(int n, const double* u, const double* s, double* out
         out[2 * i + 1] = ast::inv_sqrt(fabs(s[i]));
     }
 }
+
+// out: 1 / s[i].
+extern "C" void h_recip(int n, const double* s, double* out)
+{
+    for (int i = 0; i < n; i++) out[i] = ast::recip(s[i]);
+}

@@ -112,3 +112,68 @@ def test_magnitude(lib, b, c):
             # 2.5 / ln 10 d ln B / d alpha', below 10 up to alpha' = 2.5.  The rest: twenty roundings of the factors.
             assert abs(g - want) <= (10 * 8 / mpmath.sin(al) + 1.09 * 20) * 2.0 ** -53 + 2.0 ** -52 * abs(want)
         assert compared > 50
+
+
+def test_reciprocals(lib):
+    rng = np.random.default_rng(8)
+    n = 4000
+    s = rng.choice([-1.0, 1.0], n) * rng.uniform(1, 2, n) * 2.0 ** rng.integers(-100, 100, n)
+    s[:4] = 1.0, np.nextafter(2.0, 0), np.nextafter(1.0, 2), -2.0
+    out = np.empty(n)
+    lib.h_recip(n, s.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.c_void_p))
+    with mpmath.workprec(200):
+        for si, r in zip(s, out):
+            want = 1 / mpmath.mpf(float(si))
+            # One rounding; the cubic step's e^3 < 2^-57 for a seed within 2^-19, a 16th of half an ulp.
+            assert abs(mpmath.mpf(float(r)) - want) <= 0.54 * np.spacing(abs(float(want)))
+
+
+def _magnitude(mp, b, c, ca, s, e):
+    """The magnitude from the scaled vectors' angle and lengths (cuda.c:664-689)."""
+    al = mp.acos(ca)
+    h = mp.sqrt(s * s + e * e + 2 * s * e * ca)
+    la = mp.atan2(e * mp.sin(al) / h, (s + e * ca) / h)
+    return -2.5 * mp.log10(b * c * s * e / h * (mp.cos(la - al) + mp.cos(la) + mp.sin(la) * mp.sin(la - al) *
+                                                mp.log(1 / mp.tan(la / 2) / mp.tan((al - la) / 2))))
+
+
+# Opposition, where data are dense and half angles small, and close to pi, where the two vectors nearly cancel.
+@pytest.mark.parametrize("b,c", [(1.0, 1.0), (0.7, 0.4), (0.9, 0.02)])
+@pytest.mark.parametrize("near", [0.0, np.pi])
+def test_magnitude_at_the_ends(lib, b, c, near):
+    rng = np.random.default_rng(11)
+    n = 200
+    d = rng.normal(size=(n, 3))
+    S = rng.normal(size=(n, 3))
+    off = np.geomspace(1e-5, 0.05 if near == 0.0 else 0.5, n)[:, None]
+    # Directions of the scaled vectors (x / b, y / c, z), off by the angle; then back to the body's.
+    u = S / np.linalg.norm(S, axis=1, keepdims=True)
+    w = np.cross(u, d)
+    w /= np.linalg.norm(w, axis=1, keepdims=True)
+    r = (1.0 if near == 0.0 else -1.0) * np.cos(off) * u + np.sin(off) * w
+    v = np.empty((n, 8))
+    v[:, 0], v[:, 1] = b, c
+    for k, x in ((2, u), (5, r)):
+        x = x * np.array([b, c, 1.0])
+        v[:, k:k + 3] = x / np.linalg.norm(x, axis=1, keepdims=True)
+    got = np.empty(n)
+    lib.h_ls_algebraic(n, v.ctypes.data_as(C.c_void_p), got.ctypes.data_as(C.c_void_p))
+    u53 = mpmath.mpf(2) ** -53
+    with mpmath.workprec(200):
+        B, K = mpmath.mpf(b), mpmath.mpf(c)
+        for vi, g in zip(v, got):
+            sb, sc, sa, eb, ec, ea = (mpmath.mpf(float(x)) for x in vi[2:])
+            s = mpmath.sqrt(sb * sb / (B * B) + sc * sc / (K * K) + sa * sa)
+            e = mpmath.sqrt(eb * eb / (B * B) + ec * ec / (K * K) + ea * ea)
+            ca = (sb * eb / (B * B) + sc * ec / (K * K) + sa * ea) / (s * e)
+            want = _magnitude(mpmath, B, K, ca, s, e)
+            # What eight roundings of cos alpha' (kept a cosine) and four of each length move it by, and twenty of the
+            # factors; sin alpha', 1 - cos and the sum of the vectors lose what the angle's cosine loses.
+            tol = 1.09 * 20 * u53 + 2 * u53 * abs(want)
+            one = mpmath.mpf(1) - u53 ** 2
+            for k in (-1, 1):
+                moved = max(-one, min(one, ca + 8 * k * u53))
+                tol += abs(_magnitude(mpmath, B, K, moved, s, e) - want)
+                tol += abs(_magnitude(mpmath, B, K, ca, s * (1 + 4 * k * u53), e) - want)
+                tol += abs(_magnitude(mpmath, B, K, ca, s, e * (1 + 4 * k * u53)) - want)
+            assert abs(g - want) <= tol, (float(mpmath.acos(ca)), float(g - want), float(tol))
