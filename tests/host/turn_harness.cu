@@ -67,6 +67,29 @@ void h_turn_steps(int torque, int n, double h, const double* mu, double* y)
     }
 }
 
+// One step of the general step alone (spin_step_general).
+void h_general_step(int torque, double h, const double* mu, double* y)
+{
+    const std::vector<float4> tab = table();
+    MixedState S;
+    S.torque = torque != 0;
+    S.bw = false;
+    for (int k = 0; k < (torque ? 6 : 3); k++) {
+        S.mu[k] = df_from_double(mu[k]);
+        S.y[k] = df_from_double(torque ? y[k] : y[3 + k]);
+    }
+    mixed_begin(S);
+    const df H = df_from_double(h), H6 = df_from_double(h / 6.0), Q = df_from_double(h / kTurnStep),
+             C6 = df_from_double(kTurnStep / (6.0 * h));
+    spin_step_beyond(S, float4{H.hi, H.lo, Q.hi, Q.lo}, float4{H6.hi, H6.lo, C6.hi, C6.lo}, tab.data());
+    df a[3];
+    spin_angles(S.s, S.torque, a);
+    for (int k = 0; k < 3; k++) {
+        if (torque) y[k] = df_to_double(S.s.w[k]) + (double)S.s.r[k];
+        y[3 + k] = df_to_double(a[k]);
+    }
+}
+
 // From y at time 0 to time t, with the step constants of prep_obs_point.
 void h_turn_interval(int torque, double t, double time_step, const double* mu, double* y)
 {

@@ -129,3 +129,55 @@ def test_intervals_down_to_nothing(lib, torque, t):
     assert np.max(np.abs((got[3:] - ref[3:] + math.pi) % (2 * math.pi) - math.pi)) <= tol
     if torque:
         assert np.max(np.abs(got[:3] - ref[:3])) <= (tol * 31 if t > 1e-17 else 0.0)
+
+
+# The general step (an angle that advances by more than 1000 turns in a step) where its outcome is determined: free
+# rotation about the body axis, mu = (L, Ip, 0), theta constant, phi and psi linear.
+@pytest.mark.parametrize("rate", [1e6, -1e6, 3e6, 2e7])
+@pytest.mark.parametrize("theta", [0.4, 1.2, 2.7])
+def test_the_general_step_of_free_rotation(lib, rate, theta):
+    y = np.array([0.0, 0.0, 0.0, 0.25, float(np.float32(theta)), -0.7])
+    mu = np.array([rate, 0.7, 0.0])
+    got = y.copy()
+    lib.h_turn_steps(0, 1, 1e-2, P(mu), P(got))
+    ref = _rk4(0, 1e-2, mu, y)
+    # Ten roundings of u^2 = 2^-48 of the angle's advance (twice it, of 2 psi) and of FP64's, and of pi.
+    tol = (10 * 2.0 ** -48 + 10 * 2.0 ** -53) * 2 * abs(rate) * 1e-2 + 16 * math.pi * 2.0 ** -48
+    d = (got[3:] - ref[3:] + math.pi) % (2 * math.pi) - math.pi
+    assert np.max(np.abs(d)) <= tol
+    assert abs(abs(got[4]) - theta) < 1e-6  # (theta itself does not advance)
+
+
+# With torque: rotation about the long axis alone, so that only psi advances, and w2 by the torque.
+@pytest.mark.parametrize("rate", [1e6, -3e6, 2e7])
+def test_the_general_step_with_torque(lib, rate):
+    y = np.array([0.0, 0.0, float(np.float32(rate)), 0.25, 1.2, -0.7])
+    mu = np.array([0.0, 0.0, 0.31, 0.0, 0.0, 8192.0])
+    got = y.copy()
+    lib.h_turn_steps(1, 1, 1e-2, P(mu), P(got))
+    ref = _rk4(1, 1e-2, mu, y)
+    tol = (10 * 2.0 ** -48 + 10 * 2.0 ** -53) * abs(rate) * 1e-2 + 16 * math.pi * 2.0 ** -48
+    d = (got[3:] - ref[3:] + math.pi) % (2 * math.pi) - math.pi
+    assert np.max(np.abs(d)) <= tol
+    assert np.max(np.abs(got[:3] - ref[:3])) <= 4 * 2.0 ** -48 * abs(rate)
+
+
+# The general step alone, at rates that the compact step takes: its own h, h/2, h/6 and h/3, all of mu, both layouts.
+@pytest.mark.parametrize("torque", [1, 0])
+@pytest.mark.parametrize("rate,h", [(0.5, 1e-2), (30.0, 1e-2), (60.0, 5e-3)])
+def test_the_general_step_at_ordinary_rates(lib, torque, rate, h):
+    lib.h_general_step.argtypes = [C.c_int, C.c_double, C.c_void_p, C.c_void_p]
+    rng = np.random.default_rng(int(rate) + torque)
+    for _ in range(50):
+        y = np.concatenate([rng.uniform(-rate, rate, 3), rng.uniform(-3, 3, 1), rng.uniform(0.3, 2.8, 1), rng.uniform(-3, 3, 1)])
+        y = np.array([float(np.float32(v)) for v in y])
+        mu = np.concatenate([rng.uniform(-0.5, 0.5, 3), rng.uniform(-1, 1, 3)]) if torque else np.array([rate, 0.7, 0.2])
+        got = y.copy()
+        lib.h_general_step(torque, h, P(mu), P(got))
+        ref = _rk4(torque, h, mu, y)
+        # As test_one_step_matches_fp64's, with the general step's own sin and cos (1e-13, dfloat.cuh) an advance.
+        tol = 2.0 ** -48 * (40 * 11.5 * (1 + rate * h) ** 2 + 16 * math.pi) + 4e-13 * (1 + rate * h) * 11.5
+        d = (got[3:] - ref[3:] + math.pi) % (2 * math.pi) - math.pi
+        assert np.max(np.abs(d)) <= tol
+        if torque:
+            assert np.max(np.abs(got[:3] - ref[:3])) <= tol * (1 + rate)
