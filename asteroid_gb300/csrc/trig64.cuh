@@ -2,12 +2,10 @@
 //
 // The FP64 kernels take the number of their FP64 instructions times the unit's 64 cycles (a lone
 // warp) or 19 (four warps on an SM), and most of an RK4 step's were the sine and cosine of two angles
-// in each stage: sincos() issues 25.  With a point of a table of 1024 angles next to x, at
-// most pi/1024 away, three terms of each series are enough and x's sine and cosine take 16; memory,
-// integer and predicate instructions run beside them.  159 -> 111 instructions an RK4 step on lanes of
-// a group, 340 -> 268 on one lane (torque); 20 011 evaluations of 480 points 27.1 -> 22.6 ms, one of 300
-// points 4.48 -> 3.98, 337 of 611 (black-and-white ball) 8.9 -> 6.9, a curve of 20 000 points 153 -> 132; with
-// each function on a lane of its own 3.86 -> 3.60, 6.9 -> 5.9 and 127 -> 117.
+// in each stage: sincos() issues 25.  With a point of a table of 1024 angles next to x, at most
+// pi/1024 away, three terms of each series are enough and x's sine and cosine take 16; memory,
+// integer and predicate instructions run beside them.  20 011 evaluations of 480 points 27.1 -> 22.6 ms, a
+// curve of 20 000 points 153 -> 117 with each function on a lane of its own.
 //
 // The table holds the points' sine and cosine as unevaluated sums of two doubles: the results are
 // within 0.6 ulp of 1 for one rounding of each sum, 1.2 ulp of themselves near the zeros
@@ -160,7 +158,8 @@ AST_HD void sincos_tab(double x, double* s, double* c, int shift = 0)
     if (c) *c = DD_ADD(P.c, DD_FMA(-P.s, sr, DD_FMA(P.c, v, P.cl)));
 }
 
-// 1/s and 1/sqrt(x) to 2^-22 or better, by the special function unit: no FP64 instruction.
+// 1/s and 1/sqrt(x) within 2^-20 (measured: 2^-20.02 and 2^-20.08; the instructions read and write the upper 32 bits
+// of a double), by the special function unit: no FP64 instruction.
 AST_HD double rcp_seed(double s)
 {
 #ifdef __CUDA_ARCH__
@@ -182,7 +181,8 @@ AST_HD double rsqrt_seed(double x)
 #endif
 }
 
-// 1 / s in three instructions: one cubic step (Householder's method of order 2), y + y (e + e^2), e = 1 - s y; 0.501 ulp.
+// 1 / s in three instructions: one cubic step (Householder's method of order 2), y + y (e + e^2), e = 1 - s y, leaves
+// e^3 < 2^-60; 0.51 ulp.
 AST_HD double recip(double s)
 {
     const double y = rcp_seed(s);
@@ -199,7 +199,7 @@ AST_HD double quot(double u, double s)
     return DD_FMA(DD_FMA(-s, q, u), y, q);
 }
 // 1 / sqrt(x) in six instructions, against twenty of root and division: the same step for x^(-1/2),
-// y + y e (1/2 + 3/8 e), e = 1 - x y^2; 1 ulp.
+// y + y e (1/2 + 3/8 e), e = 1 - x y^2 < 2^-19, leaves 5/16 e^3 < 2^-58; 1 ulp.
 AST_HD double inv_sqrt(double x)
 {
     const double y0 = rsqrt_seed(x);
