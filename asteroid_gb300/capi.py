@@ -121,6 +121,7 @@ class BatchTune(C.Structure):
         ("ctas", C.c_int32),
         ("evals_per_s", C.c_double),
         ("tile", C.c_int32),
+        ("pair", C.c_int32),
     ]
 
 

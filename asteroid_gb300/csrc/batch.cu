@@ -1040,12 +1040,32 @@ static decltype(&batch_tile_kernel<double, 16>) batch_tile_ptr(int T)
     return T == 8 ? batch_tile_kernel<double, 8> : T == 32 ? batch_tile_kernel<double, 32> : batch_tile_kernel<double, 16>;
 }
 
+// Integrators and photometers, k integrators a CTA: enough CTAs for the chains, at most one an SM (what an SM
+// holds) and what the slot pool has; each integrator takes 32 chains after the other.
+template <class CF>
+static int pair_geometry(ast_pool& P, int k)
+{
+    int64_t ctas = std::min<int64_t>(P.n_slots / (32 * k), P.sm_count);
+    if (P.chain_end > 0) ctas = std::min<int64_t>(ctas, (P.chain_end + 32 * k - 1) / (32 * k));
+    if (ctas < 1) return ast_set_error(AST_E_INVALID, "batch: slot pool smaller than one CTA");
+    P.pair = k;
+    P.tpb = 32 * pair_warps(k);
+    P.refill = 32;
+    P.tile = 0;
+    P.smem = sizeof(PairChain) * k;
+    P.ctas = (int)ctas;
+    return allow_smem(batch_pair_kernel<CF>, sizeof(PairChain) * kPairIntegrators);
+}
+
 // CTA size and refill mapping (and, tile > 0, the warp-tiled evaluation with tiles of that many
-// observations) -> CTAs (full occupancy, capped by the slot pool).
+// observations; pair > 0, that many integrators a CTA) -> CTAs (full occupancy, capped by the slot pool).
 template <class CF, int PREC>
-static int pool_geometry(ast_pool& P, int tpb, int refill, int tile = 0)
+static int pool_geometry(ast_pool& P, int tpb, int refill, int tile = 0, int pair = 0)
 {
     P.pair = 0;
+    if (PREC == AST_PREC_MIXED && P.lanes == 1 && pair >= 1 && pair <= kPairIntegrators && tpb == 32 * pair && refill == 32 &&
+        tile == 0)
+        return pair_geometry<CF>(P, pair);
     if (P.lanes > 1) return coop_geometry<CF, PREC>(P, 128);
     if (tpb < 32 || tpb > 256 || (tpb & 31)) return ast_set_error(AST_E_INVALID, "batch: tpb must be 32..256, x32");
     tpb = std::min(tpb, KernShape<PREC>::tpb);  // the kernel's launch bounds
@@ -1088,15 +1108,9 @@ template <class CF, int PREC>
 static int batch_geometry_default(ast_pool& P)
 {
     const int k = PREC == AST_PREC_MIXED ? pair_integrators(P.chain_end, P.sm_count, kPairIntegrators) : 0;
-    const int64_t ctas = k ? (P.chain_end + 32 * k - 1) / (32 * k) : 0;
-    if (!k || P.chain_end <= 0 || ctas * 32 * k > P.n_slots) return pool_geometry<CF, PREC>(P, 256, 1);
-    P.pair = k;
-    P.tpb = 32 * pair_warps(k);
-    P.refill = 32;
-    P.tile = 0;
-    P.smem = sizeof(PairChain) * k;
-    P.ctas = (int)ctas;
-    return allow_smem(batch_pair_kernel<CF>, sizeof(PairChain) * kPairIntegrators);
+    if (!k || P.chain_end <= 0 || (P.chain_end + 32 * k - 1) / (32 * k) * 32 * k > P.n_slots)
+        return pool_geometry<CF, PREC>(P, 256, 1);
+    return pair_geometry<CF>(P, k);
 }
 
 // One launch of the pool's kernel (thread per chain or warp per object, the warp-tiled evaluation, or
@@ -1221,7 +1235,7 @@ static int batch_run_t(ast_batch* B, const ast_batch_launch* tune, double* kerne
     batch_order(B);
     int rc;
     if (tune) {
-        if ((rc = pool_geometry<CF, PREC>(P, tune->tpb, tune->refill, tune->tile))) return rc;
+        if ((rc = pool_geometry<CF, PREC>(P, tune->tpb, tune->refill, tune->tile, tune->pair))) return rc;
     } else if (!P.ctas) {
         if ((rc = batch_geometry_default<CF, PREC>(P))) return rc;
     }
@@ -1438,7 +1452,7 @@ extern "C" int ast_batch_result(ast_batch* B, int32_t index, ast_fit_out* out)
 template <class CF, int PREC>
 static int batch_set_geometry_t(ast_batch* B, const ast_batch_launch* g)
 {
-    return pool_geometry<CF, PREC>(B->P, g->tpb, g->refill, g->tile);
+    return pool_geometry<CF, PREC>(B->P, g->tpb, g->refill, g->tile, g->pair);
 }
 
 extern "C" int ast_batch_set_geometry(ast_batch* B, const ast_batch_launch* g)
@@ -1457,6 +1471,7 @@ extern "C" int ast_batch_geometry(ast_batch* B, ast_batch_launch* out)
     out->refill = B->P.refill;
     out->ctas = B->P.ctas;
     out->tile = B->P.tile;
+    out->pair = B->P.pair;
     out->evals_per_s = 0;
     return AST_OK;
 }

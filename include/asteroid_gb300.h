@@ -443,6 +443,10 @@ typedef struct ast_batch_launch {
                              model with observation tiles -- the warp's 32 chains are integrated
                              one per lane through a tile of this many observations, then the
                              tile's 32 x T magnitudes are spread over the lanes (same results) */
+    int32_t pair;         /* 1 to 4 (refill 32, tile 0, tpb = 32 * pair, mixed precision): that many
+                             integrator warps a CTA, 32 chains each, with two photometer warps
+                             beside each (same results).  As ast_batch_geometry and ast_batch_tune
+                             return it; where the other fields do not go with it it counts as 0 */
 } ast_batch_launch;
 
 /* n_slots: persistent chain slots (0 = 256 per SM). */
@@ -464,11 +468,12 @@ int ast_batch_step(ast_batch* batch, int64_t evals_per_slot, int32_t* done, doub
 int ast_batch_result(ast_batch* batch, int32_t index, ast_fit_out* out);
 int ast_batch_counters(ast_batch* batch, int64_t* n_evals, int64_t* n_fits, int32_t* tpb, int32_t* refill,
                        int32_t* ctas);
-/* The launch geometry the batch runs with (tpb, refill, ctas, tile); evals_per_s is 0.  A batch whose
- * geometry is neither set nor tuned and whose chains are few runs integrator and photometer warps;
- * tpb is then the threads that run chains. */
+/* The launch geometry the batch runs with (tpb, refill, ctas, tile, pair); evals_per_s is 0.  A batch
+ * whose geometry is neither set nor tuned and whose chains are few runs integrator and photometer
+ * warps (pair > 0); tpb is then the threads that run chains.  Given to ast_batch_set_geometry or
+ * ast_batch_run it selects the same kernel. */
 int ast_batch_geometry(ast_batch* batch, ast_batch_launch* out);
-/* Set the geometry (tpb, refill, tile of *geometry) for the following ast_batch_step calls,
+/* Set the geometry (tpb, refill, tile, pair of *geometry) for the following ast_batch_step calls,
  * instead of the tuned or default one. */
 int ast_batch_set_geometry(ast_batch* batch, const ast_batch_launch* geometry);
 void ast_batch_destroy(ast_batch* batch);

@@ -129,3 +129,43 @@ def test_where_fits_by_pairs_end(gpu, flags, chains, span, precision, reopt, int
         b = eng.fit(n_chains=chains, group_size=32, seed=2, evals_cap=13, precision=precision, tpb=128, **kw)
     for k in ("best_f", "best_params", "best_dv", "chain_f"):
         assert np.array_equal(getattr(a, k), getattr(b, k), equal_nan=True), k
+
+
+def test_a_paired_geometry_read_back_selects_the_pairs(gpu):
+    """What ast_batch_geometry returns, given to ast_batch_run or ast_batch_set_geometry of another batch, runs the
+    same kernel (told by its time) with the same results; beside fields that do not go with it, pair counts as 0."""
+    model, obs, P = _object("TORQUE,ACC", 300, 2, 3, 0.05)
+
+    def batch():
+        b = api.Batch(precision=api.PREC_MIXED, acc=True)
+        b.add(model, obs, n_chains=4864, group_size=32, seed=4, evals_cap=30, reopt=True, params0=P[0])
+        return b
+
+    with batch() as b:
+        pairs, ref = min(b.run() for _ in range(3)), b.result(0)
+        c = b.counters()
+        g = {k: c[k] for k in ("tpb", "refill", "tile", "pair") if k in c}
+    with batch() as b:
+        threads = min(b.run(tpb=128) for _ in range(3))
+    assert pairs < 0.85 * threads
+    with batch() as b:
+        again = min(b.run(**g) for _ in range(3))
+        assert b.counters()["pair"] == g["pair"] > 0 and b.counters()["ctas"] == c["ctas"]
+        run = b.result(0)
+    with batch() as b:
+        b.set_geometry(**g)
+        step = 0.0
+        while True:
+            done, ms = b.step(8)
+            step += ms
+            if done:
+                break
+        stepped = b.result(0)
+    assert again < 1.1 * pairs and step < 1.3 * pairs, (pairs, threads, again, step)
+    with batch() as b:
+        for other in (dict(g, tpb=64), dict(g, refill=1), dict(g, tile=8), dict(g, pair=5, tpb=160)):
+            b.set_geometry(**other)
+            assert b.counters()["pair"] == 0
+    for r in (run, stepped):
+        for k in ("best_f", "best_params", "best_dv"):
+            assert np.array_equal(getattr(r, k), getattr(ref, k), equal_nan=True)
