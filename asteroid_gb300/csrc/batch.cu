@@ -1264,10 +1264,10 @@ static int batch_run_t(ast_batch* B, const ast_batch_launch* tune, double* kerne
 
 // One bounded launch from a fresh slot state: evaluations per second of this geometry.
 template <class CF, int PREC>
-static int batch_probe(ast_batch* B, int tpb, int refill, int tile, int64_t evals_per_slot, double* rate)
+static int batch_probe(ast_batch* B, int tpb, int refill, int tile, int pair, int64_t evals_per_slot, double* rate)
 {
     ast_pool& P = B->P;
-    int rc = pool_geometry<CF, PREC>(P, tpb, refill, tile);
+    int rc = pool_geometry<CF, PREC>(P, tpb, refill, tile, pair);
     if (rc) return rc;
     if ((rc = upload_table<CF>(P))) return rc;
     const FitView<CF> V = pool_view<CF>(P);
@@ -1298,16 +1298,17 @@ static int batch_tune_t(ast_batch* B, int64_t evals_per_slot, ast_batch_launch* 
     const int refills[2] = {1, 32};
     const int tiles[3] = {8, 16, 32};
     double best_rate = -1;
-    ast_batch_launch bt{256, 1, 0, 0.0, 0};
-    auto probe = [&](int t, int r, int tile) -> int {
+    ast_batch_launch bt{256, 1, 0, 0.0, 0, 0};
+    auto probe = [&](int t, int r, int tile, int pair = 0) -> int {
         double rate = 0;
-        int rc = batch_probe<CF, PREC>(B, t, r, tile, evals_per_slot, &rate);
+        int rc = batch_probe<CF, PREC>(B, t, r, tile, pair, evals_per_slot, &rate);
         if (rc) return rc;
         if (rate > best_rate) {
             best_rate = rate;
             bt.tpb = t;
             bt.refill = r;
             bt.tile = tile;
+            bt.pair = pair;
         }
         return AST_OK;
     };
@@ -1324,7 +1325,13 @@ static int batch_tune_t(ast_batch* B, int64_t evals_per_slot, ast_batch_launch* 
                 if (t > KernShape<PREC>::tpb) continue;
                 if (int rc = probe(t, 32, tile)) return rc;
             }
-    int rc = pool_geometry<CF, PREC>(B->P, bt.tpb, bt.refill, bt.tile);
+    // Integrators and photometers where an untuned batch runs them: two and four integrators a CTA, of the
+    // sizes above (4 864 chains of 300 points: one a CTA 14.4 ms, two 13.4, three 14.7, four 16.5).
+    if (PREC == AST_PREC_MIXED && pair_integrators(B->P.chain_end, B->P.sm_count, kPairIntegrators))
+        for (int t : tpbs)
+            if (t <= 32 * kPairIntegrators && B->P.n_slots >= t)
+                if (int rc = probe(t, 32, 0, t / 32)) return rc;
+    int rc = pool_geometry<CF, PREC>(B->P, bt.tpb, bt.refill, bt.tile, bt.pair);
     if (rc) return rc;
     // Back to the untouched state: the probes ran chains that the batch will run again.
     ast_pool& P = B->P;

@@ -454,7 +454,7 @@ int ast_batch_create(int32_t device, int32_t precision, int32_t acc, int64_t n_s
 /* Upload one object; *index numbers objects from 0 in the order added. */
 int ast_batch_add(ast_batch* batch, const ast_model* model, const ast_obs_set* obs, const ast_fit_cfg* cfg,
                   int32_t* index);
-/* Autotuner: times every (tpb, refill, tile) candidate on this batch with bounded launches of
+/* Autotuner: times every (tpb, refill, tile, pair) candidate on this batch with bounded launches of
  * evals_per_slot evaluations per slot, keeps the fastest for ast_batch_run / ast_batch_step and
  * returns it.  Call it before those: it leaves the batch in its initial state. */
 int ast_batch_tune(ast_batch* batch, int64_t evals_per_slot, ast_batch_launch* best);

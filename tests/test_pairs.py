@@ -169,3 +169,20 @@ def test_a_paired_geometry_read_back_selects_the_pairs(gpu):
     for r in (run, stepped):
         for k in ("best_f", "best_params", "best_dv"):
             assert np.array_equal(getattr(r, k), getattr(ref, k), equal_nan=True)
+
+
+def test_the_tuner_times_pairs(gpu):
+    """A tuned batch of few chains is no slower than one that is not, and gives the same results."""
+    model, obs, P = _object("TORQUE,ACC", 300, 2, 3, 0.05)
+    got = []
+    for tune in (False, True):
+        with api.Batch(precision=api.PREC_MIXED, acc=True) as b:
+            b.add(model, obs, n_chains=4864, group_size=32, seed=4, evals_cap=30, reopt=True, params0=P[0])
+            if tune:
+                t = b.tune(evals_per_slot=4)
+            got.append((min(b.run() for _ in range(3)), b.result(0)))
+            if tune:
+                assert t["pair"] > 0 and t["tpb"] == 32 * t["pair"] and b.counters()["pair"] == t["pair"]
+    assert got[1][0] < 1.1 * got[0][0], (got[0][0], got[1][0])
+    for k in ("best_f", "best_params", "best_dv"):
+        assert np.array_equal(getattr(got[0][1], k), getattr(got[1][1], k), equal_nan=True)
