@@ -124,7 +124,7 @@ def build_engine(force: bool = False, ptxas_verbose: bool = False) -> Path:
 PARITY = BUILD / "parity"
 
 
-def build_parity_engine(force: bool = False) -> Path:
+def build_parity_engine(force: bool = False, contract: bool = False) -> Path:
     """The engine with engine.cu -- the evaluation kernels behind ast_eval_batch -- compiled
     without fused multiply-adds (nvcc -fmad=false), linked with the other objects of the main
     build into _build/parity/libasteroid_gb300.so.  Test infrastructure for the FP64 parity
@@ -132,18 +132,22 @@ def build_parity_engine(force: bool = False) -> Path:
     sides then round every product and sum separately, so only the order of operations and
     CUDA's libm are left to differ.  It evaluates with CUDA's sincos in the reference's
     expressions (AST_LIBRARY_TRIG, as the FP64 simplex search does), not with the table and the
-    rearranged magnitude of the evaluation kernels.  Loaded in a child process through AST_ENGINE_LIB."""
+    rearranged magnitude of the evaluation kernels.  With contract, the same expressions with nvcc's
+    multiply-adds, in _build/parity_fma: what the shipped evaluations are compared with
+    (tests/test_eval_parity.py).  Loaded in a child process through AST_ENGINE_LIB."""
     build_engine()
-    PARITY.mkdir(exist_ok=True)
+    out = BUILD / "parity_fma" if contract else PARITY
+    out.mkdir(exist_ok=True)
     nvcc = _nvcc()
     src = PKG / "csrc" / "engine.cu"
-    obj = PARITY / "engine.o"
+    obj = out / "engine.o"
+    fma = [] if contract else ["-fmad=false"]
     if force or _stale(obj, [src] + _headers()):
-        _run([nvcc, *GENCODE, "-lineinfo", "-O3", "-std=c++17", "-fmad=false", "-DAST_LIBRARY_TRIG", "-Xcompiler",
+        _run([nvcc, *GENCODE, "-lineinfo", "-O3", "-std=c++17", *fma, "-DAST_LIBRARY_TRIG", "-Xcompiler",
               "-fPIC,-O2,-ffp-contract=off", f"-I{INCLUDE}", f"-I{PKG / 'host'}", "-c", str(src), "-o", str(obj)])
     objs = [obj] + [BUILD / (Path(s).stem + ".o") for s in CU_SOURCES if Path(s).stem != "engine"]
     objs += [BUILD / (Path(s).stem + ".o") for s in C_SOURCES]
-    lib = PARITY / "libasteroid_gb300.so"
+    lib = out / "libasteroid_gb300.so"
     if force or _stale(lib, objs):
         _run([nvcc, *GENCODE, "-shared", "-o", str(lib), *map(str, objs), "-lcudart", *_zlib()[1]])
     return lib
