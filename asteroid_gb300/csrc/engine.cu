@@ -400,7 +400,7 @@ static int launch_eval(ast_ctx* c, const DevModel& dm, const double* d_params, i
                        cudaStream_t s, unsigned long long* d_err)
 {
     if (PREC == AST_PREC_FP64) {
-        const int g = group_lanes(n, c->sm_count);
+        const int g = group_lanes(n, c->sm_count, group_most_eval());
         if (g == 32) return launch_eval_group<CF, 32>(c, dm, d_params, n, d_chi2, d_dv, s);
         if (g == 8) return launch_eval_group<CF, 8>(c, dm, d_params, n, d_chi2, d_dv, s);
         // The FP64 unit is the SM's: an SM takes its warps' instructions one after the other, so the

@@ -119,14 +119,20 @@ inline int obs_smem_for(K kern, size_t bytes, size_t optin, size_t* smem)
 
 // Lanes an FP64 evaluation by the number that run side by side (1: one thread each).  A warp alone on its
 // quarter of the SM costs its FP64 instructions times 64 cycles, four on an SM 19 each (group64.cuh):
-// eight lanes an evaluation need 2.2 to 3 times fewer, so they win until the SMs hold four such
-// warps twice over; from there the FP64 unit is full either way and threads do the least.
+// eight lanes an evaluation need 2.2 to 3 times fewer, so they win until the SMs hold `most` evaluations, seven
+// such warps (a search with torque six); from there the FP64 unit is full either way and threads do the least.
 // Thirty-two lanes share the magnitudes of four times as many observations and win while every
-// evaluation still has a quarter of an SM.
-inline int group_lanes(int64_t n, int sm_count)
+// evaluation still has a quarter of an SM.  Eight lanes against threads, ms, by evaluations an SM (152 SMs, 60
+// points, 30 RK4 steps an observation; searches of 13 evaluations a chain, their sines the library's):
+//   evaluations, torque     28: 12.9/14.0   32: 14.8/14.0     free 28: 8.7/10.4   32: 9.9/10.4
+//   searches, torque        24: 521/571     28: 598/571       free 28: 299/325    32: 342/325
+// and 32 lanes against 8, 10 steps an observation: evaluations 4: 3.06/2.97, 6: 3.67/2.97; searches 4: 130/133, 6: 155/134.
+inline int group_lanes(int64_t n, int sm_count, int most)
 {
-    return n <= 4 * (int64_t)sm_count ? 32 : n <= 32 * (int64_t)sm_count ? 8 : 1;
+    return n <= 4 * (int64_t)sm_count ? 32 : n <= (int64_t)most * sm_count ? 8 : 1;
 }
+inline int group_most_eval() { return 28; }
+inline int group_most_fit(int flags) { return flags & AST_TORQUE ? 24 : 28; }
 
 // Integrator warps of a CTA of the paired mixed kernels (mixed.cuh), by the number of evaluations that run
 // side by side; 0: one thread an evaluation, both parts.  At most `most` (pair_most_eval, pair_most_fit).

@@ -414,12 +414,12 @@ static int64_t fit_slots(const FitRun& r)
 // `obs_bytes` is the observation block's size, `optin` the device's per-CTA shared-memory limit.
 template <class CF, int PREC>
 static int fit_launch_core(int sm_count, size_t obs_bytes, size_t optin, int tpb_req, int minb_req, int stage_req,
-                           int64_t n_chains, int pair_most, FitRun* r)
+                           int64_t n_chains, int group_most, int pair_most, FitRun* r)
 {
     // FP64 with no geometry asked for: lane groups while they are faster (group_lanes).
     r->lanes = 1;
     if (PREC == AST_PREC_FP64 && tpb_req <= 0 && minb_req <= 0 && stage_req == 0) {
-        r->lanes = group_lanes(n_chains, sm_count);
+        r->lanes = group_lanes(n_chains, sm_count, group_most);
         if (r->lanes > 1) {
             r->tpb = 32;
             r->ctas = (int)((n_chains * r->lanes + 31) / 32);
@@ -492,7 +492,7 @@ static int fit_launch_cfg(ast_ctx* c, const ast_fit_cfg* cfg, FitRun* r)
 {
     const int most = pair_most_fit(PREC, c->dm.flags, cfg->reopt != 0, c->span / c->dm.time_step / c->n_data);
     return fit_launch_core<CF, PREC>(c->sm_count, (size_t)c->layout.bytes, c->smem_optin, cfg->tpb, cfg->min_ctas_per_sm,
-                                     cfg->stage_obs, cfg->n_chains, most, r);
+                                     cfg->stage_obs, cfg->n_chains, group_most_fit(c->dm.flags), most, r);
 }
 
 extern "C" int ast_fit_begin(ast_ctx* c, const ast_fit_cfg* cfg)
@@ -881,14 +881,16 @@ extern "C" int ast_fit_noalloc(const ast_model* model, const ast_obs_set* obs, c
     AST_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     AST_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     FitRun r;
+    const int gm = group_most_fit(dm.flags), pm = kPairIntegrators;  // (no more than one integrator an SM)
+    const int tpb = cfg->tpb, mb = cfg->min_ctas_per_sm, so = cfg->stage_obs;
+    const int64_t C = cfg->n_chains;
+    const bool fp64 = cfg->precision == AST_PREC_FP64;
     if (acc)
-        rc = cfg->precision == AST_PREC_FP64
-                 ? fit_launch_core<double, AST_PREC_FP64>(sms, L.bytes, optin, cfg->tpb, cfg->min_ctas_per_sm, cfg->stage_obs, cfg->n_chains, kPairIntegrators, &r)
-                 : fit_launch_core<double, AST_PREC_MIXED>(sms, L.bytes, optin, cfg->tpb, cfg->min_ctas_per_sm, cfg->stage_obs, cfg->n_chains, kPairIntegrators, &r);
+        rc = fp64 ? fit_launch_core<double, AST_PREC_FP64>(sms, L.bytes, optin, tpb, mb, so, C, gm, pm, &r)
+                  : fit_launch_core<double, AST_PREC_MIXED>(sms, L.bytes, optin, tpb, mb, so, C, gm, pm, &r);
     else
-        rc = cfg->precision == AST_PREC_FP64
-                 ? fit_launch_core<float, AST_PREC_FP64>(sms, L.bytes, optin, cfg->tpb, cfg->min_ctas_per_sm, cfg->stage_obs, cfg->n_chains, kPairIntegrators, &r)
-                 : fit_launch_core<float, AST_PREC_MIXED>(sms, L.bytes, optin, cfg->tpb, cfg->min_ctas_per_sm, cfg->stage_obs, cfg->n_chains, kPairIntegrators, &r);
+        rc = fp64 ? fit_launch_core<float, AST_PREC_FP64>(sms, L.bytes, optin, tpb, mb, so, C, gm, pm, &r)
+                  : fit_launch_core<float, AST_PREC_MIXED>(sms, L.bytes, optin, tpb, mb, so, C, gm, pm, &r);
     if (rc) return rc;
     const int64_t slots = fit_slots(r), S = (slots + 31) / 32 * 32;
     int64_t off[20];

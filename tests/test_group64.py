@@ -89,3 +89,17 @@ def test_fits_by_lane_groups_equal_threads(gpu, flags, chains, group, kw):
         for k in ("best_f", "best_params", "best_dv", "chain_f"):
             assert np.array_equal(getattr(r, k), getattr(b, k), equal_nan=True), k
         assert r.n_evals == b.n_evals and r.n_fits == b.n_fits
+
+
+# The most chains by lane groups, and one more: with torque, whose step has more FP64 instructions to spread, and without.
+@pytest.mark.parametrize("flags,per_sm", [("TORQUE,ACC", 24), ("ACC", 28), ("BW_BALL", 28)])
+def test_where_fits_by_lane_groups_end(gpu, flags, per_sm):
+    model, obs, P = _object(flags, 33, 2, 5, 1.0)
+    n = per_sm * _sms()
+    with api.Engine(model, obs) as eng:
+        for chains, lanes in ((n, 8), (n + 1, 1)):
+            a = eng.fit(n_chains=chains, group_size=1, seed=9, evals_cap=13)
+            assert eng.fit_launch()["ctas"] == -(-chains * lanes // 32)
+            b = eng.fit(n_chains=chains, group_size=1, seed=9, evals_cap=13, tpb=32)
+            for k in ("best_f", "best_params", "best_dv", "chain_f"):
+                assert np.array_equal(getattr(a, k), getattr(b, k), equal_nan=True), k
