@@ -285,7 +285,9 @@ AST_HD df ls_f_df(df t)
     return df_sub(t, df_mul(one_m_z, df{0.5f * at.hi, 0.5f * at.lo}));
 }
 
-// ls_magnitude_f in double-float: the same cancellation-free Lommel-Seeliger form.
+// ls_magnitude_f in double-float: the same cancellation-free Lommel-Seeliger form.  U: the unrolling of its
+// loops (nudge_flush).
+template <int U = 1>
 AST_HD df ls_magnitude_df(const df* Sp, const df* Ep, df ib, df ic, df bc, const float4* tab)
 {
     const df sv[3] = {df_mul(Sp[0], ib), df_mul(Sp[1], ic), Sp[2]};
@@ -298,10 +300,10 @@ AST_HD df ls_magnitude_df(const df* Sp, const df* Ep, df ib, df ic, df bc, const
     df_cross3(sv, ev, cr);
     const df cn = df_sqrt(df_dot3(cr, cr));
     df x[3] = {df_dot3(sv, hv), df_dot3(hv, ev), df_neg(df_dot3(sv, ev))};  // to mu, nu, eps
-#pragma unroll 1
+#pragma unroll U
     for (int k = 0; k < 3; k++) x[k] = df_atan2(cn, x[k], tab);
     df h[2] = {df_sub(x[0], x[1]), x[2]}, sn[2], cs[2];
-#pragma unroll 1
+#pragma unroll U
     for (int k = 0; k < 2; k++) df_sincos(df{0.5f * h[k].hi, 0.5f * h[k].lo}, tab, &sn[k], &cs[k]);
     const df D = cs[0], s = sn[1];
     const df B = df_mul(df_mul(df{2.0f * D.hi, 2.0f * D.lo}, D), ls_f_df(df_div(s, D)));
@@ -355,10 +357,11 @@ AST_HD DfFrame make_df_frame(const DevModel& M, const double* params)
 
 // Model magnitude at observation i for the double-float Euler angles ang = (phi, theta, psi):
 // the body frame as in cuda.c:432-473, then ls_magnitude_df or the BW_BALL law (cuda.c:568-580).
+template <int U = 1>
 AST_HD double vmod_df(const DevModel& M, const ObsView& o, const DfFrame& F, const df* ang, int i, const float4* tab)
 {
     df sn[3], cs[3];
-#pragma unroll 1
+#pragma unroll U
     for (int k = 0; k < 3; k++) df_sincos(ang[k], tab, &sn[k], &cs[k]);
     const df sph = sn[0], cph = cs[0], sth = sn[1], cth = cs[1], sps = sn[2], cps = cs[2];
     const df N[3] = {df_add(df_mul(F.XM_x, cph), df_mul(F.YM[0], sph)), df_mul(F.YM[1], sph),
@@ -385,7 +388,7 @@ AST_HD double vmod_df(const DevModel& M, const ObsView& o, const DfFrame& F, con
     const df S[3] = {df_from_double(o.sx[i]), df_from_double(o.sy[i]), df_from_double(o.sz[i])};
     const df Sp[3] = {df_dot3(b, S), df_dot3(c, S), df_dot3(a, S)};
     const df Ep[3] = {df_dot3(b, E), df_dot3(c, E), df_dot3(a, E)};
-    return df_to_double(ls_magnitude_df(Sp, Ep, F.ib, F.ic, F.bc, tab));
+    return df_to_double(ls_magnitude_df<U>(Sp, Ep, F.ib, F.ic, F.bc, tab));
 }
 
 // NUDGE minimum candidates of the mixed path: observation i and the Euler angles at i-2, i-1, i.
@@ -404,9 +407,12 @@ struct NudgeCand {
 // The reference's test and parabola (cuda.c:716-760) on each queued triple, with double-float
 // magnitudes.  Returns false as soon as more than AST_M_MAX minima are found (the model is then
 // rejected exactly as the reference rejects it, only after a few more observations).
-// Not inlined: the magnitude code is cold and large, and one copy serves both call sites.  One copy of the
-// magnitude, too, and of its sines and arctangents: 80 KB instead of 278, which with the step did not fit the
-// instruction cache (torqued NUDGE fits from the prior, 19 456 chains of 60 points: 45 ms against 92).
+// Not inlined: the magnitude code is cold and large, and one copy serves both call sites.  U = 1, one copy of
+// the magnitude, too, and of its sines and arctangents: 80 KB instead of 278, which with the step and the general
+// step did not fit the instruction cache (torqued NUDGE fits from the prior, 19 456 chains of 60 points: 45 ms against
+// 92).  The thread kernels of the FP32 right-hand side have neither step and keep U = 3 (with U = 1 they lose 2 to
+// 4 % without NUDGE, by the code that the compiler then makes of the step; their paired kernels lose 0 to 4 % with 3).
+template <int U>
 static __host__ __device__ __noinline__ bool nudge_flush(const DevModel& M, const ObsView& o, const DfFrame& F,
                                                          const float4* tab, NudgeCand* cand, int* n_cand, int* Mmin,
                                                          float* t_mod, float* V_mod)
@@ -414,8 +420,8 @@ static __host__ __device__ __noinline__ bool nudge_flush(const DevModel& M, cons
     for (int q = 0; q < *n_cand; q++) {
         const int ic = cand[q].i;
         double v[3];
-#pragma unroll 1
-        for (int j = 0; j < 3; j++) v[j] = vmod_df(M, o, F, cand[q].a[j], ic - 2 + j, tab);
+#pragma unroll U
+        for (int j = 0; j < 3; j++) v[j] = vmod_df<U>(M, o, F, cand[q].a[j], ic - 2 + j, tab);
         const float f0 = (float)v[0], f1 = (float)v[1];
         const double v2 = v[2];
         if (f1 > f0 && f1 >= v2) {
@@ -785,6 +791,7 @@ AST_HD void mixed_sums_begin(const DevModel& M, MixedSums& Q)
 
 // Observation i (magnitude v, weight w, filter m) with model magnitude Vmod and Euler angles ang.  Returns
 // false once there are more than M_MAX minima.
+template <int U>
 AST_HD bool mixed_observe(const DevModel& M, const ObsView& o, const DfFrame& F, const float4* tab, MixedSums& Q, MixedLast& E,
                           MixedQueue& W, int i, float v, float w, int m, float Vmod, const df* ang)
 {
@@ -816,7 +823,7 @@ AST_HD bool mixed_observe(const DevModel& M, const ObsView& o, const DfFrame& F,
                 q.a[1][k] = E.ang[1][k];
                 q.a[2][k] = ang_i[k];
             }
-            if (++W.n_cand == kNudgeQueue && !nudge_flush(M, o, F, tab, W.cand, &W.n_cand, &W.Mmin, W.t_mod, W.V_mod))
+            if (++W.n_cand == kNudgeQueue && !nudge_flush<U>(M, o, F, tab, W.cand, &W.n_cand, &W.Mmin, W.t_mod, W.V_mod))
                 return false;
         }
     }
@@ -833,12 +840,12 @@ AST_HD bool mixed_observe(const DevModel& M, const ObsView& o, const DfFrame& F,
 }
 
 // chi^2 and delta_V of the sums, with the reward and punishment factors of the minima (cuda.c:887-993).
-template <class CF>
+template <class CF, int U>
 __host__ __device__ CF mixed_finish(const DevModel& M, const ObsView& o, const DfFrame& F, const float4* tab, const MixedSums& Q,
                                     MixedQueue& W, CF* delta_V)
 {
     const int N_filters = M.n_filters;
-    if ((M.flags & AST_NUDGE) && !nudge_flush(M, o, F, tab, W.cand, &W.n_cand, &W.Mmin, W.t_mod, W.V_mod)) return (CF)kHuge;
+    if ((M.flags & AST_NUDGE) && !nudge_flush<U>(M, o, F, tab, W.cand, &W.n_cand, &W.Mmin, W.t_mod, W.V_mod)) return (CF)kHuge;
     CF dv[AST_MAX_FILTERS];
     CF chi2a = mixed_combine<CF>(M, o, Q.sum_y, Q.sum_y2, dv);
     if (M.flags & AST_NUDGE) {
@@ -893,6 +900,7 @@ template <class CF, bool RHS32 = false>
 __host__ __device__ CF chi2_mixed(const DevModel& M, const ObsView& o, const double* params, CF* delta_V, const float4* tab,
                                   double* ang_out = nullptr)
 {
+    constexpr int U = RHS32 ? 3 : 1;
     MixedSums Q;
     MixedLast E;
     MixedQueue W;
@@ -909,9 +917,9 @@ __host__ __device__ CF chi2_mixed(const DevModel& M, const ObsView& o, const dou
             for (int k = 0; k < 3; k++) ang_out[3 * i + k] = df_to_double(ang[k]);
         const float Vmod = mixed_vmod(S.F, S.bw, DF_ADD(ang[0].hi, ang[0].lo), DF_ADD(ang[1].hi, ang[1].lo),
                                       DF_ADD(ang[2].hi, ang[2].lo), o, i);
-        if (!mixed_observe(M, o, F, tab, Q, E, W, i, o.v[i], o.w[i], o.f[i], Vmod, ang)) return (CF)kHuge;
+        if (!mixed_observe<U>(M, o, F, tab, Q, E, W, i, o.v[i], o.w[i], o.f[i], Vmod, ang)) return (CF)kHuge;
     }
-    return mixed_finish<CF>(M, o, F, tab, Q, W, delta_V);
+    return mixed_finish<CF, U>(M, o, F, tab, Q, W, delta_V);
 }
 
 #ifdef __CUDACC__
@@ -1050,6 +1058,7 @@ template <class CF, bool RHS32, int PW>
 __device__ CF pair_observe(const DevModel& M, const ObsView& o, const double* params, CF* delta_V, const float4* tab,
                            const PairTile& B, int chain, int id, int threads)
 {
+    constexpr int U = 1;
     const int sub = threadIdx.x & (PW - 1);
     MixedSums Q;
     MixedLast E;
@@ -1073,10 +1082,6 @@ __device__ CF pair_observe(const DevModel& M, const ObsView& o, const double* pa
             pair_read<RHS32>(B.ang[b][j], chain, torque, ang);
             const float V = mixed_vmod(S, bw, DF_ADD(ang[0].hi, ang[0].lo), DF_ADD(ang[1].hi, ang[1].lo),
                                        DF_ADD(ang[2].hi, ang[2].lo), o, i);
-            if (PW == 1) {
-                if (!huge) huge = !mixed_observe(M, o, F, tab, Q, E, W, i, v, w, m, V, ang);
-                continue;
-            }
 #pragma unroll
             for (int q = 0; q < PW; q++) {
                 const float Vq = __shfl_sync(0xffffffffu, V, q, PW), vq = __shfl_sync(0xffffffffu, v, q, PW),
@@ -1084,11 +1089,11 @@ __device__ CF pair_observe(const DevModel& M, const ObsView& o, const double* pa
                 const int mq = __shfl_sync(0xffffffffu, m, q, PW);
                 if (j0 + q >= n || huge) continue;
                 if (M.flags & AST_NUDGE) pair_read<RHS32>(B.ang[b][j0 + q], chain, torque, ang);
-                huge = !mixed_observe(M, o, F, tab, Q, E, W, i0 + j0 + q, vq, wq, mq, Vq, ang);
+                huge = !mixed_observe<U>(M, o, F, tab, Q, E, W, i0 + j0 + q, vq, wq, mq, Vq, ang);
             }
         }
     }
-    return huge ? (CF)kHuge : mixed_finish<CF>(M, o, F, tab, Q, W, delta_V);
+    return huge ? (CF)kHuge : mixed_finish<CF, U>(M, o, F, tab, Q, W, delta_V);
 }
 
 // One evaluation for the integrator of a PairChain: params on the lanes of `live` (not empty; the others
