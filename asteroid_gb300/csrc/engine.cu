@@ -399,7 +399,7 @@ template <class CF, int PREC>
 static int launch_eval(ast_ctx* c, const DevModel& dm, const double* d_params, int64_t n, double* d_chi2, double* d_dv,
                        cudaStream_t s, unsigned long long* d_err)
 {
-    if (PREC == AST_PREC_FP64) {
+    if constexpr (PREC == AST_PREC_FP64) {
         const int g = group_lanes(n, c->sm_count, group_most_eval());
         if (g == 32) return launch_eval_group<CF, 32>(c, dm, d_params, n, d_chi2, d_dv, s);
         if (g == 8) return launch_eval_group<CF, 8>(c, dm, d_params, n, d_chi2, d_dv, s);
@@ -410,31 +410,36 @@ static int launch_eval(ast_ctx* c, const DevModel& dm, const double* d_params, i
             dm, c->d_obs, c->layout, 0, d_params, n, d_chi2, d_dv, d_err);
         AST_CUDA(cudaGetLastError());
         return AST_OK;
-    }
-    if (PREC != AST_PREC_FP64)
+    } else {
         if (const int k = pair_integrators(n, c->sm_count, pair_most_eval(dm.flags)))
-            return launch_eval_pair<CF, PREC == AST_PREC_FP64 ? AST_PREC_MIXED : PREC>(c, dm, k, d_params, n, d_chi2, d_dv, s);
-    // As the fits (fit_launch_core): the precision's own shape when the vectors fill it, the full
-    // register file when they do not (1001 vectors of 480 points, mixed: 1.19 ms against 1.33).
-    constexpr int kFull = KernShape<PREC>::min_ctas;
-    auto kern = n < (int64_t)c->sm_count * 128 * kFull ? eval_kernel<CF, PREC, 1> : eval_kernel<CF, PREC, kFull>;
-    size_t smem = 0;
-    int rc = obs_smem_for(kern, (size_t)c->layout.bytes, c->smem_optin, &smem);
-    if (rc) return rc;
-    const int tpb = 128;
-    // Staged in shared memory only where that leaves the SM as many CTAs (fit_launch_core's rule).
-    int per_sm = 1, staged = 0;
-    AST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, tpb, 0));
-    if (smem) AST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&staged, kern, tpb, smem));
-    if (staged < per_sm) smem = 0;
-    if (per_sm < 1) per_sm = 1;
-    int64_t blocks = (n + tpb - 1) / tpb;
-    const int64_t cap = (int64_t)c->sm_count * per_sm;
-    if (blocks > cap) blocks = cap;
-    if (blocks < 1) blocks = 1;
-    kern<<<(unsigned)blocks, tpb, smem, s>>>(dm, c->d_obs, c->layout, smem ? 1 : 0, d_params, n, d_chi2, d_dv, d_err);
-    AST_CUDA(cudaGetLastError());
-    return AST_OK;
+            return launch_eval_pair<CF, PREC>(c, dm, k, d_params, n, d_chi2, d_dv, s);
+        // The full register file while two CTAs of 128 an SM, what it holds then, take the vectors at once;
+        // beyond, the precision's own shape, three of them (300 points, 42 000 vectors: 1.43 ms against 1.18 for
+        // half a day, the FP32 right-hand side 2.53 against 1.84 for eight).  The double-float step with torque loses
+        // more by three CTAs' registers than the few CTAs of a second round cost, until they meet on an SM
+        // (20 days: 39 000 vectors 4.79 against 4.93; black-and-white ball, 8 days: 52 000 2.24 against 2.28, 58 367
+        // 3.03 against 2.28).
+        constexpr int kFull = KernShape<PREC>::min_ctas;
+        const bool steps = PREC == AST_PREC_MIXED && (dm.flags & AST_TORQUE) && c->span >= 2 * dm.time_step * dm.n_data;
+        auto kern = n <= (int64_t)c->sm_count * (steps ? 340 : 256) ? eval_kernel<CF, PREC, 1> : eval_kernel<CF, PREC, kFull>;
+        size_t smem = 0;
+        int rc = obs_smem_for(kern, (size_t)c->layout.bytes, c->smem_optin, &smem);
+        if (rc) return rc;
+        const int tpb = 128;
+        // Staged in shared memory only where that leaves the SM as many CTAs (fit_launch_core's rule).
+        int per_sm = 1, staged = 0;
+        AST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, tpb, 0));
+        if (smem) AST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&staged, kern, tpb, smem));
+        if (staged < per_sm) smem = 0;
+        if (per_sm < 1) per_sm = 1;
+        int64_t blocks = (n + tpb - 1) / tpb;
+        const int64_t cap = (int64_t)c->sm_count * per_sm;
+        if (blocks > cap) blocks = cap;
+        if (blocks < 1) blocks = 1;
+        kern<<<(unsigned)blocks, tpb, smem, s>>>(dm, c->d_obs, c->layout, smem ? 1 : 0, d_params, n, d_chi2, d_dv, d_err);
+        AST_CUDA(cudaGetLastError());
+        return AST_OK;
+    }
 }
 
 static int eval_dispatch(ast_ctx* c, int32_t precision, const double* d_params, int64_t n, double* d_chi2,

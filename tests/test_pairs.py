@@ -1,6 +1,6 @@
 """The mixed evaluation by integrator and photometer warps (csrc/mixed.cuh) against the thread path, bit
-for bit: ast_eval_batch picks two photometers an integrator up to 32 vectors per SM, one up to 128
-per SM, and one thread a vector beyond."""
+for bit: ast_eval_batch picks pairs, two photometers an integrator, up to 128 vectors per SM (64 under TORQUE with
+NUDGE), and one thread a vector beyond."""
 import numpy as np
 import pytest
 
@@ -25,6 +25,19 @@ def test_pairs_equal_threads(gpu, flags, n, filters, span, precision):
             assert np.array_equal(c, chi2[:count], equal_nan=True), count
             assert np.array_equal(d, dv[:count], equal_nan=True), count
     assert np.isfinite(chi2).mean() > 0.3
+
+
+@pytest.mark.parametrize("precision", [api.PREC_MIXED, api.PREC_MIXED_RHS32])
+def test_both_register_budgets_of_the_thread_kernel(gpu, precision):
+    """The full register file up to two CTAs of 128 an SM, three CTAs beyond: the same bits."""
+    model, obs, P = _object("TORQUE,ACC", 33, 2, 8, 1.0)
+    n = 256 * _sms()
+    big = np.tile(P, (-(-3 * n // 2 // len(P)), 1))[:3 * n // 2]
+    with api.Engine(model, obs) as eng:
+        chi2, dv = eng.eval(big, precision)
+        for count in (n, n + 1):
+            c, d = eng.eval(big[:count], precision)
+            assert np.array_equal(c, chi2[:count], equal_nan=True) and np.array_equal(d, dv[:count], equal_nan=True)
 
 
 @pytest.mark.parametrize("flags,chains,group,kw", [
