@@ -297,7 +297,7 @@ __device__ __forceinline__ uint8_t channel(float br)
 // unit each; the frame's bytes need them only where a value falls within its error of a decision.  So the
 // corners that the float pre-test leaves are evaluated in double-float with an error bound
 // (corner_fast), the pixels from those, and what remains undecided -- grazing lines of sight, the edges
-// of the shadow and of the spot within 1e-6, a channel within 1e-4 of the next byte whose float roundings
+// of the shadow and of the spot within 1e-6, a channel within 5e-4 of the next byte whose float roundings
 // are not certain -- is listed and takes the FP64 expressions.  24 frames of 1080^2: 4.86 ms in FP64.
 __global__ void __launch_bounds__(kRenderTpb, 3) render_kernel(const double* __restrict__ geo,
                                                             const FrameConst* __restrict__ frames, int n_frames, int S,

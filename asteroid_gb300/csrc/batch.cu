@@ -1326,7 +1326,8 @@ static int batch_tune_t(ast_batch* B, int64_t evals_per_slot, ast_batch_launch* 
                 if (int rc = probe(t, 32, tile)) return rc;
             }
     // Integrators and photometers where an untuned batch runs them: two and four integrators a CTA, of the
-    // sizes above (4 864 chains of 300 points: one a CTA 14.4 ms, two 13.4, three 14.7, four 16.5).
+    // sizes above (4 864 chains of 300 points: one a CTA 14.4 ms, two 13.4, three 14.7, four 16.5; threads
+    // 38, tiles of 32 observations 24).
     if (PREC == AST_PREC_MIXED && pair_integrators(B->P.chain_end, B->P.sm_count, kPairIntegrators))
         for (int t : tpbs)
             if (t <= 32 * kPairIntegrators && B->P.n_slots >= t)

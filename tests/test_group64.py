@@ -1,6 +1,6 @@
 """The FP64 evaluation by groups of lanes (csrc/group64.cuh) against the thread path, bit for bit.
 
-ast_eval_batch picks 32 lanes a vector up to four vectors per SM, 8 up to 32 per SM, and one thread a
+ast_eval_batch picks 32 lanes a vector up to four vectors per SM, 8 up to 28 per SM, and one thread a
 vector beyond; the same vectors evaluated in one large call and in small ones must give the same
 bits, whatever the variant, the number of observations (tiles of 8 and 32, remainders) and filters."""
 import ctypes as C
