@@ -1071,8 +1071,9 @@ def main():
                                                 "(add/mul/div/sqrt 1, fma 2); transcendental calls not counted"},
                          "executed": {"achieved": executed, "frac": executed / (peak32 / 1e3),
                                       "fp32_flops_per_eval": NCU_C2["mixed_fp32_flops"] * scale,
-                                      "source": "ncu FFMA x 2 + FADD + FMUL per evaluation of this kernel "
-                                                "(the double-float formulation's own arithmetic)"},
+                                      "source": "ncu FFMA x 2 + FADD + FMUL per evaluation of the kernel with the "
+                                                "step on plain angles, less what the compact-angle step "
+                                                "saves by a count of both on the host"},
                          "peak_source": "measured in this run by ast_probe_peak (FP32 FMA loop over every SM); "
                                         "MEASURED_PEAKS.json holds HBM and bf16 only",
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per launch of the "
