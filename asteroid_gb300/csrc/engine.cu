@@ -400,7 +400,7 @@ static int launch_eval(ast_ctx* c, const DevModel& dm, const double* d_params, i
                        cudaStream_t s, unsigned long long* d_err)
 {
     if constexpr (PREC == AST_PREC_FP64) {
-        const int g = group_lanes(n, c->sm_count, group_most_eval());
+        const int g = group_lanes(n, c->sm_count, group_most_eval(dm.flags, c->steps()));
         if (g == 32) return launch_eval_group<CF, 32>(c, dm, d_params, n, d_chi2, d_dv, s);
         if (g == 8) return launch_eval_group<CF, 8>(c, dm, d_params, n, d_chi2, d_dv, s);
         // The FP64 unit is the SM's: an SM takes its warps' instructions one after the other, so the
@@ -411,7 +411,7 @@ static int launch_eval(ast_ctx* c, const DevModel& dm, const double* d_params, i
         AST_CUDA(cudaGetLastError());
         return AST_OK;
     } else {
-        if (const int k = pair_integrators(n, c->sm_count, pair_most_eval(dm.flags)))
+        if (const int k = pair_integrators(n, c->sm_count, kPairIntegrators))
             return launch_eval_pair<CF, PREC>(c, dm, k, d_params, n, d_chi2, d_dv, s);
         // The full register file while two CTAs of 128 an SM, what it holds then, take the vectors at once;
         // beyond, the precision's own shape, three of them (300 points, 42 000 vectors: 1.43 ms against 1.18 for
@@ -420,7 +420,7 @@ static int launch_eval(ast_ctx* c, const DevModel& dm, const double* d_params, i
         // (20 days: 39 000 vectors 4.79 against 4.93; black-and-white ball, 8 days: 52 000 2.24 against 2.28, 58 367
         // 3.03 against 2.28).
         constexpr int kFull = KernShape<PREC>::min_ctas;
-        const bool steps = PREC == AST_PREC_MIXED && (dm.flags & AST_TORQUE) && c->span >= 2 * dm.time_step * dm.n_data;
+        const bool steps = PREC == AST_PREC_MIXED && (dm.flags & AST_TORQUE) && c->steps() >= 2;
         auto kern = n <= (int64_t)c->sm_count * (steps ? 340 : 256) ? eval_kernel<CF, PREC, 1> : eval_kernel<CF, PREC, kFull>;
         size_t smem = 0;
         int rc = obs_smem_for(kern, (size_t)c->layout.bytes, c->smem_optin, &smem);

@@ -74,6 +74,7 @@ struct ast_ctx {
     ast::DevModel dm{};
     int32_t n_data = 0, n_filters = 0;
     double span = 0;  // days from the first observation to the last
+    double steps() const { return span / dm.time_step / n_data; }  // the span in RK4 steps an observation
     ast::ObsLayout layout{};
     void* d_obs = nullptr;
     // evaluation scratch
@@ -119,23 +120,34 @@ inline int obs_smem_for(K kern, size_t bytes, size_t optin, size_t* smem)
 
 // Lanes an FP64 evaluation by the number that run side by side (1: one thread each).  A warp alone on its
 // quarter of the SM costs its FP64 instructions times 64 cycles, four on an SM 19 each (group64.cuh):
-// eight lanes an evaluation need 2.2 to 3 times fewer, so they win until the SMs hold `most` evaluations, seven
-// such warps (a search with torque six); from there the FP64 unit is full either way and threads do the least.
+// eight lanes an evaluation need 2.2 to 3 times fewer, so they win until the SMs hold `most` evaluations, six to
+// eight such warps; from there the FP64 unit is full either way and threads do the least.
 // Thirty-two lanes share the magnitudes of four times as many observations and win while every
 // evaluation still has a quarter of an SM.  Eight lanes against threads, ms, by evaluations an SM (152 SMs, 60
 // points, 30 RK4 steps an observation; searches of 13 evaluations a chain, their sines the library's):
 //   evaluations, torque     28: 12.9/14.0   32: 14.8/14.0     free 28: 8.7/10.4   32: 9.9/10.4
 //   searches, torque        24: 521/571     28: 598/571       free 28: 299/325    32: 342/325
+//   the same, 10 steps      28: 199/209     32: 226/209            32: 114/121
+//   the same, 3 steps       32: 72/88                              32: 36/51
+//   torque, 10 steps: P_PSI 32: 161/173     from a model 24: 155/172  28: 178/172  32: 203/172
+//   the ball, whose magnitude is a third: torque, 10 steps 24: 101/109; from a model 3 steps 28: 27/30  32: 31/30
 // and 32 lanes against 8, 10 steps an observation: evaluations 4: 3.06/2.97, 6: 3.67/2.97; searches 4: 130/133, 6: 155/134.
+// `steps`: the curve's span in RK4 steps an observation.
 inline int group_lanes(int64_t n, int sm_count, int most)
 {
     return n <= 4 * (int64_t)sm_count ? 32 : n <= (int64_t)most * sm_count ? 8 : 1;
 }
-inline int group_most_eval() { return 28; }
-inline int group_most_fit(int flags) { return flags & AST_TORQUE ? 24 : 28; }
+inline int group_most_eval(int flags, double steps) { return (flags & AST_TORQUE) && steps >= 15 ? 28 : 32; }
+inline int group_most_fit(int flags, bool from_model, double steps)
+{
+    if (!(flags & AST_TORQUE)) return steps < 15 ? 32 : 28;
+    const double w = flags & AST_BW_BALL ? 3 * steps : steps;
+    if (from_model) return w < 5 ? 32 : w < 8 ? 28 : 24;
+    return w < 5 ? 32 : w < 15 ? (flags & AST_P_PSI ? 32 : 28) : 24;
+}
 
 // Integrator warps of a CTA of the paired mixed kernels (mixed.cuh), by the number of evaluations that run
-// side by side; 0: one thread an evaluation, both parts.  At most `most` (pair_most_eval, pair_most_fit).
+// side by side; 0: one thread an evaluation, both parts.  At most `most` (pair_most_fit).
 constexpr int kPairIntegrators = 4;
 inline int pair_integrators(int64_t n, int sm_count, int most)
 {
@@ -154,22 +166,27 @@ inline int pair_integrators(int64_t n, int sm_count, int most)
 //   fits, 60 points, steps 2.1: free, 16 evaluations a chain  3.4/4.8    4.0/4.9      4.4/4.8
 //     100 evaluations:
 //                torque, from a model                      21.7/30.0    25.9/30.6    38.6/29.3
+//                                        steps 0.1         13.1/19.8    14.1/20.2    16.3/20.0
 //                        from the prior                    45.1/46.0    66.7/52.4    88.3/58.6
 //                                        steps 9.1         75.3/88.0    84.7/88.4    98.4/89.0
+//                                        steps 29          174/190      178/189      182/189
+//                        with P_PSI, from the prior        29.9/37.4    36.5/38.6    47.0/38.2
 //                torque, NUDGE, from the prior              143/138      206/183      274/205
 //                FP32 right-hand side, from a model        21.9/27.2    24.7/29.0    31.7/28.2
-// Evaluations are taken for those of models near a solution.  A batch's objects share a launch and its thread kernel keeps three CTAs of 128
-// an SM: pairs up to four (six objects of three variants, 30 evaluations a chain: 26/67, 29/68, 36/67).
-inline int pair_most_eval(int flags)
-{
-    return (flags & AST_TORQUE) && (flags & AST_NUDGE) ? 2 : kPairIntegrators;
-}
+//                                        steps 9.1         53.4/61.4    55.5/62.8    57.3/62.0
+// Evaluations, which are of models near a solution for the most part, take pairs up to four.  So do batches, whose
+// thread kernel keeps three CTAs of 128 an SM (six objects of three variants, 30 evaluations a chain: 26/67,
+// 29/68, 36/67).
 inline int pair_most_fit(int precision, int flags, bool from_model, double steps)
 {
-    if (flags & AST_NUDGE) return 2;
-    if (precision == AST_PREC_MIXED_RHS32) return 3;
+    const bool few = steps >= 1 && steps < 6;  // below, an integrator has little to run
+    if (precision == AST_PREC_MIXED_RHS32 && (flags & AST_NUDGE)) return 3;
+    if (flags & AST_NUDGE) return steps < 20 ? 2 : 3;
     if (!(flags & AST_TORQUE)) return kPairIntegrators;
-    return from_model || steps >= 6 ? 3 : 2;
+    if (precision == AST_PREC_MIXED_RHS32) return few ? 3 : 4;
+    // A period's range (P_PSI) keeps most of the prior's models within the compact step, as a model does.
+    if (from_model || (flags & AST_P_PSI)) return few ? 3 : 4;
+    return steps < 6 ? 2 : steps < 20 ? 3 : 4;
 }
 
 int build_dev_model(const ast_model* m, const ast_obs_set* obs, DevModel* dm);

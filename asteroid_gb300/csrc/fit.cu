@@ -490,9 +490,9 @@ static int fit_launch_core(int sm_count, size_t obs_bytes, size_t optin, int tpb
 template <class CF, int PREC>
 static int fit_launch_cfg(ast_ctx* c, const ast_fit_cfg* cfg, FitRun* r)
 {
-    const int most = pair_most_fit(PREC, c->dm.flags, cfg->reopt != 0, c->span / c->dm.time_step / c->n_data);
+    const int most = pair_most_fit(PREC, c->dm.flags, cfg->reopt != 0, c->steps());
     return fit_launch_core<CF, PREC>(c->sm_count, (size_t)c->layout.bytes, c->smem_optin, cfg->tpb, cfg->min_ctas_per_sm,
-                                     cfg->stage_obs, cfg->n_chains, group_most_fit(c->dm.flags), most, r);
+                                     cfg->stage_obs, cfg->n_chains, group_most_fit(c->dm.flags, cfg->reopt != 0, c->steps()), most, r);
 }
 
 extern "C" int ast_fit_begin(ast_ctx* c, const ast_fit_cfg* cfg)
@@ -881,7 +881,8 @@ extern "C" int ast_fit_noalloc(const ast_model* model, const ast_obs_set* obs, c
     AST_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     AST_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     FitRun r;
-    const int gm = group_most_fit(dm.flags), pm = kPairIntegrators;  // (no more than one integrator an SM)
+    // The span is on the device: lane groups as for few steps (at most 27 chains an SM); one integrator an SM.
+    const int gm = group_most_fit(dm.flags, cfg->reopt != 0, 0.0), pm = kPairIntegrators;
     const int tpb = cfg->tpb, mb = cfg->min_ctas_per_sm, so = cfg->stage_obs;
     const int64_t C = cfg->n_chains;
     const bool fp64 = cfg->precision == AST_PREC_FP64;

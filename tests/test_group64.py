@@ -1,7 +1,7 @@
 """The FP64 evaluation by groups of lanes (csrc/group64.cuh) against the thread path, bit for bit.
 
-ast_eval_batch picks 32 lanes a vector up to four vectors per SM, 8 up to 28 per SM, and one thread a
-vector beyond; the same vectors evaluated in one large call and in small ones must give the same
+ast_eval_batch picks 32 lanes a vector up to four vectors per SM, 8 up to 32 per SM (28 with torque and many steps
+an observation), and one thread a vector beyond; the same vectors evaluated in one large call and in small ones must give the same
 bits, whatever the variant, the number of observations (tiles of 8 and 32, remainders) and filters."""
 import ctypes as C
 
@@ -91,10 +91,13 @@ def test_fits_by_lane_groups_equal_threads(gpu, flags, chains, group, kw):
         assert r.n_evals == b.n_evals and r.n_fits == b.n_fits
 
 
-# The most chains by lane groups, and one more: with torque, whose step has more FP64 instructions to spread, and without.
-@pytest.mark.parametrize("flags,per_sm", [("TORQUE,ACC", 24), ("ACC", 28), ("BW_BALL", 28)])
-def test_where_fits_by_lane_groups_end(gpu, flags, per_sm):
-    model, obs, P = _object(flags, 33, 2, 5, 1.0)
+# The most chains by lane groups, and one more, with few steps an observation (3) and many: with torque, whose steps
+# have more FP64 instructions to spread, and without; the ball's magnitudes have fewer.
+@pytest.mark.parametrize("flags,span,per_sm", [
+    ("TORQUE,ACC", 1.0, 32), ("TORQUE,ACC", 3.0, 28), ("TORQUE", 6.0, 24), ("TORQUE,P_PSI", 3.0, 32), ("TORQUE,BW_BALL,ACC", 1.0, 28), ("ACC", 3.0, 32),
+    ("BW_BALL", 6.0, 28)])
+def test_where_fits_by_lane_groups_end(gpu, flags, span, per_sm):
+    model, obs, P = _object(flags, 33, 2, 5, span)
     n = per_sm * _sms()
     with api.Engine(model, obs) as eng:
         for chains, lanes in ((n, 8), (n + 1, 1)):

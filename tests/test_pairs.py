@@ -1,6 +1,6 @@
 """The mixed evaluation by integrator and photometer warps (csrc/mixed.cuh) against the thread path, bit
-for bit: ast_eval_batch picks pairs, two photometers an integrator, up to 128 vectors per SM (64 under TORQUE with
-NUDGE), and one thread a vector beyond."""
+for bit: ast_eval_batch picks pairs, two photometers an integrator, up to 128 vectors per SM, and one thread a vector
+beyond."""
 import numpy as np
 import pytest
 
@@ -121,14 +121,20 @@ def test_a_requested_geometry_is_not_run_by_the_paired_graph(gpu):
         assert np.array_equal(getattr(g, k), getattr(ref, k), equal_nan=True)
 
 
-# One integrator to four, and where threads take over: with torque at the third or fourth (a start from the prior
-# or from a model, a sparse or a dense curve), with NUDGE at the third, with the FP32 right-hand side at the fourth.
+# One integrator to four, and where threads take over: with torque at the third or fourth (a start from the prior,
+# without a period's range, or from a model; few steps an observation or many), with NUDGE at the third, with the FP32
+# right-hand side and few steps at the fourth.
 @pytest.mark.parametrize("flags,chains,span,precision,reopt,integrators", [
     ("ACC", 4864, 1.0, api.PREC_MIXED, False, 1), ("ACC", 19456, 1.0, api.PREC_MIXED, False, 4), ("ACC", 19488, 1.0, api.PREC_MIXED, False, 0),
     ("TORQUE,ACC", 9728, 1.0, api.PREC_MIXED, False, 2), ("TORQUE,ACC", 9760, 1.0, api.PREC_MIXED, False, 0),
-    ("TORQUE,ACC", 9760, 5.0, api.PREC_MIXED, False, 3), ("TORQUE,ACC", 14592, 1.0, api.PREC_MIXED, True, 3),
-    ("TORQUE", 14624, 5.0, api.PREC_MIXED, True, 0), ("NUDGE", 9728, 1.0, api.PREC_MIXED, True, 2), ("NUDGE", 9760, 5.0, api.PREC_MIXED, True, 0),
-    ("TORQUE,ACC", 14592, 1.0, api.PREC_MIXED_RHS32, False, 3), ("ACC", 14624, 1.0, api.PREC_MIXED_RHS32, True, 0)])
+    ("TORQUE,ACC", 9760, 5.0, api.PREC_MIXED, False, 3), ("TORQUE,ACC", 14624, 5.0, api.PREC_MIXED, False, 0),
+    ("TORQUE,ACC", 14624, 12.0, api.PREC_MIXED, False, 4), ("TORQUE,ACC", 14592, 1.0, api.PREC_MIXED, True, 3),
+    ("TORQUE", 14624, 1.0, api.PREC_MIXED, True, 0), ("TORQUE", 14624, 5.0, api.PREC_MIXED, True, 4),
+    ("TORQUE,P_PSI,ACC", 9760, 1.0, api.PREC_MIXED, False, 3), ("TORQUE,P_PSI,ACC", 14624, 1.0, api.PREC_MIXED, False, 0), ("NUDGE", 9728, 1.0, api.PREC_MIXED, True, 2), ("NUDGE", 9760, 5.0, api.PREC_MIXED, True, 0),
+    ("TORQUE,ACC", 14592, 1.0, api.PREC_MIXED_RHS32, False, 3), ("TORQUE,ACC", 14624, 1.0, api.PREC_MIXED_RHS32, True, 0),
+    ("TORQUE", 14624, 0.4, api.PREC_MIXED, True, 4), ("TORQUE,NUDGE", 9760, 12.0, api.PREC_MIXED, True, 3),
+    ("TORQUE,NUDGE", 9760, 1.0, api.PREC_MIXED_RHS32, True, 3),
+    ("TORQUE,ACC", 14624, 5.0, api.PREC_MIXED_RHS32, True, 4)])
 def test_where_fits_by_pairs_end(gpu, flags, chains, span, precision, reopt, integrators):
     if _sms() != 152:
         pytest.skip("the chain counts are those of 152 SMs")
